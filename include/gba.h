@@ -182,10 +182,13 @@ typedef struct gba_options {
   int32_t schur;                      /* gba_schur, GBA_SCHUR_AUTO                   */
   int32_t persistent_pcg;             /* 1 = with the explicit Schur complement, run
                                          the whole PCG of an LM iteration in one
-                                         launch where the form allows: the mixed
-                                         precision as a thread-block cluster per
-                                         problem, the FP64 form of a single problem
-                                         over the whole GPU (grid-wide barriers; it
+                                         launch where the form allows: as a
+                                         thread-block cluster per problem (mixed
+                                         precision up to 1,024 cameras; FP64 up to
+                                         128 cameras whose blocks of S fit the
+                                         cluster's shared memory), a larger single
+                                         FP64 problem over the whole GPU
+                                         (grid-wide barriers; it
                                          expects the GPU to itself: beside other
                                          kernels it runs on the SMs it finds free,
                                          correct but slower; the server's slots

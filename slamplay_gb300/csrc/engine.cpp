@@ -443,10 +443,15 @@ gba_status Engine::upload(const HostBatch &hb, std::string *err) {
   if (mixed_ && hb.explicit_schur && o_.persistent_pcg &&
       !pcg_cluster_plan(hb.prob.data(), (int)hb.prob.size(), hb.sblk_row.data(), cluster_cams_, &cl_plan_))
     cl_plan_ = ClusterPlan();
-  // the PCG as one grid-wide launch per LM iteration: FP64 form, explicit
-  // Schur complement, one problem
+  // the same in the FP64 form, where the rows of S fit the clusters; a single
+  // problem too large for that takes one grid-wide launch per LM iteration
+  c64_plan_ = Cluster64Plan();
+  if (!mixed_ && hb.explicit_schur && o_.persistent_pcg && !grid_wait_test_ &&
+      !pcg_cluster64_plan(hb.prob.data(), (int)hb.prob.size(), hb.sblk_row.data(),
+                          o_.pcg_criterion == GBA_PCG_QUADRATIC_MODEL, &c64_plan_))
+    c64_plan_ = Cluster64Plan();
   gr_plan_ = GridPlan();
-  if (o_.persistent_pcg && !pcg_grid_plan((int)hb.prob.size(), mixed_, hb.explicit_schur, hb.nc,
+  if (o_.persistent_pcg && c64_plan_.cs == 0 && !pcg_grid_plan((int)hb.prob.size(), mixed_, hb.explicit_schur, hb.nc,
                                           hb.explicit_schur ? hb.sblk_row.data() : nullptr, grid_ctas_, &gr_plan_))
     gr_plan_ = GridPlan();
   // current batch shape + pointers + options + PCG form = graph key
@@ -455,6 +460,9 @@ gba_status Engine::upload(const HostBatch &hb, std::string *err) {
   cur_key_.push_back(cl_plan_.cs);
   cur_key_.push_back(cl_plan_.threads);
   cur_key_.push_back(cl_plan_.cache_blocks);
+  cur_key_.push_back(c64_plan_.cs);
+  cur_key_.push_back(c64_plan_.R);
+  cur_key_.push_back(c64_plan_.pairs_max);
   cur_key_.push_back(gr_plan_.grid);
   cur_key_.push_back(gr_plan_.cap_blocks);
   cur_key_.push_back(gr_plan_.cap_pairs);
@@ -681,7 +689,7 @@ gba_status Engine::build_graph(std::string *err, bool cont) {
   cudaGraph_t lmbody = nullptr, pcgbody = nullptr, tmp = nullptr;
   if ((e = add_while(stream_, lmh, &lmbody)) != cudaSuccess) return fail(e, "LM conditional node");
   // (a conditional handle must belong to a node: none for the cluster PCG)
-  const bool one_launch = cl_plan_.cs > 0 || gr_plan_.grid > 0;
+  const bool one_launch = one_launch_pcg();
   if (!one_launch &&
       (e = cudaGraphConditionalHandleCreate(&pcgh, lmbody, 1, cudaGraphCondAssignDefault)) != cudaSuccess)
     return fail(e, "PCG conditional handle");
@@ -692,6 +700,8 @@ gba_status Engine::build_graph(std::string *err, bool cont) {
   if (cl_plan_.cs > 0) {
     // the whole PCG of every problem in one cluster launch
     if ((e = launch_pcg_cluster(db_, cl_plan_, cap_[0])) != cudaSuccess) return fail(e, "PCG cluster kernel");
+  } else if (c64_plan_.cs > 0) {
+    if ((e = launch_pcg_cluster64(db_, c64_plan_, cap_[0])) != cudaSuccess) return fail(e, "PCG cluster kernel");
   } else if (gr_plan_.grid > 0) {
     // the whole PCG of the problem in one grid-wide launch
     if ((e = launch_pcg_grid(db_, gr_plan_, cap_[0])) != cudaSuccess) return fail(e, "PCG grid kernel");
@@ -785,7 +795,7 @@ gba_status Engine::run_host_driven(std::string *err) {
   while (hstat[1] && hstat[0] == 0) {
     if (++bodies > max_lm_bodies() + 2) break;
     enqueue_lm_head(stream_);
-    if (cl_plan_.cs > 0 || gr_plan_.grid > 0) {
+    if (one_launch_pcg()) {
       if ((st = enqueue_pcg_one_launch(stream_, err)) != GBA_OK) return st;
       enqueue_lm_tail(stream_);
       if ((st = read_status()) != GBA_OK) return st;
@@ -827,6 +837,11 @@ static double bytes_pcg_grid(const DeviceBatch &b) {
 
 gba_status Engine::enqueue_pcg_one_launch(cudaStream_t s, std::string *err) {
   prof_begin(s);
+  if (c64_plan_.cs > 0) {
+    const gba_status st = check(launch_pcg_cluster64(db_, c64_plan_, s), "PCG cluster kernel", err);
+    prof_end(s, PF_GRID, bytes_pcg_grid(db_));  // (the FP64 form's one-launch PCG)
+    return st;
+  }
   if (gr_plan_.grid > 0) {
     const gba_status st = check(launch_pcg_grid(db_, gr_plan_, s), "PCG grid kernel", err);
     prof_end(s, PF_GRID, bytes_pcg_grid(db_));
@@ -1246,7 +1261,7 @@ gba_status Engine::compute_step(const gba_problem_view *v, double radius, double
   launch_camera_schur(db_, mixed_, stream_);
   launch_schur_form(db_, mixed_, stream_);
   if ((st = read_status()) != GBA_OK) return st;
-  if (cl_plan_.cs > 0 || gr_plan_.grid > 0) {
+  if (one_launch_pcg()) {
     if ((st = enqueue_pcg_one_launch(stream_, err)) != GBA_OK) return st;
   } else {
     int pcg = 0;

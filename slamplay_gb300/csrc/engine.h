@@ -46,7 +46,7 @@ class Engine {
   void set_tuning(int chunk_observations, int pcg_unroll, int cluster_cams = 0, int pcg_cap = 0, int grid_ctas = 0);
   bool cluster_pcg() const { return cl_plan_.cs > 0; }
   int grid_pcg_ctas() const { return gr_plan_.grid; }
-  bool one_launch_pcg() const { return cl_plan_.cs > 0 || gr_plan_.grid > 0; }
+  bool one_launch_pcg() const { return cl_plan_.cs > 0 || c64_plan_.cs > 0 || gr_plan_.grid > 0; }
   double last_solve_ms() const { return last_solve_ms_; }
   PrepOptions prep_options() const;
   cudaStream_t stream() const { return stream_; }
@@ -144,6 +144,7 @@ class Engine {
   int sm_count_ = 0;
   bool pdl_ = true;        // programmatic dependent launches inside the PCG body
   ClusterPlan cl_plan_;    // cs > 0: the PCG runs as one cluster launch per LM iteration
+  Cluster64Plan c64_plan_; // cs > 0: the same in the FP64 form
   GridPlan gr_plan_;       // grid > 0: the PCG runs as one grid-wide launch per LM iteration
   HostBatch hb_;           // the last solve's prepared batch (storage reused)
   gba_status enqueue_pcg_one_launch(cudaStream_t s, std::string *err);

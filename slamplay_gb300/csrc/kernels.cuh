@@ -29,13 +29,19 @@ struct Prec<true> {
 // 1/a: the FP32 hardware reciprocal refined by two Newton-Raphson steps
 // x <- x + x (1 - a x), each of which doubles the number of correct bits
 // (about 23 -> 46 -> FP64 rounding).  Falls back to a division outside the
-// FP32 normal range.
+// FP32 normal range.  The range test and the conversions to and from FP32
+// are integer instructions (same values): as FP64 instructions each would
+// hold the FP64 pipe for 64 clocks a warp, as long as a Newton step's FMA.
 __device__ __forceinline__ double recip_nr(double a) {
-  const double aa = fabs(a);
-  if (!(aa > 1e-30 && aa < 1e30)) return 1.0 / a;
+  const long long ab = __double_as_longlong(a) & 0x7fffffffffffffffLL;
+  if (!(ab > 0x39b4484bfeebc2a0LL && ab < 0x46293e5939a08ceaLL)) return 1.0 / a;  // 1e-30 < |a| < 1e30
+  // |a| rounded to the nearest float (ties to even), its sign put back after
+  const unsigned fb = (unsigned)((ab + 0xfffffffLL + ((ab >> 29) & 1)) >> 29) - (896u << 23);
   float xf;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(xf) : "f"((float)a));
-  double x = (double)xf;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(xf) : "f"(__uint_as_float(fb)));
+  const unsigned xb = __float_as_uint(xf);
+  const unsigned hi = ((xb >> 3) + (896u << 20)) | ((unsigned)__double2hiint(a) & 0x80000000u);
+  double x = __hiloint2double((int)hi, (int)(xb << 29));
   double e = fma(-a, x, 1.0);
   x = fma(x, e, x);
   e = fma(-a, x, 1.0);

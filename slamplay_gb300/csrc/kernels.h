@@ -52,6 +52,22 @@ struct ClusterPlan {
 bool pcg_cluster_plan(const ProblemInfo *prob, int num_problems, const int32_t *sblk_row, int cams_per_cta,
                       ClusterPlan *plan);
 cudaError_t launch_pcg_cluster(const DeviceBatch &b, const ClusterPlan &plan, cudaStream_t s);
+// K4 cluster form of the FP64 precision: as the above, the FP64 arithmetic of
+// the two-kernel PCG addition for addition (the same bits), problems whose
+// rows of S fit the shared memory of a cluster.
+constexpr int kC64MaxCS = 16;
+constexpr int kC64MaxCams = 128;
+struct Cluster64Plan {
+  int cs = 0, R = 0;  // CTAs per problem, rows of S per thread of the product
+  bool quad = false;
+  int n_max = 0, own_max = 0, pairs_max = 0;
+  size_t smem = 0;
+  double clocks = 0;  // estimated clocks of the largest problem's PCG iteration
+};
+// quad: the quadratic-model stopping test (gba_pcg_criterion).
+bool pcg_cluster64_plan(const ProblemInfo *prob, int num_problems, const int32_t *sblk_row, bool quad,
+                        Cluster64Plan *plan);
+cudaError_t launch_pcg_cluster64(const DeviceBatch &b, const Cluster64Plan &plan, cudaStream_t s);
 // K4 grid form: the whole PCG of one problem in one launch, one CTA per SM
 // with grid-wide barriers (FP64 form, explicit Schur complement).
 struct GridPlan {
