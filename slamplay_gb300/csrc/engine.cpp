@@ -441,7 +441,8 @@ gba_status Engine::upload(const HostBatch &hb, std::string *err) {
   // Schur complement, every problem small enough
   cl_plan_ = ClusterPlan();
   if (mixed_ && hb.explicit_schur && o_.persistent_pcg &&
-      !pcg_cluster_plan(hb.prob.data(), (int)hb.prob.size(), hb.sblk_row.data(), cluster_cams_, &cl_plan_))
+      !pcg_cluster_plan(hb.prob.data(), (int)hb.prob.size(), hb.sblk_row.data(), cluster_cams_,
+                        o_.pcg_criterion == GBA_PCG_QUADRATIC_MODEL, &cl_plan_))
     cl_plan_ = ClusterPlan();
   // the same in the FP64 form, where the rows of S fit the clusters; a single
   // problem too large for that takes one grid-wide launch per LM iteration

@@ -40,6 +40,7 @@ constexpr int kClMaxCams = 1024; // cameras per problem
 struct ClusterPlan {
   int cs = 0, n_max = 0, own_max = 0;
   int threads = 0;
+  bool quad = false;
   int cache_blocks = 0;  // > 0: each CTA keeps its rows of S (this many 9x9 blocks at most) in shared memory
   size_t smem = 0;
 };
@@ -48,8 +49,9 @@ struct ClusterPlan {
 // explicit complement's row structure (sblk_row, nc + 1); false when the
 // form does not apply or cannot be launched.
 // cams_per_cta: the cameras of a problem one CTA of its cluster takes (the
-// cluster size follows); 0 = 16 for a single problem, 64 for a batch.
-bool pcg_cluster_plan(const ProblemInfo *prob, int num_problems, const int32_t *sblk_row, int cams_per_cta,
+// cluster size follows); 0 = the shortest estimated iteration.
+// quad: the quadratic-model stopping test (gba_pcg_criterion).
+bool pcg_cluster_plan(const ProblemInfo *prob, int num_problems, const int32_t *sblk_row, int cams_per_cta, bool quad,
                       ClusterPlan *plan);
 cudaError_t launch_pcg_cluster(const DeviceBatch &b, const ClusterPlan &plan, cudaStream_t s);
 // K4 cluster form of the FP64 precision: as the above, the FP64 arithmetic of
