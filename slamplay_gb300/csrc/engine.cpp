@@ -109,6 +109,8 @@ gba_status Engine::init(std::string *err) {
   {
     const char *e = std::getenv("GBA_TEST_GRID_WAIT");
     grid_wait_test_ = e && e[0] == '1';
+    const char *c = std::getenv("GBA_TEST_GRID_CTAS");
+    grid_ctas_test_ = c ? std::max(0, std::atoi(c)) : 0;
   }
   if ((st = check(probe_kernel_image(), "loading the sm_103a kernels", err)) != GBA_OK) return st;
   if (o_.stream) {
@@ -281,8 +283,7 @@ size_t Engine::layout(const HostBatch &hb, char *base, DeviceBatch *db, size_t *
   b.cam_Sii = cv.take<char>(ex ? 81 * nc * rs : 0);
   b.pcg_q = cv.take<double>(ex ? 9 * nc : 0);
   b.spmv_red = cv.take<double>(ex ? nc : 0);
-  b.pcg_p2 = cv.take<double>(ex ? 9 * nc : 0);
-  b.pq_row = cv.take<double>(ex ? 9 * nc : 0);
+  b.grid_slots = cv.take<GridSlot>(ex && !mixed_ && P == 1 ? grid_slot_count(nc, nb) : 0);
   b.grid_ctl = cv.take<uint32_t>(8);
   b.prob_counter = cv.take<uint32_t>(4 * P);
   b.global_counter = cv.take<uint32_t>(8);
@@ -447,14 +448,17 @@ gba_status Engine::upload(const HostBatch &hb, std::string *err) {
   // the same in the FP64 form, where the rows of S fit the clusters; a single
   // problem too large for that takes one grid-wide launch per LM iteration
   c64_plan_ = Cluster64Plan();
-  if (!mixed_ && hb.explicit_schur && o_.persistent_pcg && !grid_wait_test_ &&
+  if (!mixed_ && hb.explicit_schur && o_.persistent_pcg && !grid_wait_test_ && grid_ctas_test_ == 0 &&
       !pcg_cluster64_plan(hb.prob.data(), (int)hb.prob.size(), hb.sblk_row.data(),
                           o_.pcg_criterion == GBA_PCG_QUADRATIC_MODEL, &c64_plan_))
     c64_plan_ = Cluster64Plan();
   gr_plan_ = GridPlan();
   if (o_.persistent_pcg && c64_plan_.cs == 0 && !pcg_grid_plan((int)hb.prob.size(), mixed_, hb.explicit_schur, hb.nc,
-                                          hb.explicit_schur ? hb.sblk_row.data() : nullptr, grid_ctas_, &gr_plan_))
+                                          hb.explicit_schur ? hb.sblk_row.data() : nullptr,
+                                          hb.explicit_schur ? hb.sblk_col.data() : nullptr, grid_ctas_,
+                                          o_.pcg_criterion == GBA_PCG_QUADRATIC_MODEL, &gr_plan_))
     gr_plan_ = GridPlan();
+  if (grid_ctas_test_ > 0 && gr_plan_.grid > 0) gr_plan_.grid = std::min(gr_plan_.grid, grid_ctas_test_);
   // current batch shape + pointers + options + PCG form = graph key
   DeviceBatch k = db_;
   cur_key_.assign(reinterpret_cast<const char *>(&k), reinterpret_cast<const char *>(&k) + sizeof k);
@@ -465,7 +469,7 @@ gba_status Engine::upload(const HostBatch &hb, std::string *err) {
   cur_key_.push_back(c64_plan_.R);
   cur_key_.push_back(c64_plan_.pairs_max);
   cur_key_.push_back(gr_plan_.grid);
-  cur_key_.push_back(gr_plan_.cap_blocks);
+  cur_key_.push_back(gr_plan_.cap_cols);
   cur_key_.push_back(gr_plan_.cap_pairs);
   return GBA_OK;
 }
@@ -576,6 +580,11 @@ void Engine::zero_counters(cudaStream_t s) {
   cudaMemsetAsync(db_.global_counter, 0, 8 * sizeof(uint32_t), s);
   if (db_.nchunks > 0) cudaMemsetAsync(db_.chunk_counter, 0, sizeof(uint32_t) * (size_t)db_.nchunks, s);
   if (!mixed_ && db_.nc > 0) cudaMemsetAsync(db_.cam_counter, 0, sizeof(uint32_t) * (size_t)db_.nc, s);
+  if (gr_plan_.grid > 0) {
+    // no slot carries a tag of an earlier solve, and the launches count from 0
+    cudaMemsetAsync(db_.grid_slots, 0, sizeof(GridSlot) * grid_slot_count(db_.nc, db_.cam_blocks), s);
+    cudaMemsetAsync(db_.grid_ctl, 0, 8 * sizeof(uint32_t), s);
+  }
 }
 
 void Engine::enqueue_setup(cudaStream_t s) {

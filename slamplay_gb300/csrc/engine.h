@@ -126,6 +126,8 @@ class Engine {
   int segment_bodies_ = 0;
   int cluster_cams_ = 0;  // cameras per CTA of the cluster PCG (0 = default)
   int grid_ctas_ = 0;     // CTAs of the grid PCG (0 = every SM)
+  int grid_ctas_test_ = 0;       // test of the grid PCG with fewer CTAs than planned (environment
+                                 // GBA_TEST_GRID_CTAS at handle creation), as beside other kernels
   bool grid_wait_test_ = false;  // the grid PCG's wait-runs-out test (DeviceOptions::grid_wait_test)
   int graph_segment_ = -1, graph_c_segment_ = -1;
   std::vector<long long> cur_key_;

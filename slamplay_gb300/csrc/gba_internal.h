@@ -53,10 +53,10 @@ struct DeviceOptions {
   int32_t max_bodies;  // LM bodies (trials) a solve may run
   int32_t pinhole;     // local-BA windows: the stereo-rig pinhole model, SE3 poses
   int32_t bodies_cap;  // > 0: the LM loop of one launch stops after this many counted bodies
-  int32_t grid_wait_test;  // failure test of the grid PCG (environment GBA_TEST_GRID_WAIT=1 at
-                           // handle creation): every barrier waits for one CTA more than
-                           // registered, so its bounded wait runs out (GBA_ERR_TIMEOUT)
                        // (the problems stay active; a later launch continues them)
+  int32_t grid_wait_test;  // failure test of the grid PCG (environment GBA_TEST_GRID_WAIT=1 at
+                           // handle creation): every wait is for a tag that nothing writes,
+                           // so it runs out (GBA_ERR_TIMEOUT)
 };
 
 // Per problem of a local-BA batch: fx, fy, cx, cy, then R (9, row-major) and
@@ -96,6 +96,19 @@ struct LMState {
   int32_t pad_;
   int64_t total_pcg_iterations;
 };
+
+// A value the grid PCG's CTAs publish: the double and the tag of its launch
+// and iteration, accessed as 16 bytes at once.
+struct alignas(16) GridSlot {
+  double value;
+  unsigned long long tag;
+};
+// Slots of a problem of nc cameras in nb camera blocks: two sets (by
+// iteration parity) of q, z and p per coordinate, five p.q values per camera
+// and, in kGridCopies copies (what every CTA reads), one per chunk of 32
+// cameras and three per block.
+constexpr int kGridCopies = 8;
+inline size_t grid_slot_count(size_t nc, size_t nb) { return 2 * (27 * nc + 5 * nc + kGridCopies * (3 * nb + (nc + 31) / 32)); }
 
 // Everything a kernel may touch, as raw device pointers.  Built by the host
 // (solver.cpp) and passed by value to every launch.
@@ -213,10 +226,6 @@ struct DeviceBatch {
   void *cam_Sii;             // 81 * nc
   double *pcg_q;             // 9 * nc
   double *spmv_red;          // nc
-  // the grid PCG (FP64, one problem): the second direction buffer (the
-  // directions alternate between pcg_p and pcg_p2 by iteration parity) and
-  // its control words (kGrid* slots), zeroed by K3b before each launch
-  double *pcg_p2;            // 9 * nc
   // a resumed batch (a problem continued in a new batch at an LM-iteration
   // boundary): per problem a flag and the LM state to continue from, per
   // camera / point the Jacobi scales of its first evaluation (internal
@@ -224,7 +233,10 @@ struct DeviceBatch {
   const int32_t *prob_resume;
   const LMState *lm_resume;
   const double *cam_scale_in, *pt_scale_in;
-  double *pq_row;            // 9 * nc: each row's p_i q_i, [row of the camera][camera of the problem]
+  // the grid PCG (FP64, one problem): the published values (grid_slot_count
+  // of them, zeroed before a solve) and its control words (kGrid* slots),
+  // zeroed by K3b before each launch but for the launch count
+  GridSlot *grid_slots;
   uint32_t *grid_ctl;        // 8
 };
 
@@ -256,12 +268,12 @@ constexpr int kGC_SCHUR = 0, kGC_UPDATE = 1, kGC_POST = 2, kGC_LMBODIES = 3;
 // grid PCG: threads per CTA (16 warps: four per SM sub-partition, so up to
 // 128 registers a thread) and the control words: registration (64-bit:
 // count, and the closed bit), the published participant count + 1, the
-// barrier counter, the abort word
+// abort word, the launch count of the solve
 constexpr int kPcgGridThreads = 512;
 // chunk sums (32 cameras each) of the explicit FP64 form's p.q in the camera
 // kernel: problems of up to 32 * kPcgChunkSums cameras
 constexpr int kPcgChunkSums = 1024;
-constexpr int kGridReg = 0, kGridCount = 2, kGridBar = 3, kGridAbort = 4;
+constexpr int kGridReg = 0, kGridCount = 2, kGridAbort = 4, kGridLaunch = 7;
 
 // A problem without observations has no parameter blocks in the
 // reference's problem (each observation adds its camera and point through

@@ -57,7 +57,7 @@ constexpr int kC64Slot = 96;  // threads per camera block in the update (3 warps
 constexpr int kC64Own = kC64Threads / kC64Slot;  // camera blocks a CTA updates, at most
 constexpr int kC64Coords = 9 * kPcgBlockCams;
 constexpr int kC64MaxBlocks = kC64MaxCams / kPcgBlockCams;
-constexpr double kC64GridClocks = 15000.0;  // estimated iteration from which one problem takes the grid form
+constexpr double kC64GridClocks = 10500.0;  // estimated iteration from which one problem takes the grid form
 constexpr int kC64Levels = 8;  // levels of the pairwise tree (rows of up to kC64MaxCams + 1 blocks)
 static_assert(kC64Coords <= kC64Slot && kC64Slot % 32 == 0, "a camera block's coordinates fit three whole warps");
 static_assert(kC64MaxBlocks <= 16, "half a warp holds one quantity of every block");

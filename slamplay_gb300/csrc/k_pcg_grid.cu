@@ -1,55 +1,64 @@
 // k_pcg_grid.cu — the whole PCG of one problem in one launch spread over the
-// whole GPU (FP64 form, explicit Schur complement).
+// whole GPU (FP64 form, explicit Schur complement), for problems whose rows
+// of S do not fit a cluster (k_pcg_cluster64.cu) or keep it too busy.
 //
-// In the FP64 form a PCG iteration is about 0.6 M FP64 FMAs (the product
-// with the 9x9 blocks of S) separated by two problem-wide reductions.  GB300
-// issues FP64 at about two FMAs per clock per SM, so the product alone takes
-// some 10 us on the 16 SMs of a thread-block cluster and ~1 us on all SMs;
-// as two kernels per iteration (k_schur.cu's product, k_pcg.cu's camera
-// kernel) the iteration costs two kernel boundaries (~27 us).  Here one CTA
-// per SM runs every iteration of the problem's PCG, with a grid-wide
-// barrier after each reduction:
-//   A. q = S p_k for the rows the CTA owns (runs of about equal numbers of
-//      row blocks of S): p_k = z_k + beta_k p_{k-1} at the columns of the
-//      touched cameras' blocks staged in shared memory; a thread per (row,
-//      block) pair of the owned rows (a nine-column FMA chain), each row's
-//      block dots summed by the pairwise tree (the additions of each tree
-//      level listed once per launch and spread over all threads); each
-//      row's p_i q_i.                                           barrier
-//   B. every CTA: each camera's p.q (sum9_tree of its rows), their sum
-//      (chunks of 32 and a tree), alpha; for the camera blocks (8 cameras)
-//      the CTA owns: p_k, x, r, z = M r, each block's r.z, r.r, x.(v + r).
-//                                                                barrier
-//   C. in every CTA: the stopping test and beta_{k+1} from the blocks'
-//      values (three warps, one sum each), while the other warps load what
-//      the next iteration's staged direction needs.
-// The touched cameras' blocks of S stay in shared memory for the launch (S
-// is fixed during the PCG) when they fit; a CTA with more than the layout
-// holds reads them from L2.  GB300's FP64 pipe retires about one warp
-// instruction per 64 clocks per SM sub-partition, so the work is split by
-// rows (not cameras) for an even load over the CTAs and spread over all 16
-// warps of a CTA, and the direction is formed once per (block, column), not
-// once per row.
-// Every CTA takes the same decisions from the same values, so all reach the
-// same barriers.  The arithmetic is the two-kernel FP64 PCG's, operation
-// for operation (the fixed trees of kernels.cuh, k_schur.cu's product and
-// the camera kernel's reductions), so both forms give the same bits, and no
-// result depends on how many CTAs took part.
+// In the FP64 form a PCG iteration is a product with the 9x9 blocks of S
+// (0.6 M FMAs on 250 cameras of a walk, about 1 us of the FP64 pipes of all
+// SMs) between two problem-wide reductions; GB300 issues a dependent FP64
+// instruction every 64 clocks, so the rest is the chain of the reductions
+// and the exchanges between SMs through L2 (about 0.4 us a trip each way).
+// One CTA per SM runs every iteration:
+//   A. q = S p for the rows the CTA owns (runs of about equal numbers of row
+//      blocks): p at the columns the rows touch and the rows of S in shared
+//      memory, a thread per (row, block) pair (a nine-column FMA chain), each
+//      row's block dots summed by the pairwise tree; q_i, and p_i q_i summed
+//      over the row pairs (0,1) (2,3) (4,5) (6,7) of a camera (the first
+//      level of sum9_tree; row 8 alone), are published;
+//   B. the CTAs that own a chunk of 32 cameras: each camera's p.q from its
+//      five values, the chunk's sum, published; every CTA: the chunks' sum (a
+//      tree), alpha; for the camera blocks (8 cameras) the CTA owns: x, r,
+//      z = M r, each block's r.z, r.r (and x.(v + r) when the stopping test
+//      reads it), published with z;
+//   C. every CTA: the sums over the blocks, the stopping test and beta in
+//      warp 0, while the other warps fetch z of the touched columns;
+//      p = z + beta p there.
+// A published value is a 16-byte slot, the double and a tag of the launch
+// and the iteration, written and read as one 128-bit access: a reader polls
+// the slot itself until the tag is the one it waits for.  So an exchange
+// costs the store's way to L2 and one read, no barrier, no fence and no
+// second read; the slots alternate between two sets by iteration parity, and
+// a set is only written again after every reader of its values has published
+// what depends on them.  One exchange from every CTA to every CTA would be
+// 152 x 152 readers of the same lines (5 us, measured), so the p.q goes in
+// two hops, over the CTAs that sum a chunk of 32 cameras, and what every CTA
+// reads is published in kGridCopies copies.  A hop costs 0.4-1.3 us, most of
+// it the lines' way between the SMs and the two dies' L2.  Measured per PCG
+// iteration, against two grid-wide counter barriers with the values read
+// after them (which the values' copies and one read more replace): 75 cameras
+// of a walk 8.1 -> 6.7 us, 120 8.5 -> 7.1, 170 8.9 -> 7.5, 250 9.9 -> 8.0.
+// Left out, measured slower: two warps or one pipelined warp polling a slot
+// in turns (250 cameras 8.9 and 10.7 us), no copies, slots 128 bytes apart.
+// Every CTA takes the same decisions from the same values.  The arithmetic
+// is the two-kernel FP64 PCG's, operation for operation (the fixed trees of
+// kernels.cuh, k_schur.cu's product and the camera kernel's reductions), so
+// both forms give the same bits, and no result depends on how many CTAs took
+// part.
 //
 // Participation.  The CTAs that start register on a counter; the first one
 // closes the registration once every CTA of the launch has registered, or
 // after kRegisterNs (another stream's kernels may hold SMs), and the work is
 // split over the P CTAs that registered; a CTA that arrives after the
-// closing leaves at once.  So every CTA that waits at a barrier waits only
-// for CTAs that are running, whatever else the GPU is doing.  Every wait is
-// bounded (kWaitNs, about a second): a CTA whose wait runs out raises the
-// abort word, which ends every other CTA's waits; the problem's solve then
-// ends with GBA_ERR_TIMEOUT in the status word and the LM loop stops.  The
-// control words are zeroed by the camera Schur kernel K3b before each
+// closing leaves at once.  So every CTA waits only for CTAs that are running,
+// whatever else the GPU is doing.  Every wait is bounded (kWaitNs, about a
+// second): a CTA whose wait runs out raises the abort word, which ends every
+// other CTA's waits; the problem's solve then ends with GBA_ERR_TIMEOUT in
+// the status word and the LM loop stops.  The control words are zeroed, and
+// the launch's tag counted up, by the camera Schur kernel K3b before each
 // launch.
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <vector>
 
 #include "kernels.cuh"
 #include "kernels.h"
@@ -60,12 +69,11 @@ namespace {
 
 constexpr int kGThreads = kPcgGridThreads;
 constexpr int kGWarps = kGThreads / 32;
-constexpr int kGMaxOwn = 64;    // touched cameras a CTA's shared-memory layout indexes
 constexpr int kGRows = 64;      // rows of one pass of the product (tables in shared memory)
-constexpr int kGLevels = 24;    // levels of the pairwise tree (rows of up to 2^24 blocks)
+constexpr int kGSteps = 12;     // steps of the pairwise tree, two levels each (rows of up to 2^24 blocks)
 constexpr int kGBlkSlot = 96;   // threads per camera block in the update (3 warps)
 constexpr int kGBlksPerRound = kGThreads / kGBlkSlot;
-constexpr int kGPreThreads = kGThreads - 96;  // threads that prefetch while warps 0-2 decide
+constexpr int kGMaxCams = 8192;  // cameras of the touched-column bitmap
 static_assert(kGBlksPerRound >= 1 && kGThreads % 32 == 0 && kGWarps >= 4, "whole warps, at least one slot");
 static_assert(kGBlkSlot % 32 == 0, "block slots of whole warps");
 static_assert(9 * kPcgBlockCams <= kGBlkSlot, "a camera block's coordinates fit its slot");
@@ -93,8 +101,22 @@ __device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long
 __device__ __forceinline__ void st_release_u32(unsigned *p, unsigned v) {
   asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
-__device__ __forceinline__ void red_release_add_u32(unsigned *p, unsigned v) {
-  asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+
+// Publishes a value: the slot's 16 bytes as one access.
+__device__ __forceinline__ void slot_put(GridSlot *p, double v, unsigned long long tag) {
+  asm volatile("{\n\t.reg .b128 r;\n\tmov.b128 r, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], r;\n\t}" ::"l"(p),
+               "l"(__double_as_longlong(v)), "l"(tag)
+               : "memory");
+}
+__device__ __forceinline__ unsigned long long slot_get(const GridSlot *p, double &v) {
+  long long a;
+  unsigned long long b;
+  asm volatile("{\n\t.reg .b128 r;\n\tld.relaxed.gpu.global.b128 r, [%2];\n\tmov.b128 {%0, %1}, r;\n\t}"
+               : "=l"(a), "=l"(b)
+               : "l"(p)
+               : "memory");
+  v = __longlong_as_double(a);
+  return b;
 }
 
 // Raises the abort word (first one wins) and records the timeout.
@@ -103,94 +125,101 @@ __device__ void grid_abort(const DeviceBatch &B) {
     atomicExch(reinterpret_cast<unsigned *>(B.status), (unsigned)GBA_ERR_TIMEOUT);
 }
 
-// Grid-wide barrier of the P registered CTAs (generation `gen`, from 1):
-// every thread's earlier writes are ordered before thread 0's release
-// increment by the CTA barrier (causality order is transitive: CTA barrier,
-// then the gpu-scope release, the other CTA's gpu-scope acquire, its CTA
-// barrier), so no separate fence is needed on either side; after thread 0's
-// acquire wait and the CTA barrier every thread reads the other CTAs'
-// writes (with __ldcg: L2, not a stale L1 line).
-// Returns false (in every thread) when the wait ran out or was aborted.
-__device__ __forceinline__ bool grid_barrier(const DeviceBatch &B, unsigned gen, unsigned P, int *s_ok) {
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int ok = 1;
-    unsigned *bar = B.grid_ctl + kGridBar;
-    red_release_add_u32(bar, 1u);
-    const unsigned target = gen * P;
-    if (ld_acquire_u32(bar) < target) {
-      const unsigned long long t0 = global_ns();
-      unsigned n = 0;
-      while (ld_acquire_u32(bar) < target) {
-        if ((++n & 63u) == 0u) {
-          if (ld_acquire_u32(B.grid_ctl + kGridAbort) != 0u) {
-            ok = 0;
-            break;
-          }
-          if (global_ns() - t0 > kWaitNs) {
-            grid_abort(B);
-            ok = 0;
-            break;
-          }
-        }
+// Waits until the N slots of every lane with `need` carry `tag` and returns
+// their values; on a wait that ran out or was aborted sets *fail (the CTA
+// looks at it after its next barrier).  Call from a whole warp: the lanes
+// leave the loop together (lanes that left one by one would run on apart, an
+// FP64 instruction issued for each).
+template <int N>
+__device__ __forceinline__ void slots_wait(const DeviceBatch &B, const GridSlot *const (&p)[N], unsigned long long tag,
+                                           bool need, double (&v)[N], int *fail) {
+  unsigned n = 0;
+  unsigned long long t0 = 0;
+#pragma unroll
+  for (int j = 0; j < N; ++j) v[j] = 0.0;
+  for (;;) {
+    bool ok = true;
+    if (need) {
+#pragma unroll
+      for (int j = 0; j < N; ++j) ok = (slot_get(p[j], v[j]) == tag) && ok;
+    }
+    if (__all_sync(0xffffffffu, ok)) return;
+    if ((++n & 63u) == 0u) {
+      const unsigned long long now = global_ns();
+      if (t0 == 0) t0 = now;
+      if (now - t0 > kWaitNs) grid_abort(B);
+      if (__any_sync(0xffffffffu, ld_acquire_u32(B.grid_ctl + kGridAbort) != 0u)) {
+        *fail = 1;
+        return;
       }
     }
-    *s_ok = ok;
   }
-  __syncthreads();
-  return *s_ok != 0;
+}
+__device__ __forceinline__ double slot_wait(const DeviceBatch &B, const GridSlot *p, unsigned long long tag, bool need,
+                                            int *fail) {
+  const GridSlot *const a[1] = {p};
+  double v[1];
+  slots_wait<1>(B, a, tag, need, v, fail);
+  return v[0];
 }
 
 // Dynamic shared memory: the rows of the block-Jacobi inverse of the
-// update's coordinates (one row per thread), the cameras' p.q chunk sums,
-// per touched camera its first block (boff, the diagonal block last in each
-// camera's run), per touched block its column camera, its 81 values (when
-// cached) and the direction at its nine columns; for the product's pass
-// (at most kGRows rows, cap_pairs (row, block) pairs): each pair's dot and
-// (row, block), each row's first pair, the tree's additions by level.
+// update's coordinates (one row per thread), the cameras' p.q chunk sums; per
+// touched column its camera, the direction and z there; for the product's
+// pass (at most kGRows rows, cap_pairs (row, block) pairs): each pair's row
+// of S (when cached), dot and column, each row's first pair, the tree's steps.
 struct GridSmem {
-  size_t mrow, chs, boff, scol, sval, pst, pd, pinfo, ldst, roff, lbeg, total;
+  size_t mrow, chs, clist, p, zc, sval, pd, pcol, ldst, roff, total;
 };
 __host__ __device__ inline size_t grid_align(size_t x) { return (x + 15) & ~size_t(15); }
-__host__ __device__ inline GridSmem grid_smem(int n, int cap_blocks, bool cache_s, int cap_pairs) {
+__host__ __device__ inline GridSmem grid_smem(int n, int cap_cols, int cap_pairs) {
   GridSmem l;
   size_t o = 0;
   l.mrow = o, o = grid_align(o + 8 * 9 * (size_t)kGThreads);
   l.chs = o, o = grid_align(o + 8 * (size_t)((n + 31) / 32 + 1));
-  l.boff = o, o = grid_align(o + 4 * (size_t)(kGMaxOwn + 1));
-  l.scol = o, o = grid_align(o + 4 * (size_t)cap_blocks);
-  l.sval = o, o = grid_align(o + (cache_s ? 8 * 81 * (size_t)cap_blocks : 0));
-  l.pst = o, o = grid_align(o + 8 * 9 * (size_t)cap_blocks);
+  l.clist = o, o = grid_align(o + 2 * (size_t)cap_cols);
+  l.p = o, o = grid_align(o + 8 * 9 * (size_t)cap_cols);
+  l.zc = o, o = grid_align(o + 8 * 9 * (size_t)cap_cols);
+  l.sval = o, o = grid_align(o + 8 * 9 * (size_t)cap_pairs);
   l.pd = o, o = grid_align(o + 8 * (size_t)cap_pairs);
-  l.pinfo = o, o = grid_align(o + 4 * (size_t)cap_pairs);
+  l.pcol = o, o = grid_align(o + 4 * (size_t)cap_pairs);
   l.ldst = o, o = grid_align(o + 4 * (size_t)cap_pairs);
   l.roff = o, o = grid_align(o + 4 * (size_t)(kGRows + 1));
-  l.lbeg = o, o = grid_align(o + 4 * (size_t)(kGLevels + 1));
   l.total = o;
   return l;
 }
 
-// The rows of a CTA: row rho (camera rho / 9, row rho % 9 of the problem)
-// costs the camera's blocks m_c (off-diagonal + diagonal); the 9 n rows are
-// cut into P runs of about equal cost.  Rows of camera c before the cost
-// bound t: min(9, ceil((t - 9 before_c) / m_c)), 0 when t <= 9 before_c.
-__host__ __device__ inline int rows_below(long long t, long long before9, long long m) {
-  if (t <= before9) return 0;
-  const long long r = (t - before9 + m - 1) / m;
-  return r > 9 ? 9 : (int)r;
+// The units of a CTA: a camera's rows in the pairs (0,1) (2,3) (4,5) (6,7)
+// and row 8, the first level of the camera's p.q sum.  A row costs the
+// camera's blocks m (off-diagonal + diagonal), a pair 2 m; the units are cut
+// into P runs of about equal cost.  Units of a camera that start before the
+// cost bound t, the rows before the camera costing `before` in all.
+__host__ __device__ inline int units5_below(long long t, long long before, long long m) {
+  if (t <= before) return 0;
+  const long long r = (t - before + 2 * m - 1) / (2 * m);
+  return r > 5 ? 5 : (int)r;
 }
+// First row of unit u (5 per camera).
+__host__ __device__ inline int unit_row(int u) { return 9 * (u / 5) + 2 * (u % 5); }
+
+// A tree step does two levels of the pairwise tree, s and 2 s: entry i (a
+// multiple of 4 s with i + s < m) adds up to four sums, (i + i+s) +
+// (i+2s + i+3s), those that exist.
+__host__ __device__ __forceinline__ int step_entries(int m, int s) { return m > s ? (m - 1 - s) / (4 * s) + 1 : 0; }
 
 }  // namespace
 
-__global__ void __launch_bounds__(kGThreads, 1) k_pcg_grid(DeviceBatch B, int cap_blocks, int cache_s,
-                                                         int cap_pairs) {
+template <bool QUAD>
+__global__ void __launch_bounds__(kGThreads, 1) k_pcg_grid(DeviceBatch B, int cap_cols, int cap_pairs) {
   extern __shared__ __align__(16) unsigned char g_smem[];
-  __shared__ int s_ticket, s_P, s_ok, s_ra, s_rb, s_stop, s_pass_end, s_npairs, s_nlev, s_good;
-  __shared__ double sc[4], s_inv_rz;
-  __shared__ double tot3[3];
+  __shared__ int s_ticket, s_P, s_ua, s_ub, s_stop, s_pass_end, s_npairs, s_nstep, s_good, s_fail, s_ncol;
+  __shared__ unsigned cmask[kGMaxCams / 32], cpre[kGMaxCams / 32];
+  __shared__ int lbeg[kGSteps + 1];
+  __shared__ double sc[3], s_inv_rz;
   __shared__ double rv[kGThreads];  // r_{k+1} of the update's coordinates, for M r
   __shared__ double red3[kGWarps][3];
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const unsigned full = 0xffffffffu;
   LMState *L = B.lm;  // one problem
   // the same state in every CTA (written by the kernels before this one)
   if (!(L->active && L->pcg_active)) return;
@@ -226,15 +255,18 @@ __global__ void __launch_bounds__(kGThreads, 1) k_pcg_grid(DeviceBatch B, int ca
     }
     s_ticket = ticket;
     s_P = P;
-    s_ra = 0;
-    s_rb = 0;
+    s_ua = 0;
+    s_ub = 0;
+    s_fail = 0;
+    s_ncol = 0;
   }
+  for (int i = t; i < kGMaxCams / 32; i += kGThreads) cmask[i] = 0u;
   __syncthreads();
   const int w = s_ticket, P = s_P;
   if (w < 0) return;  // arrived after the closing (or the closing never came)
 
   // ---- ownership -------------------------------------------------------------
-  // product: the problem's rows in P runs of about equal cost (rows_below)
+  // product: the problem's units in P runs of about equal cost
   const int n = pi.cam_count, c0 = pi.cam_begin;
   const int r0 = B.sblk_row[c0];
   {
@@ -244,437 +276,480 @@ __global__ void __launch_bounds__(kGThreads, 1) k_pcg_grid(DeviceBatch B, int ca
     for (int c = t; c < n; c += kGThreads) {
       const long long before = (long long)(B.sblk_row[c0 + c] - r0) + c;
       const long long m = (long long)(B.sblk_row[c0 + c + 1] - B.sblk_row[c0 + c]) + 1;
-      a += rows_below(ta, 9 * before, m);
-      b += rows_below(tb, 9 * before, m);
+      a += units5_below(ta, 9 * before, m);
+      b += units5_below(tb, 9 * before, m);
     }
-    if (a) atomicAdd(&s_ra, a);
-    if (b) atomicAdd(&s_rb, b);
+    if (a) atomicAdd(&s_ua, a);
+    if (b) atomicAdd(&s_ub, b);
   }
   // update: camera blocks in P equal runs
   const int nblk = pi.cam_block_count;
-  const int kb0 = pi.cam_block_begin + (int)((long long)w * nblk / P);
-  const int kb1 = pi.cam_block_begin + (int)((long long)(w + 1) * nblk / P);
+  const int kb0 = (int)((long long)w * nblk / P), kb1 = (int)((long long)(w + 1) * nblk / P);
   __syncthreads();
-  const int ra = s_ra, rb = s_rb, own_rows = rb - ra;  // rows of the problem (local)
-  const int cA = ra / 9, cB = own_rows > 0 ? (rb - 1) / 9 : cA - 1;  // touched cameras (local)
-  const int ntc = cB - cA + 1;
+  const int ua = s_ua, nu = s_ub - ua;
+  const int ra = unit_row(ua), own_rows = nu > 0 ? unit_row(ua + nu) - ra : 0;  // rows of the problem (local)
   const double *vals = reinterpret_cast<const double *>(B.sblk_val);
   const double *Sii = reinterpret_cast<const double *>(B.cam_Sii);
-  // the touched blocks in shared memory: staged directions (and cached
-  // values) when they fit the layout, else everything from L2
-  const GridSmem lay = grid_smem(n, cap_blocks, cache_s != 0, cap_pairs);
+  const GridSmem lay = grid_smem(n, cap_cols, cap_pairs);
   double *chs = reinterpret_cast<double *>(g_smem + lay.chs);
-  int *boff = reinterpret_cast<int *>(g_smem + lay.boff);
-  int *scol = reinterpret_cast<int *>(g_smem + lay.scol);
+  unsigned short *clist = reinterpret_cast<unsigned short *>(g_smem + lay.clist);
+  double *pc = reinterpret_cast<double *>(g_smem + lay.p);
+  double *zc = reinterpret_cast<double *>(g_smem + lay.zc);
   double *sval = reinterpret_cast<double *>(g_smem + lay.sval);
-  double *pst = reinterpret_cast<double *>(g_smem + lay.pst);
   double *pd = reinterpret_cast<double *>(g_smem + lay.pd);
-  int *pinfo = reinterpret_cast<int *>(g_smem + lay.pinfo);
+  int *pcol = reinterpret_cast<int *>(g_smem + lay.pcol);
   int *ldst = reinterpret_cast<int *>(g_smem + lay.ldst);
   int *roff = reinterpret_cast<int *>(g_smem + lay.roff);
-  int *lbeg = reinterpret_cast<int *>(g_smem + lay.lbeg);
-  const int nbo = ntc > 0 ? (B.sblk_row[c0 + cB + 1] - B.sblk_row[c0 + cA]) + ntc : 0;
-  const bool staged = ntc <= kGMaxOwn && nbo <= cap_blocks;
-  const bool cached = staged && cache_s != 0;
-  if (staged) {
-    if (t <= ntc) boff[t] = B.sblk_row[c0 + cA + t] - B.sblk_row[c0 + cA] + t;
-    __syncthreads();
-    for (int lc = 0; lc < ntc; ++lc) {
-      const int c = c0 + cA + lc;
-      const int rr0 = B.sblk_row[c], nb = B.sblk_row[c + 1] - rr0, b0 = boff[lc];
-      for (int v = t; v <= nb; v += kGThreads) scol[b0 + v] = v < nb ? B.sblk_col[rr0 + v] : c;
-      if (cached)
-        for (int e = t; e < 81 * (nb + 1); e += kGThreads) {
-          const int v = e / 81, el = e - 81 * v;
-          sval[81 * (size_t)(b0 + v) + el] = v < nb ? vals[81 * (size_t)(rr0 + v) + el] : Sii[81 * (size_t)c + el];
-        }
-    }
-    __syncthreads();
-  }
-  // The product's pass over local rows [rl0, s_pass_end): at most kGRows rows
-  // and cap_pairs (row, block) pairs; its tables: each row's first pair
-  // (roff), each pair's (row, block) (pinfo), the tree's additions of each
-  // level (their destinations, ldst[lbeg[L] ..]).
+  // the slots' two sets (by iteration parity): per row q, per coordinate z
+  // and p, per unit p.q (by unit of the camera), and in kGridCopies copies
+  // per chunk its p.q and per block its three sums
+  const int nch = (n + 31) / 32;
+  const size_t n9 = 9 * (size_t)n;
+  const size_t set = 3 * n9 + 5 * (size_t)n + kGridCopies * (3 * (size_t)nblk + (size_t)nch);
+  GridSlot *const sl_q = B.grid_slots, *const sl_z = sl_q + n9, *const sl_p = sl_z + n9, *const sl_pq = sl_p + n9,
+                  *const sl_c = sl_pq + 5 * (size_t)n, *const sl_b = sl_c + kGridCopies * (size_t)nch;
+  const int copy = w % kGridCopies;  // the copy this CTA reads
+  // the chunks whose p.q this CTA sums
+  const int ch0 = (int)((long long)w * nch / P), ch1 = (int)((long long)(w + 1) * nch / P);
+  const unsigned long long launch_tag = (unsigned long long)B.grid_ctl[kGridLaunch] << 32;
+  // (the failure test waits for a tag that nothing writes)
+  const unsigned long long miss = B.opt.grid_wait_test ? 1ull << 31 : 0ull;
+
   auto row_m = [&](int rl) -> int {
     const int c = c0 + (ra + rl) / 9;
     return B.sblk_row[c + 1] - B.sblk_row[c] + 1;
   };
+  // The product's pass over local rows [rl0, s_pass_end): whole units, at
+  // most kGRows rows and cap_pairs (row, block) pairs; its tables: each row's
+  // first pair (roff), each pair's column camera (pcol), the tree's steps
+  // (ldst[lbeg[s] ..]: the first sum, and how many there are).
   auto build_pass = [&](int rl0) {
     if (t == 0) {
       int rl = rl0, np = 0, mx = 1;
       roff[0] = 0;
-      while (rl < own_rows && rl - rl0 < kGRows) {
-        const int m = row_m(rl);
-        if (rl > rl0 && np + m > cap_pairs) break;
-        np += m;
+      while (rl < own_rows) {
+        const int rows = (ra + rl) % 9 == 8 ? 1 : 2, m = row_m(rl);
+        if (rl > rl0 && (np + rows * m > cap_pairs || rl + rows - rl0 > kGRows)) break;
+        for (int r = 0; r < rows; ++r) np += m, ++rl, roff[rl - rl0] = np;
         mx = max(mx, m);
-        roff[rl - rl0 + 1] = np;
-        ++rl;
       }
-      int nl = 0;
-      while ((1 << nl) < mx) ++nl;
-      int o = 0;
-      for (int L2 = 0; L2 < nl; ++L2) {
-        lbeg[L2] = o;
-        for (int j = 0; j < rl - rl0; ++j) o += tree_adds(roff[j + 1] - roff[j], 1 << L2);
+      int ns = 0, o = 0;
+      for (int s = 1; s < mx; s <<= 2, ++ns) {
+        lbeg[ns] = o;
+        for (int j = 0; j < rl - rl0; ++j) o += step_entries(roff[j + 1] - roff[j], s);
       }
-      lbeg[nl] = o;
-      s_pass_end = rl, s_npairs = np, s_nlev = nl;
+      lbeg[ns] = o;
+      s_pass_end = rl, s_npairs = np, s_nstep = ns;
     }
     __syncthreads();
-    const int nr = s_pass_end - rl0, nl = s_nlev;
-    for (int j = 0; j < nr; ++j)
-      for (int v = t; v < roff[j + 1] - roff[j]; v += kGThreads) pinfo[roff[j] + v] = (j << 20) | v;
-    for (int L2 = 0; L2 < nl; ++L2) {
-      const int sp = 1 << L2, base = lbeg[L2], cnt = lbeg[L2 + 1] - base;
+    const int nr = s_pass_end - rl0, ns = s_nstep;
+    for (int j = warp; j < nr; j += kGWarps) {
+      const int c = (ra + rl0 + j) / 9, rr0 = B.sblk_row[c0 + c], m = roff[j + 1] - roff[j];
+      for (int v = lane; v < m; v += 32) pcol[roff[j] + v] = v < m - 1 ? B.sblk_col[rr0 + v] - c0 : c;
+    }
+    for (int s2 = 0; s2 < ns; ++s2) {
+      const int s = 1 << (2 * s2), base = lbeg[s2], cnt = lbeg[s2 + 1] - base;
       for (int kk = t; kk < cnt; kk += kGThreads) {
         int j = 0, acc = 0;
         for (;;) {
-          const int a = tree_adds(roff[j + 1] - roff[j], sp);
+          const int a = step_entries(roff[j + 1] - roff[j], s);
           if (kk < acc + a) break;
           acc += a;
           ++j;
         }
-        ldst[base + kk] = roff[j] + 2 * sp * (kk - acc);
+        const int i = 4 * s * (kk - acc), m = roff[j + 1] - roff[j];
+        ldst[base + kk] = (roff[j] + i) | (i + 3 * s < m ? 2 : i + 2 * s < m ? 1 : 0) << 28;
       }
     }
     __syncthreads();
   };
-  bool one_pass = true;
+  bool one_pass = true, staged = false;
+  int ncol = 0;
   if (own_rows > 0) {
     build_pass(0);
     one_pass = s_pass_end == own_rows;
+    if (one_pass) {
+      // the touched columns, in camera order, and the pairs' indexes among them
+      const int np = s_npairs;
+      for (int e = t; e < np; e += kGThreads) atomicOr(&cmask[pcol[e] >> 5], 1u << (pcol[e] & 31));
+      __syncthreads();
+      if (t == 0) {
+        int o = 0;
+        for (int i = 0; i < (n + 31) / 32; ++i) cpre[i] = o, o += __popc(cmask[i]);
+        s_ncol = o;
+      }
+      __syncthreads();
+      ncol = s_ncol;
+      staged = ncol <= cap_cols;
+      if (staged) {
+        for (int c = t; c < n; c += kGThreads) {
+          const unsigned bit = 1u << (c & 31);
+          if (cmask[c >> 5] & bit) clist[cpre[c >> 5] + __popc(cmask[c >> 5] & (bit - 1u))] = (unsigned short)c;
+        }
+        for (int j = warp; j < own_rows; j += kGWarps) {
+          const int c = (ra + j) / 9, q = ra + j - 9 * c, rr0 = B.sblk_row[c0 + c], m = roff[j + 1] - roff[j];
+          for (int i = lane; i < 9 * m; i += 32) {
+            const int v = i / 9, cc = i - 9 * v;
+            sval[9 * roff[j] + i] = v < m - 1 ? vals[81 * (size_t)(rr0 + v) + 9 * q + cc] : Sii[81 * (size_t)(c0 + c) + 9 * q + cc];
+          }
+        }
+        __syncthreads();
+        for (int e = t; e < np; e += kGThreads) {
+          const int c = pcol[e];
+          pcol[e] = cpre[c >> 5] + __popc(cmask[c >> 5] & ((1u << (c & 31)) - 1u));
+        }
+        for (int e = t; e < 9 * ncol; e += kGThreads) pc[e] = B.pcg_z[9 * (size_t)(c0 + clist[e / 9]) + e % 9];  // p_0 = z_0
+      }
+    }
+  }
+
+  // the row that this thread publishes, when the CTA's rows are one pass: its
+  // dot's and its own coordinates' addresses
+  const double *w_d0 = pd, *w_d1 = pd, *w_p = pc;
+  bool w_in = false, w_even = false, w_pair = false;
+  int w_row = 0, w_unit = 0;
+  // and its additions in the tree's steps (kGKeep of them at most, one entry
+  // per thread in each; else from the tables)
+  constexpr int kGKeep = 4;
+  int w_tree[kGKeep];
+  bool keep_tree = staged && s_nstep <= kGKeep;
+  if (staged) {
+    __syncthreads();
+#pragma unroll
+    for (int s2 = 0; s2 < kGKeep; ++s2) {
+      w_tree[s2] = -1;
+      if (s2 < s_nstep) {
+        const int kk = lbeg[s2] + t;
+        if (kk < lbeg[s2 + 1]) w_tree[s2] = ldst[kk];
+        keep_tree = keep_tree && lbeg[s2 + 1] - lbeg[s2] <= kGThreads;
+      }
+    }
+    w_in = t < own_rows;
+    const int tr = min(t, own_rows - 1), cl = (ra + tr) / 9, q = ra + tr - 9 * cl;
+    w_even = w_in && (q & 1) == 0, w_pair = w_even && q < 8;
+    w_row = ra + tr, w_unit = (q >> 1) * n + cl;
+    w_d0 = pd + roff[tr], w_d1 = pd + roff[w_pair ? tr + 1 : tr];
+    w_p = pc + 9 * pcol[roff[tr + 1] - 1] + q;
   }
 
   const DeviceOptions &o = B.opt;
-  // the direction of iteration k lives in pbuf(k): pcg_p for even k, pcg_p2 for odd k
-  auto pbuf = [&](int kk) -> double * { return (kk & 1) ? B.pcg_p2 : B.pcg_p; };
   double rz_k = L->rz, beta = L->beta, q0 = L->q0;
   double last_rr = L->rr, last_pq = L->pq;
   const double lim = o.pcg_tolerance * L->r0_norm;
+  const long long lim2_bits = __double_as_longlong(lim * lim);
   int k = 0;
   bool linear_ok = true, aborted = false;
-  unsigned gen = 0;
-  // CTAs a barrier waits for (one more under the wait-runs-out test)
-  const unsigned bar_n = (unsigned)P + (B.opt.grid_wait_test ? 1u : 0u);
 
-  // the update's coordinate of this thread (the camera kernel's lead
-  // threads: coordinate m of a camera block in the lanes of 3 warps); with
-  // at most kGBlksPerRound owned blocks its state stays in registers
+  // the update's coordinate of this thread (coordinate m of a camera block
+  // in the lanes of 3 warps); with at most kGBlksPerRound owned blocks its
+  // state stays in registers, else in global memory
   const bool one_round = kb1 - kb0 <= kGBlksPerRound;
-  const int u_slot = t / kGBlkSlot, u_m = t - kGBlkSlot * u_slot;
-  const int u_lc = u_m / 9, u_q = u_m - 9 * u_lc;
+  const int u_slot = t / kGBlkSlot, u_m = t - kGBlkSlot * u_slot, u_q = u_m % 9;
   double ux = 0.0, ur = 0.0, uz = 0.0, uv = 0.0, up = 0.0;
   double *umrow = reinterpret_cast<double *>(g_smem + lay.mrow) + 9 * t;
-  bool u_in = false, u_lead = false;
-  size_t u_i = 0;
-  if (one_round) {
-    const int blk = kb0 + u_slot;
-    u_in = u_slot < kGBlksPerRound && blk < kb1;
-    int4 cbk = make_int4(0, 0, 0, 0);
-    if (u_in) cbk = B.camblk[blk];
-    u_lead = u_in && u_m < 9 * kPcgBlockCams && u_lc < cbk.z;
-    u_i = 9 * (size_t)(cbk.y + (u_lead ? u_lc : 0)) + u_q;
-    if (u_lead) {
-      const double *M = B.cam_Minv + 9 * u_i;  // row u_q of the camera's block: 81 c + 9 q = 9 i
+  auto load_coordinate = [&](int blk, bool first) -> bool {  // of block blk; true in the threads that hold one
+    const bool lead = u_slot < kGBlksPerRound && blk < kb1 && u_m < 9 * min(kPcgBlockCams, n - kPcgBlockCams * blk);
+    if (lead) {
+      const size_t i = 9 * (size_t)(c0 + kPcgBlockCams * blk) + u_m;
 #pragma unroll
-      for (int kk = 0; kk < 9; ++kk) umrow[kk] = M[kk];
-      ux = B.pcg_x[u_i];
-      ur = B.pcg_r[u_i];
-      uz = B.pcg_z[u_i];
-      uv = B.pcg_v[u_i];
+      for (int kk = 0; kk < 9; ++kk) umrow[kk] = B.cam_Minv[9 * i + kk];  // row u_q of the camera's block
+      ux = B.pcg_x[i], ur = B.pcg_r[i], uz = B.pcg_z[i], uv = B.pcg_v[i];
+      up = first ? 0.0 : B.pcg_p[i];
     }
-  }
-  // the staged direction of the touched blocks' columns: p_0 = z_0
-  if (staged) {
-    for (int e = t; e < 9 * nbo; e += kGThreads) {
-      const int bl = e / 9, cc = e - 9 * bl;
-      pst[e] = __ldcg(B.pcg_z + 9 * (size_t)scol[bl] + cc);
-    }
-  }
+    return lead;
+  };
+  bool u_lead = one_round && load_coordinate(kb0 + u_slot, true);
   __syncthreads();
   for (;;) {
-    // ---- A. q = S p_k for the owned rows, each row's p_i q_i ---------------
-    const double *pprev = pbuf(k + 1);  // p_{k-1}
-    auto pdir = [&](size_t idx) -> double {
-      const double z = __ldcg(B.pcg_z + idx);
-      if (k == 0) return z;
-      return fma(beta, __ldcg(pprev + idx), z);
-    };
+    const unsigned long long tag = launch_tag | (unsigned)(k + 1);
+    const unsigned long long wait_tag = tag ^ miss;
+    const size_t so = (k & 1) ? set : 0;  // this iteration's slots
+    // ---- the owned blocks' p_k, published for the CTAs that do not hold the
+    // direction themselves (more rows or columns than the layout holds)
+    if (one_round) {
+      if (u_lead) {
+        up = k == 0 ? uz : fma(beta, up, uz);
+        slot_put(sl_p + so + kPcgBlockCams * 9 * (size_t)(kb0 + u_slot) + u_m, up, tag);
+      }
+    } else {
+      for (int kb = kb0; kb < kb1; kb += kGBlksPerRound)
+        if (load_coordinate(kb + u_slot, k == 0)) {
+          const size_t i = kPcgBlockCams * 9 * (size_t)(kb + u_slot) + u_m;
+          up = k == 0 ? uz : fma(beta, up, uz);
+          B.pcg_p[9 * (size_t)c0 + i] = up;
+          slot_put(sl_p + so + i, up, tag);
+        }
+    }
+    // ---- A. q = S p_k for the owned rows, each unit's p_i q_i ---------------
     for (int rl0 = 0; rl0 < own_rows;) {
       if (!one_pass) build_pass(rl0);
-      const int pend = one_pass ? own_rows : s_pass_end, np = s_npairs, nl = s_nlev;
+      const int pend = one_pass ? own_rows : s_pass_end, np = s_npairs, ns = s_nstep;
       // the pairs' block dots (nine-column FMA chains)
-      for (int e = t; e < np; e += kGThreads) {
-        const int j = pinfo[e] >> 20, v = pinfo[e] & 0xfffff;
-        const int rho = ra + rl0 + j, cl = rho / 9, q = rho - 9 * cl, c = c0 + cl;
-        double d = 0.0;
-        if (staged) {
-          const int b0 = boff[cl - cA], nb = boff[cl - cA + 1] - b0 - 1;
-          const double *row = cached ? sval + 81 * (size_t)(b0 + v) + 9 * q
-                                     : (v < nb ? vals + 81 * (size_t)(B.sblk_row[c] + v) : Sii + 81 * (size_t)c) + 9 * q;
-          const double *pp = pst + 9 * (b0 + v);
+      if (staged) {
+        for (int e = t; e < np; e += kGThreads) {
+          const double *row = sval + 9 * e, *pp = pc + 9 * pcol[e];
+          double d = 0.0;
 #pragma unroll
           for (int cc = 0; cc < 9; ++cc) d = fma(row[cc], pp[cc], d);
-        } else {
-          const int rr0 = B.sblk_row[c], nb = B.sblk_row[c + 1] - rr0;
-          const double *row = (v < nb ? vals + 81 * (size_t)(rr0 + v) : Sii + 81 * (size_t)c) + 9 * q;
-          const int col = v < nb ? B.sblk_col[rr0 + v] : c;
-#pragma unroll
-          for (int cc = 0; cc < 9; ++cc) d = fma(row[cc], pdir(9 * (size_t)col + cc), d);
+          pd[e] = d;
         }
-        pd[e] = d;
+      } else {
+        for (int j = warp; j < pend - rl0; j += kGWarps) {
+          const int rho = ra + rl0 + j, cl = rho / 9, q = rho - 9 * cl, rr0 = B.sblk_row[c0 + cl];
+          const int m = roff[j + 1] - roff[j];
+          for (int v0 = 0; v0 < m; v0 += 32) {
+            const int v = min(v0 + lane, m - 1);
+            const double *row = (v < m - 1 ? vals + 81 * (size_t)(rr0 + v) : Sii + 81 * (size_t)(c0 + cl)) + 9 * q;
+            const GridSlot *ps = sl_p + so + 9 * (size_t)pcol[roff[j] + v];
+            double d = 0.0;
+            for (int cc = 0; cc < 9; ++cc) d = fma(row[cc], slot_wait(B, ps + cc, wait_tag, true, &s_fail), d);
+            if (v0 + lane < m) pd[roff[j] + v] = d;
+          }
+        }
       }
       __syncthreads();
-      // each row's pairwise tree, level by level
-      for (int L2 = 0; L2 < nl; ++L2) {
-        const int sp = 1 << L2;
-        for (int kk = lbeg[L2] + t; kk < lbeg[L2 + 1]; kk += kGThreads) {
-          const int dst = ldst[kk];
-          pd[dst] += pd[dst + sp];
+      // each row's pairwise tree, two levels a step
+      auto step = [&](int e, int sp) {
+        const int more = e >> 28;
+        double *d = pd + (e & 0xfffffff);
+        double x = d[0] + d[sp];
+        if (more > 0) {
+          double y = d[2 * sp];
+          if (more > 1) y += d[3 * sp];
+          x += y;
         }
-        __syncthreads();
+        d[0] = x;
+      };
+      if (keep_tree) {
+#pragma unroll
+        for (int s2 = 0; s2 < kGKeep; ++s2)
+          if (s2 < ns) {
+            if (w_tree[s2] >= 0) step(w_tree[s2], 1 << (2 * s2));
+            __syncthreads();
+          }
+      } else {
+        for (int s2 = 0; s2 < ns; ++s2) {
+          for (int kk = lbeg[s2] + t; kk < lbeg[s2 + 1]; kk += kGThreads) step(ldst[kk], 1 << (2 * s2));
+          __syncthreads();
+        }
       }
-      if (t < pend - rl0) {
-        const int rho = ra + rl0 + t, cl = rho / 9, q = rho - 9 * cl, c = c0 + cl;
-        const size_t i = 9 * (size_t)c + q;
-        const double qv = pd[roff[t]];
-        // p_k at the row's own coordinate: the diagonal block's column
-        const double pk = staged ? pst[9 * (boff[cl - cA + 1] - 1) + q] : pdir(i);
-        B.pcg_q[i] = qv;
-        B.pq_row[(size_t)q * n + cl] = pk * qv;  // row-major by row index: a camera's rows n apart
+      // q_i per row and p_i q_i per unit (a thread each)
+      if (staged) {
+        if (32 * warp < own_rows) {
+          const double qv = *w_d0, qv1 = *w_d1, p0 = w_p[0], p1 = w_pair ? w_p[1] : 0.0;
+          if (w_in) slot_put(sl_q + so + w_row, qv, tag);
+          const double y0 = __dmul_rn(p0, qv), y1 = __dadd_rn(y0, __dmul_rn(p1, qv1));
+          if (w_even) slot_put(sl_pq + so + w_unit, w_pair ? y1 : y0, tag);
+        }
+      } else if (t < ((pend - rl0 + 31) & ~31)) {  // (whole warps)
+        const bool in = t < pend - rl0;
+        const int tr = min(t, pend - rl0 - 1);
+        const int rho = ra + rl0 + tr, cl = rho / 9, q = rho - 9 * cl;
+        const bool even = in && (q & 1) == 0, pair = even && q < 8;
+        const double qv = pd[roff[tr]], qv1 = pair ? pd[roff[tr + 1]] : 0.0;
+        if (in) slot_put(sl_q + so + rho, qv, tag);
+        // p_k at the unit's own coordinates: the diagonal block's column
+        const double p0 = slot_wait(B, sl_p + so + rho, wait_tag, even, &s_fail);
+        const double p1 = slot_wait(B, sl_p + so + rho + (pair ? 1 : 0), wait_tag, pair, &s_fail);
+        const double y0 = __dmul_rn(p0, qv), y1 = __dadd_rn(y0, __dmul_rn(p1, qv1));
+        if (even) slot_put(sl_pq + so + (size_t)(q >> 1) * n + cl, pair ? y1 : y0, tag);
       }
-      __syncthreads();  // pd and the pass tables are used again
+      if (!one_pass) __syncthreads();  // pd and the pass tables are used again
       rl0 = pend;
     }
-    if (!grid_barrier(B, ++gen, bar_n, &s_ok)) {
+    // ---- B. the p.q of the CTA's chunks of 32 cameras, each camera's from
+    // its five values (the rest of sum9_tree), then a butterfly; published.
+    // The chunks from the last warp down: the first warps hold the update -----
+    for (int j = ch0 + kGWarps - 1 - warp; j < ch1; j += kGWarps) {
+      const int c = 32 * j + lane;
+      const GridSlot *const pq0 = sl_pq + so + min(c, n - 1);
+      const GridSlot *const a[5] = {pq0, pq0 + n, pq0 + 2 * (size_t)n, pq0 + 3 * (size_t)n, pq0 + 4 * (size_t)n};
+      double y[5];
+      slots_wait<5>(B, a, wait_tag, c < n, y, &s_fail);
+      double x = ((y[0] + y[1]) + (y[2] + y[3])) + y[4];  // (0 beyond the problem's cameras)
+      x = warp_sum(x);
+      if (lane < kGridCopies) slot_put(sl_c + so + (size_t)lane * nch + j, x, tag);
+    }
+    // the owned coordinates' q; every CTA: the chunks' sum (the pairwise
+    // tree: cta_chunked_sum's order), alpha; the update
+    double qv = 0.0;
+    if (one_round && __any_sync(full, u_lead))
+      qv = slot_wait(B, sl_q + so + (u_lead ? kPcgBlockCams * 9 * (size_t)(kb0 + u_slot) + u_m : 0), wait_tag, u_lead, &s_fail);
+    if (nch > 32) {
+      for (int j0 = 32 * warp; j0 < nch; j0 += kGThreads) {
+        const int j = min(j0 + lane, nch - 1);
+        chs[j] = slot_wait(B, sl_c + so + (size_t)copy * nch + j, wait_tag, true, &s_fail);
+      }
+      __syncthreads();
+      cta_pairwise_tree(chs, nch);
+    }
+    if (warp == 0) {
+      double s2;
+      if (nch <= 32) {  // the tree by one warp's shuffles
+        s2 = slot_wait(B, sl_c + so + (size_t)copy * nch + min(lane, nch - 1), wait_tag, lane < nch, &s_fail);
+        for (int s = 1; s < nch; s <<= 1) {
+          const double y = __shfl_down_sync(full, s2, s);
+          s2 += (lane & (2 * s - 1)) == 0 && lane + s < nch ? y : 0.0;
+        }
+      } else {
+        s2 = chs[0];
+      }
+      if (lane == 0) {
+        const long long b2 = __double_as_longlong(s2);
+        sc[0] = s2, sc[1] = rz_k * recip_nr(s2);
+        s_good = b2 > 0 && b2 < 0x7ff0000000000000LL;  // positive and finite
+      }
+    } else if (t == kGThreads - 32) {
+      s_inv_rz = recip_nr(rz_k);  // for beta, off the deciding warp's chain
+    }
+    __syncthreads();
+    if (s_fail) {
       aborted = true;
       break;
     }
-    // ---- B. each camera's p.q (sum9_tree), their sum (chunks of 32 and the
-    // pairwise tree: cta_chunked_sum's order), alpha; the update ---------------
-    double qv_pre = 0.0, up_k = 0.0;
-    if (one_round && u_lead) {
-      qv_pre = __ldcg(B.pcg_q + u_i);         // in flight while the cameras are summed
-      up_k = k == 0 ? uz : fma(beta, up, uz);  // p_k from p_{k-1} (alpha not needed)
-    }
-    {
-      const int nch = (n + 31) / 32;
-      for (int j = warp; j < nch; j += kGWarps) {
-        const int c = 32 * j + lane;
-        double x = 0.0;
-        if (c < n) {
-          double x9[9];  // coalesced over the lanes' cameras
-#pragma unroll
-          for (int r = 0; r < 9; ++r) x9[r] = __ldcg(B.pq_row + (size_t)r * n + c);
-          x = sum9_tree(x9);
-        }
-        x = warp_sum(x);
-        if (lane == 0) chs[j] = x;
-      }
-      if (nch == 0 && t == 0) chs[0] = 0.0;
-      __syncthreads();
-      if (nch <= 32) {  // the tree by one warp's shuffles (no barrier per level)
-        if (warp == 0) {
-          const double s2 = warp_pairwise_tree(lane < nch ? chs[lane] : 0.0, nch);
-          if (lane == 0) sc[0] = s2, sc[1] = rz_k * recip_nr(s2), s_good = s2 > 0.0 && isfinite(s2);
-        }
-      } else {
-        cta_pairwise_tree(chs, nch);
-        if (t == 0) {
-          const double s2 = chs[0];
-          sc[0] = s2;
-          sc[1] = rz_k * recip_nr(s2);
-          s_good = s2 > 0.0 && isfinite(s2);
-        }
-      }
-      __syncthreads();
-    }
     const double pq = sc[0], alpha = sc[1];
-    // pq > 0 and finite, tested once (else S is not positive definite along
-    // p_k): an FP64 comparison in every warp would queue on the FP64 pipes
-    const bool good = s_good != 0;
-    if (!good) {                                  // the PCG ends with x_k
+    if (s_good == 0) {  // S is not positive definite along p_k: the PCG ends with x_k
       if (k == 0) linear_ok = false;
       break;
     }
-    if (one_round) {
-      if (u_lead) {
-        up = up_k;
-        ux = fma(alpha, up, ux);
-        ur = fma(-alpha, qv_pre, ur);
+    for (int kb = kb0; kb < kb1; kb += kGBlksPerRound) {
+      const int blk = kb + u_slot;
+      const bool in = u_slot < kGBlksPerRound && blk < kb1;  // uniform over the slot's three warps
+      const int coords = in ? 9 * min(kPcgBlockCams, n - kPcgBlockCams * blk) : 0;
+      const size_t i = kPcgBlockCams * 9 * (size_t)blk + u_m;
+      bool lead = u_lead;
+      if (!one_round) {
+        lead = load_coordinate(blk, false);
+        qv = slot_wait(B, sl_q + so + (lead ? i : 0), wait_tag, lead, &s_fail);
+      }
+      if (lead) {
+        ur = fma(-alpha, qv, ur);
         rv[t] = ur;
       }
       __syncthreads();
-      if (u_in) {
+      if (in && 32 * (warp - 3 * u_slot) < coords) {
         double rz = 0.0, rr = 0.0, qx = 0.0;
-        if (u_lead) {
+        if (lead) {
           double zz = 0;
 #pragma unroll
           for (int kk = 0; kk < 9; ++kk) zz += umrow[kk] * rv[t - u_q + kk];
           uz = zz;
-          pbuf(k)[u_i] = up;
-          B.pcg_z[u_i] = uz;
-          rz = ur * uz, rr = ur * ur, qx = ux * (uv + ur);
+          slot_put(sl_z + so + i, uz, tag);
+          rz = ur * uz, rr = ur * ur;
         }
-        // the block's r.z, r.r, x.(v + r): butterflies in its three warps,
-        // then the warps in order
-        warp_sum3(rz, rr, qx);
-        if (lane == 0) red3[warp][0] = rz, red3[warp][1] = rr, red3[warp][2] = qx;
-      }
-      __syncthreads();
-      if (u_m < 3 && u_in) {
-        double b = 0.0;
-        for (int ww = 0; ww < 3; ++ww) b += red3[3 * u_slot + ww][u_m];
-        B.blk_red[3 * (size_t)(kb0 + u_slot) + u_m] = b;
-      }
-    } else {
-      // more owned blocks than one round: the state from L2, round by round
-      for (int kb = kb0; kb < kb1; kb += kGBlksPerRound) {
-        const int slot = u_slot, m = u_m;
-        const int blk = kb + slot;
-        const bool in = slot < kGBlksPerRound && blk < kb1;  // uniform over the slot's three warps
-        int4 cbk = make_int4(0, 0, 0, 0);
-        if (in) cbk = B.camblk[blk];
-        const int lc = u_lc, q = u_q;
-        const bool lead = in && m < 9 * kPcgBlockCams && lc < cbk.z;
-        const int c = cbk.y + (lead ? lc : 0);
-        const size_t i = 9 * (size_t)c + q;
-        double x = 0.0, r = 0.0, z = 0.0, v = 0.0, pp = 0.0;
-        if (lead) {
-          const double *M = B.cam_Minv + 81 * (size_t)c + 9 * q;
-#pragma unroll
-          for (int kk = 0; kk < 9; ++kk) umrow[kk] = M[kk];
-          x = B.pcg_x[i];
-          r = B.pcg_r[i];
-          z = B.pcg_z[i];
-          v = B.pcg_v[i];
-          pp = k == 0 ? z : fma(beta, __ldcg(pprev + i), z);
-          const double qv = __ldcg(B.pcg_q + i);
-          x = fma(alpha, pp, x);
-          r = fma(-alpha, qv, r);
-          rv[t] = r;
-        }
-        __syncthreads();
-        if (in) {
-          double rz = 0.0, rr = 0.0, qx = 0.0;
+        if (QUAD) {
           if (lead) {
-            double zz = 0;
-#pragma unroll
-            for (int kk = 0; kk < 9; ++kk) zz += umrow[kk] * rv[t - q + kk];
-            z = zz;
-            pbuf(k)[i] = pp;
-            B.pcg_x[i] = x;
-            B.pcg_r[i] = r;
-            B.pcg_z[i] = z;
-            rz = r * z, rr = r * r, qx = x * (v + r);
+            ux = fma(alpha, up, ux);
+            qx = ux * (uv + ur);
           }
           warp_sum3(rz, rr, qx);
           if (lane == 0) red3[warp][0] = rz, red3[warp][1] = rr, red3[warp][2] = qx;
-        }
-        __syncthreads();
-        if (m < 3 && in) {
-          double b = 0.0;
-          for (int ww = 0; ww < 3; ++ww) b += red3[3 * slot + ww][m];
-          B.blk_red[3 * (size_t)blk + m] = b;
-        }
-        __syncthreads();
-      }
-    }
-    if (!grid_barrier(B, ++gen, bar_n, &s_ok)) {
-      aborted = true;
-      break;
-    }
-    // ---- C. the stopping test on (x_{k+1}, r_{k+1}) and beta_{k+1}: warp j < 3
-    // sums quantity j over the blocks (the camera kernel's order), while the
-    // other warps load z_{k+1} and p_k of the staged columns ------------------
-    constexpr int kPre = 2;
-    double zpre[kPre], ppre[kPre];
-    if (warp < 3) {
-      double a = 0.0;
-      for (int bb = lane; bb < nblk; bb += 32) a += __ldcg(B.blk_red + 3 * (size_t)(pi.cam_block_begin + bb) + warp);
-      a = warp_sum(a);
-      if (lane == 0) tot3[warp] = a;
-    } else {
-      if (staged) {
-        const double *pkb = pbuf(k);
-#pragma unroll
-        for (int u = 0; u < kPre; ++u) {
-          const int e = (t - 96) + u * kGPreThreads;
-          zpre[u] = ppre[u] = 0.0;
-          if (e < 9 * nbo) {
-            const size_t gi = 9 * (size_t)scol[e / 9] + e % 9;
-            zpre[u] = __ldcg(B.pcg_z + gi);
-            ppre[u] = __ldcg(pkb + gi);
-          }
+        } else {
+          // both butterflies at once: lanes 0-15 end with r.z, 16-31 with r.r
+          const bool lo = lane < 16;
+          double v = (lo ? rz : rr) + __shfl_xor_sync(full, lo ? rr : rz, 16);
+          v += __shfl_xor_sync(full, v, 8);
+          v += __shfl_xor_sync(full, v, 4);
+          v += __shfl_xor_sync(full, v, 2);
+          v += __shfl_xor_sync(full, v, 1);
+          if ((lane & 15) == 0) red3[warp][lane >> 4] = v;
         }
       }
-      // 1 / r_k.z_k for beta, off the deciding warps' dependent chain
-      if (t == 96) s_inv_rz = recip_nr(rz_k);
+      __syncthreads();
+      // the block's sums, its warps in order (a warp without coordinates adds nothing)
+      if (in && warp == 3 * u_slot) {
+        constexpr int kSums = QUAD ? 3 : 2;
+        const int u = lane % kSums, cp = lane / kSums;
+        double b = red3[3 * u_slot][u];
+        if (coords > 32) b += red3[3 * u_slot + 1][u];
+        if (coords > 64) b += red3[3 * u_slot + 2][u];
+        if (cp < kGridCopies) slot_put(sl_b + so + (size_t)(3 * cp + u) * nblk + blk, b, tag);
+      }
+      if (lead && !QUAD) ux = fma(alpha, up, ux);
+      if (!one_round) {
+        if (lead) {
+          const size_t g = 9 * (size_t)c0 + i;
+          B.pcg_x[g] = ux, B.pcg_r[g] = ur, B.pcg_z[g] = uz;
+        }
+        __syncthreads();  // rv and red3 are used again
+      }
     }
-    __syncthreads();
-    if (t == 0) {
-      const double rz1 = tot3[0], rr1 = tot3[1], qk = -tot3[2];  // Q(x) = x'Sx - 2 v'x = -x.(v + r)
+    // ---- C. the stopping test on (x_{k+1}, r_{k+1}) and beta_{k+1} in warp 0,
+    // from the blocks' values (the camera kernel's order), while the other
+    // warps fetch z_{k+1} of the touched columns --------------------------------
+    if (warp == 0) {
+      double a = 0.0, b = 0.0, x = 0.0;
+      for (int b0 = 0; b0 < nblk; b0 += 32) {
+        const int bb = b0 + lane;
+        const GridSlot *const p3 = sl_b + so + 3 * (size_t)copy * nblk + min(bb, nblk - 1);
+        constexpr int N = QUAD ? 3 : 2;
+        const GridSlot *s3[3] = {p3, p3 + nblk, p3 + 2 * (size_t)nblk};
+        const GridSlot *const(&sN)[N] = *reinterpret_cast<const GridSlot *const(*)[N]>(&s3);
+        double y[N];
+        slots_wait<N>(B, sN, wait_tag, bb < nblk, y, &s_fail);
+        if (b0 == 0)
+          a = y[0], b = y[1], x = QUAD ? y[N - 1] : 0.0;
+        else if (bb < nblk)
+          a += y[0], b += y[1], x += QUAD ? y[N - 1] : 0.0;
+      }
+      // the blocks' owners published z before their sums: the other warps may
+      // read it now (polling it from the start would slow the sums' way)
+      asm volatile("bar.arrive 1, %0;" ::"n"(kGThreads) : "memory");
+      const bool lo = lane < 16;
+      double v = (lo ? a : b) + __shfl_xor_sync(full, lo ? b : a, 16);
+      for (int s = nblk > 8 ? 8 : nblk > 4 ? 4 : nblk > 2 ? 2 : nblk > 1 ? 1 : 0; s > 0; s >>= 1)
+        v += __shfl_xor_sync(full, v, s);  // (a level that would only add zeros is left out)
+      const double rz1 = __shfl_sync(full, v, 0), rr1 = __shfl_sync(full, v, 16);
       const int k1 = k + 1;
       bool stop = false;
-      if (o.pcg_criterion == GBA_PCG_QUADRATIC_MODEL) {
+      if (QUAD) {
+        const double qk = -warp_sum(x);  // Q(x) = x'Sx - 2 v'x = -x.(v + r)
         const double lhs = k1 * (qk - q0), rhs = o.eta * qk;
         const bool below = qk > 0.0 ? lhs < rhs : (qk < 0.0 ? lhs > rhs : q0 > 0.0);
         if (below && k1 >= o.min_pcg_iterations) stop = true;
-      } else {
-        if (rr1 <= lim * lim && k1 >= o.min_pcg_iterations) stop = true;
+        q0 = qk;
+      } else if (__double_as_longlong(rr1) <= lim2_bits && k1 >= o.min_pcg_iterations) {
+        stop = true;  // rr1 <= lim^2 (neither negative; a NaN's bits are above every number's)
       }
       if (k1 >= o.max_pcg_iterations) stop = true;
-      if (!(rz1 != 0.0 && isfinite(rz1))) stop = true;
-      sc[0] = rz1 * s_inv_rz;  // beta_{k+1} (the reciprocal as recip_nr(rz_k))
-      sc[1] = rz1;
-      sc[2] = rr1;
-      sc[3] = qk;
-      s_stop = stop ? 1 : 0;
+      const long long bz = __double_as_longlong(rz1) & 0x7fffffffffffffffLL;
+      if (!(bz != 0 && bz < 0x7ff0000000000000LL)) stop = true;  // zero or not finite
+      if (lane == 0) {
+        sc[0] = rz1 * s_inv_rz;  // beta_{k+1}
+        sc[1] = rz1;
+        sc[2] = rr1;
+        s_stop = stop ? 1 : 0;
+      }
+    } else {
+      asm volatile("bar.sync 1, %0;" ::"n"(kGThreads) : "memory");
+      if (staged)
+        for (int e0 = 32 * (warp - 1); e0 < 9 * ncol; e0 += kGThreads - 32) {
+          const int e = min(e0 + lane, 9 * ncol - 1), cl = e / 9;
+          zc[e] = slot_wait(B, sl_z + so + 9 * (size_t)clist[cl] + (e - 9 * cl), wait_tag, true, &s_fail);
+        }
     }
     __syncthreads();
+    if (s_fail) {
+      aborted = true;
+      break;
+    }
     beta = sc[0];
     rz_k = sc[1];
     last_rr = sc[2];
-    q0 = sc[3];
     last_pq = pq;
     ++k;
-    const bool stop = s_stop != 0;
-    if (stop) break;
-    // p_k = z_k + beta_k p_{k-1} at the staged columns
-    if (staged) {
-      if (t >= 96) {
-#pragma unroll
-        for (int u = 0; u < kPre; ++u) {
-          const int e = (t - 96) + u * kGPreThreads;
-          if (e < 9 * nbo) pst[e] = fma(beta, ppre[u], zpre[u]);
-        }
-      }
-      for (int e = kPre * kGPreThreads + t; e < 9 * nbo; e += kGThreads) {  // beyond the prefetched ones
-        const size_t gi = 9 * (size_t)scol[e / 9] + e % 9;
-        pst[e] = fma(beta, __ldcg(pbuf(k + 1) + gi), __ldcg(B.pcg_z + gi));
-      }
-    }
-    __syncthreads();  // the staged direction; sc and s_stop are written again in the next iteration
+    if (s_stop != 0) break;
+    // p_k = z_k + beta_k p_{k-1} at the touched columns
+    if (staged)
+      for (int e = t; e < 9 * ncol; e += kGThreads) pc[e] = fma(beta, pc[e], zc[e]);
+    __syncthreads();  // the direction; sc and s_stop are written again in the next iteration
   }
-  // the owned coordinates' x and r, and the last direction in pcg_p, as the
-  // two-kernel form leaves them
-  if (!aborted) {
-    if (one_round) {
-      if (u_lead) {
-        B.pcg_x[u_i] = ux;
-        B.pcg_r[u_i] = ur;
-        if (k > 0) B.pcg_p[u_i] = up;
-      }
-    } else if (k > 0 && ((k - 1) & 1) == 1) {
-      for (int kb = kb0; kb < kb1; ++kb) {
-        const int4 cbk = B.camblk[kb];
-        for (int e = t; e < 9 * cbk.z; e += kGThreads) {
-          const size_t i = 9 * (size_t)cbk.y + e;
-          B.pcg_p[i] = B.pcg_p2[i];
-        }
-      }
-    }
+  // the owned coordinates' x, r, z and the last direction, as the two-kernel
+  // form leaves them
+  if (!aborted && u_lead) {
+    const size_t g = 9 * (size_t)(c0 + kPcgBlockCams * (kb0 + u_slot)) + u_m;
+    B.pcg_x[g] = ux, B.pcg_r[g] = ur, B.pcg_z[g] = uz;
+    if (k > 0) B.pcg_p[g] = up;
   }
   if (w == 0 && t == 0) {
     L->pcg_iterations = k;
@@ -695,81 +770,88 @@ __global__ void __launch_bounds__(kGThreads, 1) k_pcg_grid(DeviceBatch B, int ca
   }
 }
 
-bool pcg_grid_plan(int num_problems, bool mixed, bool explicit_schur, int nc, const int32_t *sblk_row, int ctas,
-                   GridPlan *plan) {
+static const void *grid_kernel(bool quad) {
+  return quad ? (const void *)k_pcg_grid<true> : (const void *)k_pcg_grid<false>;
+}
+
+bool pcg_grid_plan(int num_problems, bool mixed, bool explicit_schur, int nc, const int32_t *sblk_row,
+                   const int32_t *sblk_col, int ctas, bool quad, GridPlan *plan) {
   *plan = GridPlan();
-  if (num_problems != 1 || mixed || !explicit_schur || nc <= 0 || !sblk_row) return false;
+  if (num_problems != 1 || mixed || !explicit_schur || nc <= 0 || nc > kGMaxCams || !sblk_row) return false;
+  const void *kernel = grid_kernel(quad);
   int dev = 0, sms = 0, optin = 0;
   cudaFuncAttributes fa;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
-      cudaFuncGetAttributes(&fa, k_pcg_grid) != cudaSuccess) {
+      cudaFuncGetAttributes(&fa, kernel) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
-  // one CTA per SM at most, and no more CTAs than rows
-  const int grid = std::max(1, std::min(ctas > 0 ? std::min(ctas, sms) : sms, 9 * nc));
-  // the kernel's split of the rows (all CTAs registered): the most blocks of
-  // touched cameras a CTA stages, the most touched cameras, the most (row,
-  // block) pairs, the longest row
+  // one CTA per SM at most, and no more CTAs than units
+  const int grid = std::max(1, std::min(ctas > 0 ? std::min(ctas, sms) : sms, 5 * nc));
+  // the kernel's split of the units (all CTAs registered): the most (row,
+  // block) pairs and touched columns of a CTA, the longest row
   const long long wtot = (long long)(sblk_row[nc] - sblk_row[0]) + nc;
   auto m_of = [&](int c) { return (long long)(sblk_row[c + 1] - sblk_row[c]) + 1; };
-  auto rows_before = [&](long long tb) {
-    long long r = 0;
-    for (int c = 0; c < nc; ++c) r += rows_below(tb, 9 * ((long long)(sblk_row[c] - sblk_row[0]) + c), m_of(c));
-    return r;
-  };
-  long long most = 0, most_pairs = 0, m_max = 0;
-  int most_cams = 0;
+  long long most_pairs = 0, m_max = 0;
+  int most_cols = 0;
   for (int c = 0; c < nc; ++c) m_max = std::max(m_max, m_of(c));
-  long long ra = 0;
+  std::vector<int> seen(nc, -1);
+  int c = 0, j = 0;  // the next unit: camera, unit of the camera
+  long long before = 0;
   for (int r = 0; r < grid; ++r) {
-    const long long rb = rows_before(((long long)(r + 1) * 9 * wtot + grid - 1) / grid);
-    if (rb > ra) {
-      const int cA = (int)(ra / 9), cB = (int)((rb - 1) / 9);
-      most = std::max(most, (long long)(sblk_row[cB + 1] - sblk_row[cA]) + (cB - cA + 1));
-      most_cams = std::max(most_cams, cB - cA + 1);
-      long long pairs = 0;
-      for (long long rho = ra; rho < rb; ++rho) pairs += m_of((int)(rho / 9));
-      most_pairs = std::max(most_pairs, pairs);
+    const long long tb = ((long long)(r + 1) * 9 * wtot + grid - 1) / grid;
+    long long pairs = 0;
+    int cols = 0;
+    while (c < nc) {
+      const long long m = m_of(c);
+      if (9 * before + 2 * m * j >= tb) break;
+      pairs += j == 4 ? m : 2 * m;
+      if (seen[c] != r) cols += 1, seen[c] = r;
+      for (int e = sblk_row[c]; e < sblk_row[c + 1]; ++e) {
+        const int k = sblk_col[e];
+        if (seen[k] != r) cols += 1, seen[k] = r;
+      }
+      if (++j == 5) j = 0, before += m, ++c;
     }
-    ra = rb;
+    most_pairs = std::max(most_pairs, pairs);
+    most_cols = std::max(most_cols, cols);
   }
   const size_t static_bytes = fa.sharedSizeBytes + 1024;  // the kernel's static shared memory, with margin
-  auto fits = [&](int cap, bool cache, int pairs) { return grid_smem(nc, cap, cache, pairs).total + static_bytes <= (size_t)optin; };
-  // room for a few CTAs fewer than launched; a pass holds one whole row at least
-  int cap_pairs = (int)std::max<long long>(m_max, most_pairs + most_pairs / 4 + 64);
-  while (cap_pairs > m_max && !fits(0, false, cap_pairs)) cap_pairs = std::max<int>((int)m_max, cap_pairs * 3 / 4);
-  if (!fits(0, false, cap_pairs)) return false;
-  int cap = most_cams <= kGMaxOwn ? (int)(most + most / 4 + 16) : 0;
-  const bool cache = cap > 0 && fits(cap, true, cap_pairs);
-  // the form pays off while every CTA keeps its blocks of S in shared memory
-  // for the launch; a complement too large for that is streamed from memory
-  // on every PCG iteration, which the two-kernel product (a CTA per camera
-  // row, the blocks loaded ahead of the wait) does better (1,800 cameras,
-  // 5.8M observations: 85 us per PCG iteration against 378 us here)
-  if (!cache) return false;
-  const size_t smem = grid_smem(nc, cap, cache, cap_pairs).total;
-  if (raise_smem_limit((const void *)k_pcg_grid, smem) != cudaSuccess) {
+  // room for a few CTAs fewer than launched; a pass holds one whole unit at
+  // least.  The form pays off while every CTA keeps its rows of S in shared
+  // memory for the launch; a complement too large for that is streamed from
+  // memory on every PCG iteration, which the two-kernel product (a CTA per
+  // camera row, the blocks loaded ahead of the wait) does better (1,800
+  // cameras, 5.8M observations: 85 us per PCG iteration against 378 us here)
+  const int cap_pairs = (int)std::max<long long>(2 * m_max, most_pairs + most_pairs / 4 + 64);
+  const int cap_cols = std::min(nc, most_cols + most_cols / 4 + 16);
+  if (cap_pairs >= 1 << 28) return false;
+  const size_t smem = grid_smem(nc, cap_cols, cap_pairs).total;
+  if (smem + static_bytes > (size_t)optin) return false;
+  if (raise_smem_limit(kernel, smem) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
   int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_pcg_grid, kGThreads, smem) != cudaSuccess || per_sm < 1) {
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kGThreads, smem) != cudaSuccess || per_sm < 1) {
     cudaGetLastError();
     return false;
   }
   plan->grid = grid;
-  plan->cap_blocks = cap;
-  plan->cache_s = cache ? 1 : 0;
+  plan->cap_cols = cap_cols;
   plan->cap_pairs = cap_pairs;
+  plan->quad = quad;
   plan->smem = smem;
   return true;
 }
 
 cudaError_t launch_pcg_grid(const DeviceBatch &b, const GridPlan &plan, cudaStream_t s) {
   if (plan.grid <= 0) return cudaSuccess;
-  k_pcg_grid<<<plan.grid, kGThreads, plan.smem, s>>>(b, plan.cap_blocks, plan.cache_s, plan.cap_pairs);
+  if (plan.quad)
+    k_pcg_grid<true><<<plan.grid, kGThreads, plan.smem, s>>>(b, plan.cap_cols, plan.cap_pairs);
+  else
+    k_pcg_grid<false><<<plan.grid, kGThreads, plan.smem, s>>>(b, plan.cap_cols, plan.cap_pairs);
   return cudaGetLastError();
 }
 

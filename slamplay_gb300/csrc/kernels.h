@@ -74,18 +74,19 @@ cudaError_t launch_pcg_cluster64(const DeviceBatch &b, const Cluster64Plan &plan
 // with grid-wide barriers (FP64 form, explicit Schur complement).
 struct GridPlan {
   int grid = 0;        // CTAs launched (the ones that register share the work)
-  int cap_blocks = 0;  // blocks of S a CTA's shared-memory layout holds
-  int cache_s = 0;     // 1: the blocks' values too (else only the staged direction)
+  int cap_cols = 0;    // touched columns a CTA's shared-memory layout holds
   int cap_pairs = 0;   // (row, block) pairs of one pass of the product
+  bool quad = false;
   size_t smem = 0;
 };
-// Sizes the launch from the problem's explicit-complement rows (sblk_row,
-// nc + 1); false when the form does not apply (a batch, the mixed form,
-// the implicit complement), when the CTAs' blocks of S would not stay in
-// shared memory, or when its kernel cannot be resident.  ctas: the
-// CTAs of the launch (one per SM at most; 0 = every SM).
-bool pcg_grid_plan(int num_problems, bool mixed, bool explicit_schur, int nc, const int32_t *sblk_row, int ctas,
-                   GridPlan *plan);
+// Sizes the launch from the problem's explicit-complement structure
+// (sblk_row, nc + 1, and sblk_col); false when the form does not apply (a
+// batch, the mixed form, the implicit complement), when the CTAs' rows of S
+// would not stay in shared memory, or when its kernel cannot be resident.
+// ctas: the CTAs of the launch (one per SM at most; 0 = every SM).  quad: the
+// quadratic-model stopping test (gba_pcg_criterion).
+bool pcg_grid_plan(int num_problems, bool mixed, bool explicit_schur, int nc, const int32_t *sblk_row,
+                   const int32_t *sblk_col, int ctas, bool quad, GridPlan *plan);
 cudaError_t launch_pcg_grid(const DeviceBatch &b, const GridPlan &plan, cudaStream_t s);
 // K4a-b: one PCG iteration (implicit Schur mat-vec, camera-side update).
 void launch_pcg_iteration(const DeviceBatch &b, bool mixed, cudaStream_t s);
