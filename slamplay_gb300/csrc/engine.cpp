@@ -78,7 +78,7 @@ Engine::~Engine() {
   for (cudaStream_t &s : cap_)
     if (s) cudaStreamDestroy(s);
   if (own_stream_ && stream_) cudaStreamDestroy(stream_);
-  for (cudaEvent_t e : {ev_start_, ev_stop_, pev_[0], pev_[1]})
+  for (cudaEvent_t e : {ev_start_, ev_stop_, ev_fork_, ev_join_, pev_[0], pev_[1]})
     if (e) cudaEventDestroy(e);
 }
 
@@ -123,6 +123,8 @@ gba_status Engine::init(std::string *err) {
     if ((st = check(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "stream", err)) != GBA_OK) return st;
   for (cudaEvent_t *e : {&ev_start_, &ev_stop_, &pev_[0], &pev_[1]})
     if ((st = check(cudaEventCreate(e), "event", err)) != GBA_OK) return st;
+  for (cudaEvent_t *e : {&ev_fork_, &ev_join_})
+    if ((st = check(cudaEventCreateWithFlags(e, cudaEventDisableTiming), "event", err)) != GBA_OK) return st;
   if ((st = check(cudaDeviceGetAttribute(&sm_count_, cudaDevAttrMultiProcessorCount, device_), "SM count", err)) !=
       GBA_OK)
     return st;
@@ -599,24 +601,48 @@ void Engine::enqueue_setup(cudaStream_t s) {
   launch_post_eval(db_, s);
 }
 
-void Engine::enqueue_lm_head(cudaStream_t s) {
+// side: a second stream to capture what does not depend on each other as
+// parallel branches (nullptr: one after the other on s): the formation reads
+// only what the point elimination wrote, as the camera side does, and the
+// candidate cameras and the points only need the PCG's result.  On a small
+// problem each of these kernels is a chain of FP64 latencies on a few SMs.
+cudaError_t Engine::fork(cudaStream_t s, cudaStream_t side) {
+  cudaError_t e = cudaEventRecord(ev_fork_, s);
+  return e == cudaSuccess ? cudaStreamWaitEvent(side, ev_fork_, 0) : e;
+}
+cudaError_t Engine::join(cudaStream_t s, cudaStream_t side) {
+  cudaError_t e = cudaEventRecord(ev_join_, side);
+  return e == cudaSuccess ? cudaStreamWaitEvent(s, ev_join_, 0) : e;
+}
+
+cudaError_t Engine::enqueue_lm_head(cudaStream_t s, cudaStream_t side) {
+  cudaError_t e = cudaSuccess;
   prof_begin(s);
   launch_point_prepare(db_, mixed_, s);
   prof_end(s, PF_POINT, bytes_point_schur(db_));
-  prof_begin(s);
-  launch_camera_schur(db_, mixed_, s);
-  prof_end(s, PF_SCHUR, bytes_schur(db_));
+  const bool forked = side && db_.explicit_schur;
+  if (forked && (e = fork(s, side)) != cudaSuccess) return e;
   if (db_.explicit_schur) {
     prof_begin(s);
     launch_schur_form(db_, mixed_, s);
     prof_end(s, PF_FORM, bytes_schur_form(db_));
   }
+  prof_begin(s);
+  launch_camera_schur(db_, mixed_, forked ? side : s);
+  prof_end(s, PF_SCHUR, bytes_schur(db_));
+  return forked ? join(s, side) : cudaSuccess;
 }
 
-void Engine::enqueue_lm_tail(cudaStream_t s) {
+cudaError_t Engine::enqueue_lm_tail(cudaStream_t s, cudaStream_t side) {
+  cudaError_t e = cudaSuccess;
+  if (side && (e = fork(s, side)) != cudaSuccess) return e;
   prof_begin(s);
   launch_back_substitute(db_, mixed_, s);
   prof_end(s, PF_BACKSUB, bytes_backsub(db_));
+  prof_begin(s);
+  launch_candidate_cameras(db_, side ? side : s);
+  prof_end(s, PF_TABLE, (double)db_.nc * (72.0 + kCamTable * 8.0));
+  if (side && (e = join(s, side)) != cudaSuccess) return e;
   prof_begin(s);
   launch_candidate_cost(db_, s);
   prof_end(s, PF_CANDIDATE, bytes_cost(db_));
@@ -624,14 +650,12 @@ void Engine::enqueue_lm_tail(cudaStream_t s) {
   launch_decide(db_, s);
   prof_end(s, PF_DECIDE, 0.0);
   prof_begin(s);
-  launch_camera_table(db_, s);
-  prof_end(s, PF_TABLE, (double)db_.nc * (72.0 + kCamTable * 8.0));
-  prof_begin(s);
   launch_eval_jacobian(db_, mixed_, false, s);
   prof_end(s, PF_EVAL, bytes_eval(db_));
   prof_begin(s);
   launch_post_eval(db_, s);
   prof_end(s, PF_POST, 0.0);
+  return cudaSuccess;
 }
 
 // The solve as one graph: setup, WHILE(LM) { head; PCG; tail }, gather.
@@ -706,7 +730,7 @@ gba_status Engine::build_graph(std::string *err, bool cont) {
   db_.pcg_cond = one_launch ? 0 : pcgh;
   e = cudaStreamBeginCaptureToGraph(cap_[0], lmbody, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
   if (e != cudaSuccess) return fail(e, "capture LM body");
-  enqueue_lm_head(cap_[0]);
+  if ((e = enqueue_lm_head(cap_[0], cap_[2])) != cudaSuccess) return fail(e, "LM body");
   if (cl_plan_.cs > 0) {
     // the whole PCG of every problem in one cluster launch
     if ((e = launch_pcg_cluster(db_, cl_plan_, cap_[0])) != cudaSuccess) return fail(e, "PCG cluster kernel");
@@ -730,7 +754,7 @@ gba_status Engine::build_graph(std::string *err, bool cont) {
     }
     if ((e = cudaStreamEndCapture(cap_[1], &tmp)) != cudaSuccess) return fail(e, "end capture PCG body");
   }
-  enqueue_lm_tail(cap_[0]);
+  if ((e = enqueue_lm_tail(cap_[0], cap_[2])) != cudaSuccess) return fail(e, "LM body");
   if ((e = cudaStreamEndCapture(cap_[0], &tmp)) != cudaSuccess) return fail(e, "end capture LM body");
   enqueue_gather(stream_);
   if ((e = cudaStreamEndCapture(stream_, &tmp)) != cudaSuccess) return fail(e, "end capture");
@@ -753,7 +777,7 @@ gba_status Engine::build_graph(std::string *err, bool cont) {
 // caller destroys the graph being built, which owns the bodies.
 void Engine::end_captures() {
   cudaStreamCaptureStatus cs;
-  for (cudaStream_t s : {cap_[1], cap_[0], stream_}) {
+  for (cudaStream_t s : {cap_[1], cap_[0], cap_[2], stream_}) {
     if (cudaStreamIsCapturing(s, &cs) == cudaSuccess && cs != cudaStreamCaptureStatusNone) {
       cudaGraph_t g = nullptr;
       cudaStreamEndCapture(s, &g);
@@ -804,10 +828,10 @@ gba_status Engine::run_host_driven(std::string *err) {
   int bodies = 0;
   while (hstat[1] && hstat[0] == 0) {
     if (++bodies > max_lm_bodies() + 2) break;
-    enqueue_lm_head(stream_);
+    enqueue_lm_head(stream_, nullptr);
     if (one_launch_pcg()) {
       if ((st = enqueue_pcg_one_launch(stream_, err)) != GBA_OK) return st;
-      enqueue_lm_tail(stream_);
+      enqueue_lm_tail(stream_, nullptr);
       if ((st = read_status()) != GBA_OK) return st;
       continue;
     }
@@ -823,7 +847,7 @@ gba_status Engine::run_host_driven(std::string *err) {
       prof_end(stream_, PF_PCGCAM, bytes_pcg_camera(db_));
       if ((st = read_status()) != GBA_OK) return st;
     }
-    enqueue_lm_tail(stream_);
+    enqueue_lm_tail(stream_, nullptr);
     if ((st = read_status()) != GBA_OK) return st;
   }
   enqueue_gather(stream_);
@@ -1282,6 +1306,7 @@ gba_status Engine::compute_step(const gba_problem_view *v, double radius, double
     }
   }
   launch_back_substitute(db_, mixed_, stream_);
+  launch_candidate_cameras(db_, stream_);
   launch_candidate_cost(db_, stream_);
   launch_decide(db_, stream_);
   if ((st = check(cudaStreamSynchronize(stream_), "step kernels", err)) != GBA_OK) return st;

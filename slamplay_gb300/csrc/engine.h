@@ -96,8 +96,10 @@ class Engine {
   gba_status check(cudaError_t e, const char *what, std::string *err);
   void enqueue_setup(cudaStream_t s);
   void zero_counters(cudaStream_t s);
-  void enqueue_lm_head(cudaStream_t s);
-  void enqueue_lm_tail(cudaStream_t s);
+  cudaError_t enqueue_lm_head(cudaStream_t s, cudaStream_t side);
+  cudaError_t enqueue_lm_tail(cudaStream_t s, cudaStream_t side);
+  cudaError_t fork(cudaStream_t s, cudaStream_t side);
+  cudaError_t join(cudaStream_t s, cudaStream_t side);
   // profiling helpers (host-driven mode)
   void prof_begin(cudaStream_t s);
   void prof_end(cudaStream_t s, int entry, double bytes);
@@ -108,7 +110,7 @@ class Engine {
   int device_ = 0;
   cudaStream_t stream_ = nullptr;
   bool own_stream_ = false;
-  cudaStream_t cap_[2] = {nullptr, nullptr};
+  cudaStream_t cap_[3] = {nullptr, nullptr, nullptr};  // graph building: LM body, PCG body, parallel branches
   char *d_arena_ = nullptr;
   size_t d_cap_ = 0;
   char *h_stage_ = nullptr;
@@ -132,7 +134,7 @@ class Engine {
   int graph_segment_ = -1, graph_c_segment_ = -1;
   std::vector<long long> cur_key_;
   // events
-  cudaEvent_t ev_start_ = nullptr, ev_stop_ = nullptr;
+  cudaEvent_t ev_start_ = nullptr, ev_stop_ = nullptr, ev_fork_ = nullptr, ev_join_ = nullptr;
   cudaEvent_t pev_[2] = {nullptr, nullptr};
   std::vector<ProfileEntry> profile_;
   double last_setup_ms_ = 0.0, last_solve_ms_ = 0.0;

@@ -53,33 +53,74 @@ void launch_init_state(const DeviceBatch &b, cudaStream_t s) {
 }
 
 // ---------------------------------------------------------------------------
-// K0
-__global__ void k_camera_table(DeviceBatch B) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= B.nc) return;
-  const LMState *L = B.lm + B.cam_problem[c];
-  if (!L->active || !L->need_jacobian) return;
-  double *tab = B.cam_table + (size_t)kCamTable * c;
-  camera_table_entry(B.cam_param[L->parity] + 9 * (size_t)c, tab, true);
-  if (B.opt.so3_left) so3_left_derivatives(tab);
-  if (B.opt.mixed) {
-    float *tf = B.cam_tablef + (size_t)kCamTable * c;
-    float2 *td = B.cam_tabledf + (size_t)kCamTable * c;
-    for (int k = 0; k < kCamTable; ++k) {
-      const DF d = df_from_double(tab[k]);
-      tf[k] = d.hi;
-      td[k] = make_float2(d.hi, d.lo);
+// Camera tables of up to 32 cameras by one CTA of kCamTableThreads threads:
+// the work is FP64 (sin, cos, the dual-number derivatives: some 700
+// instructions a camera, each holding a sub-partition's pipe for 64 clocks
+// however few cameras there are), so a column of R and dR goes to each of
+// three warps (the common part in all three) and the double-float copies of
+// the mixed form to all four.  sc: the CTA's staging, the cameras' parameters
+// in sc.cam; cameras [c0, c0 + m), of which those with live[.] get a table.
+// (one thread a camera: 16-19 us a launch for up to 250 cameras FP64, 20-31
+// us mixed)
+constexpr int kCamTableCams = 32;
+constexpr int kCamTableThreads = 128;
+struct CamStage {
+  double cam[kCamTableCams][9];
+  double tab[kCamTableCams][45];
+  int live[kCamTableCams];
+};
+__device__ __forceinline__ void camera_tables(const DeviceBatch &B, CamStage &sc, int c0, int m) {
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  if (warp < 3 && lane < m && sc.live[lane]) {
+    double *tab = sc.tab[lane];
+    const double *cam = sc.cam[lane];
+    if (warp == 0)
+      rotation_columns<0, 1>(cam, tab);
+    else if (warp == 1)
+      rotation_columns<1, 2>(cam, tab);
+    else
+      rotation_columns<2, 3>(cam, tab);
+  }
+  if (warp == 3 && lane < m)
+    for (int k = 36; k < kCamTable; ++k) sc.tab[lane][k] = k < 42 ? sc.cam[lane][k - 33] : 0.0;
+  __syncthreads();
+  if (B.opt.so3_left) {
+    if (warp == 0 && lane < m) so3_left_derivatives(sc.tab[lane]);
+    __syncthreads();
+  }
+  for (int i = t; i < kCamTable * m; i += kCamTableThreads) {
+    const int c = i / kCamTable, k = i - kCamTable * c;
+    if (!sc.live[c]) continue;
+    const double v = sc.tab[c][k];
+    const size_t g = (size_t)kCamTable * c0 + i;
+    B.cam_table[g] = v;
+    if (B.opt.mixed) {
+      const DF d = df_from_double(v);
+      B.cam_tablef[g] = d.hi;
+      B.cam_tabledf[g] = make_float2(d.hi, d.lo);
     }
   }
 }
 
-// One warp per block: the per-camera work is FP64 (sin, cos, the dual-number
-// derivatives), and GB300's FP64 rate is per SM, so small warps spread the
-// cameras over more SMs.
-constexpr int kCamTableThreads = 32;
+// K0, of a problem's first evaluation: the later tables are written with the
+// candidate cameras (K5b), which the accepted step makes current.
+__global__ void __launch_bounds__(kCamTableThreads) k_camera_table(DeviceBatch B) {
+  __shared__ CamStage sc;
+  const int c0 = blockIdx.x * kCamTableCams, m = min(kCamTableCams, B.nc - c0);
+  const int t = threadIdx.x;
+  for (int i = t; i < 9 * m; i += kCamTableThreads) {
+    const int c = i / 9;
+    const LMState *L = B.lm + B.cam_problem[c0 + c];
+    const bool live = L->active && L->need_jacobian;
+    if (i == 9 * c) sc.live[c] = live;
+    if (live) sc.cam[c][i - 9 * c] = B.cam_param[L->parity][9 * (size_t)c0 + i];
+  }
+  __syncthreads();
+  camera_tables(B, sc, c0, m);
+}
 
 void launch_camera_table(const DeviceBatch &b, cudaStream_t s) {
-  k_camera_table<<<(b.nc + kCamTableThreads - 1) / kCamTableThreads, kCamTableThreads, 0, s>>>(b);
+  k_camera_table<<<(b.nc + kCamTableCams - 1) / kCamTableCams, kCamTableThreads, 0, s>>>(b);
 }
 
 // ---------------------------------------------------------------------------
@@ -902,44 +943,54 @@ void launch_post_eval(const DeviceBatch &b, cudaStream_t s) {
 
 // ---------------------------------------------------------------------------
 // K5b: candidate cameras x + step * scale (step = -y_c from the PCG), the
-// camera part of |x - x_cand|^2, and the candidate camera tables (R only).
-__global__ void k_candidate_cameras(DeviceBatch B) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= B.nc) return;
-  const LMState *L = B.lm + B.cam_problem[c];
-  if (!L->active || !L->linear_ok) return;
-  const double *x = B.cam_param[L->parity] + 9 * (size_t)c;
-  double *xc = B.cam_param[L->parity ^ 1] + 9 * (size_t)c;
-  double cand[9];
-  double s2 = 0.0;
-  const bool used = B.cam_used[c] != 0;
-  for (int q = 0; q < 9; ++q) {
-    const double step = -B.pcg_x[9 * (size_t)c + q];
-    cand[q] = used ? x[q] + step * B.cam_scale[9 * (size_t)c + q] : x[q];
+// camera part of |x - x_cand|^2, and the candidate cameras' tables with their
+// derivatives: K2 reads R, and if the step is accepted K1 the rest.
+__global__ void __launch_bounds__(kCamTableThreads) k_candidate_cameras(DeviceBatch B) {
+  __shared__ CamStage sc;
+  const int c0 = blockIdx.x * kCamTableCams, m = min(kCamTableCams, B.nc - c0);
+  const int t = threadIdx.x, lane = t & 31, c = c0 + lane;
+  const LMState *L = B.lm + B.cam_problem[c0 + min(lane, m - 1)];
+  const bool live = lane < m && L->active && L->linear_ok;
+  const bool used = live && B.cam_used[c] != 0;
+  if (t < 32) {
+    sc.live[lane] = live;
+    if (live) {
+      const double *x = B.cam_param[L->parity] + 9 * (size_t)c;
+      double *xc = B.cam_param[L->parity ^ 1] + 9 * (size_t)c;
+      double cand[9];
+      double s2 = 0.0;
+      for (int q = 0; q < 9; ++q) {
+        const double step = -B.pcg_x[9 * (size_t)c + q];
+        cand[q] = used ? x[q] + step * B.cam_scale[9 * (size_t)c + q] : x[q];
+      }
+      if (B.opt.pinhole && used) {
+        // local-BA windows: the pose moves on SE3, T <- exp(xi) T
+        const double *y = B.pcg_x + 9 * (size_t)c, *s9 = B.cam_scale + 9 * (size_t)c;
+        const double dw[3] = {-y[0] * s9[0], -y[1] * s9[1], -y[2] * s9[2]};
+        const double du[3] = {-y[3] * s9[3], -y[4] * s9[4], -y[5] * s9[5]};
+        se3_compose_left(dw, du, x, cand);
+      } else if (B.opt.so3_left && used) {
+        const double dw[3] = {-B.pcg_x[9 * (size_t)c + 0] * B.cam_scale[9 * (size_t)c + 0],
+                              -B.pcg_x[9 * (size_t)c + 1] * B.cam_scale[9 * (size_t)c + 1],
+                              -B.pcg_x[9 * (size_t)c + 2] * B.cam_scale[9 * (size_t)c + 2]};
+        compose_left(dw, x, cand);
+      }
+      for (int q = 0; q < 9; ++q) {
+        const double d = x[q] - cand[q];
+        s2 += d * d;
+        xc[q] = cand[q];
+        sc.cam[lane][q] = cand[q];
+      }
+      B.cam_scal[(size_t)kCamScal * c + kCC_STEP2] = used ? s2 : 0.0;
+    }
+  } else if (t >= 96 && live) {
+    // the camera part of step.g (the mixed form's model cost change)
+    double yg = 0.0;
+    for (int q = 0; q < 9; ++q) yg += B.pcg_x[9 * (size_t)c + q] * B.cam_g[9 * (size_t)c + q];
+    B.cam_scal[(size_t)kCamScal * c + kCC_YG] = used ? -yg : 0.0;
   }
-  if (B.opt.pinhole && used) {
-    // local-BA windows: the pose moves on SE3, T <- exp(xi) T
-    const double *y = B.pcg_x + 9 * (size_t)c, *sc = B.cam_scale + 9 * (size_t)c;
-    const double dw[3] = {-y[0] * sc[0], -y[1] * sc[1], -y[2] * sc[2]};
-    const double du[3] = {-y[3] * sc[3], -y[4] * sc[4], -y[5] * sc[5]};
-    se3_compose_left(dw, du, x, cand);
-  } else if (B.opt.so3_left && used) {
-    const double dw[3] = {-B.pcg_x[9 * (size_t)c + 0] * B.cam_scale[9 * (size_t)c + 0],
-                          -B.pcg_x[9 * (size_t)c + 1] * B.cam_scale[9 * (size_t)c + 1],
-                          -B.pcg_x[9 * (size_t)c + 2] * B.cam_scale[9 * (size_t)c + 2]};
-    compose_left(dw, x, cand);
-  }
-  for (int q = 0; q < 9; ++q) {
-    const double d = x[q] - cand[q];
-    s2 += d * d;
-    xc[q] = cand[q];
-  }
-  B.cam_scal[(size_t)kCamScal * c + kCC_STEP2] = used ? s2 : 0.0;
-  // the camera part of step.g (the mixed form's model cost change)
-  double yg = 0.0;
-  for (int q = 0; q < 9; ++q) yg += B.pcg_x[9 * (size_t)c + q] * B.cam_g[9 * (size_t)c + q];
-  B.cam_scal[(size_t)kCamScal * c + kCC_YG] = used ? -yg : 0.0;
-  camera_table_entry(cand, B.cam_table + (size_t)kCamTable * c, false);
+  __syncthreads();
+  camera_tables(B, sc, c0, m);
 }
 
 // K2: candidate cost, FP64 in both precision modes.
@@ -980,10 +1031,11 @@ __global__ void __launch_bounds__(kChunkCap) k_cost_chunk(DeviceBatch B) {
   }
 }
 
-void launch_candidate_cost(const DeviceBatch &b, cudaStream_t s) {
-  k_candidate_cameras<<<(b.nc + kCamTableThreads - 1) / kCamTableThreads, kCamTableThreads, 0, s>>>(b);
-  k_cost_chunk<<<b.nchunks, kChunkCap, 0, s>>>(b);
+void launch_candidate_cameras(const DeviceBatch &b, cudaStream_t s) {
+  k_candidate_cameras<<<(b.nc + kCamTableCams - 1) / kCamTableCams, kCamTableThreads, 0, s>>>(b);
 }
+
+void launch_candidate_cost(const DeviceBatch &b, cudaStream_t s) { k_cost_chunk<<<b.nchunks, kChunkCap, 0, s>>>(b); }
 
 // Cost at the second parameter buffer with the current camera tables (the
 // kernel-level evaluate entry point, where both buffers hold the same point).
@@ -1050,7 +1102,7 @@ void launch_gather_results(const DeviceBatch &b, double *out_cam, double *out_pt
 __global__ void k_window_tables(DeviceBatch B, const double *out_cam) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= B.nc) return;
-  camera_table_entry(out_cam + 9 * (size_t)c, B.cam_table + (size_t)kCamTable * c, false);
+  camera_table_entry(out_cam + 9 * (size_t)c, B.cam_table + (size_t)kCamTable * c);
 }
 
 __global__ void k_window_chi2(DeviceBatch B, const double *out_pt) {

@@ -55,7 +55,7 @@ gba_status fail(gba_status st, const std::string &msg);
 __global__ void k_na_tables(const double *cameras, int nc, double *tables) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= nc) return;
-  camera_table_entry(cameras + 9 * (size_t)c, tables + (size_t)kCamTable * c, false);
+  camera_table_entry(cameras + 9 * (size_t)c, tables + (size_t)kCamTable * c);
 }
 
 // Per observation: residual (pred - observed) and the block's cost partial.

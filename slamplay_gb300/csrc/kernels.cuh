@@ -428,8 +428,10 @@ __device__ __forceinline__ J3 j3mul(J3 x, J3 y) {
   return J3{x.a * y.a, x.a * y.d0 + x.d0 * y.a, x.a * y.d1 + x.d1 * y.a, x.a * y.d2 + x.d2 * y.a};
 }
 
-// Fills tab[0..8] = R (row-major), tab[9 + 9k + 3i + j] = dR_k[i][j].
-__device__ inline void rotation_and_derivatives(const double *aa_in, double *tab) {
+// Columns J0 .. J1 - 1 of R and dR: tab[3 i + j] = R (row-major),
+// tab[9 + 9k + 3i + j] = dR_k[i][j].
+template <int J0, int J1>
+__device__ inline void rotation_columns(const double *aa_in, double *tab) {
   const J3 aa[3] = {J3{aa_in[0], 1.0, 0.0, 0.0}, J3{aa_in[1], 0.0, 1.0, 0.0}, J3{aa_in[2], 0.0, 0.0, 1.0}};
   const J3 theta2 = j3add(j3add(j3mul(aa[0], aa[0]), j3mul(aa[1], aa[1])), j3mul(aa[2], aa[2]));
   if (theta2.a > DBL_EPSILON) {
@@ -447,7 +449,7 @@ __device__ inline void rotation_and_derivatives(const double *aa_in, double *tab
     const J3 w[3] = {j3mul(aa[0], inv), j3mul(aa[1], inv), j3mul(aa[2], inv)};
     const J3 omc = j3sub(j3c(1.0), c);
 #pragma unroll
-    for (int j = 0; j < 3; ++j) {
+    for (int j = J0; j < J1; ++j) {
       const J3 pt[3] = {j3c(j == 0 ? 1.0 : 0.0), j3c(j == 1 ? 1.0 : 0.0), j3c(j == 2 ? 1.0 : 0.0)};
       const J3 wx[3] = {j3sub(j3mul(w[1], pt[2]), j3mul(w[2], pt[1])),
                         j3sub(j3mul(w[2], pt[0]), j3mul(w[0], pt[2])),
@@ -466,7 +468,7 @@ __device__ inline void rotation_and_derivatives(const double *aa_in, double *tab
   } else {
     // R X = X + w x X:  R = I + [w]_x,  dR_k X = e_k x X
 #pragma unroll
-    for (int j = 0; j < 3; ++j) {
+    for (int j = J0; j < J1; ++j) {
       const J3 pt[3] = {j3c(j == 0 ? 1.0 : 0.0), j3c(j == 1 ? 1.0 : 0.0), j3c(j == 2 ? 1.0 : 0.0)};
       const J3 wx[3] = {j3sub(j3mul(aa[1], pt[2]), j3mul(aa[2], pt[1])),
                         j3sub(j3mul(aa[2], pt[0]), j3mul(aa[0], pt[2])),
@@ -483,19 +485,13 @@ __device__ inline void rotation_and_derivatives(const double *aa_in, double *tab
   }
 }
 
-// R only (candidate-point cost evaluation).  Must produce bit-identical R to
-// rotation_and_derivatives, so it runs the same code and drops the rest.
-__device__ inline void camera_table_entry(const double *cam, double *tab, bool derivatives) {
+// A camera's table without the derivatives (the compiler drops them): the
+// same R as a table with them.
+__device__ inline void camera_table_entry(const double *cam, double *tab) {
   double t[kCamTable];
-  rotation_and_derivatives(cam, t);
-  const int n = derivatives ? 36 : 9;
-  for (int k = 0; k < n; ++k) tab[k] = t[k];
-  tab[36] = cam[3];
-  tab[37] = cam[4];
-  tab[38] = cam[5];
-  tab[39] = cam[6];
-  tab[40] = cam[7];
-  tab[41] = cam[8];
+  rotation_columns<0, 3>(cam, t);
+  for (int k = 0; k < 9; ++k) tab[k] = t[k];
+  for (int k = 0; k < 6; ++k) tab[36 + k] = cam[3 + k];
 }
 
 // ---------------------------------------------------------------------------

@@ -10,7 +10,8 @@ namespace gba {
 
 // LM state initialisation (per problem).
 void launch_init_state(const DeviceBatch &b, cudaStream_t s);
-// K0: camera tables (R, dR/dw, t, f, k1, k2) of the current parameters.
+// K0: camera tables (R, dR/dw, t, f, k1, k2) of the current parameters (a
+// problem's first evaluation; K5b writes the later ones).
 void launch_camera_table(const DeviceBatch &b, cudaStream_t s);
 // K1 + K1c: residuals, scaled & corrected Jacobian, point blocks (chunk
 // kernel) and camera blocks (camera kernel).  norms = first pass of the
@@ -104,7 +105,9 @@ cudaError_t raise_smem_limit(const void *func, size_t bytes);
 void pcg_init();
 // K5: point back-substitution, model cost change, candidate points.
 void launch_back_substitute(const DeviceBatch &b, bool mixed, cudaStream_t s);
-// K5b + K2: candidate cameras (+ their tables) and the candidate cost.
+// K5b: candidate cameras and their tables.
+void launch_candidate_cameras(const DeviceBatch &b, cudaStream_t s);
+// K2: the candidate cost.
 void launch_candidate_cost(const DeviceBatch &b, cudaStream_t s);
 // K6: accept / reject, trust-region radius update, termination tests.
 void launch_decide(const DeviceBatch &b, cudaStream_t s);
