@@ -17,6 +17,8 @@
 //  K2  k_cost_chunk     per chunk: candidate cost in FP64.
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "kernels.cuh"
 #include "kernels.h"
 
@@ -146,7 +148,7 @@ __device__ __forceinline__ double eval_rig(const DeviceBatch &B, int64_t o, int 
     ru *= cr.residual_scaling;
     rv *= cr.residual_scaling;
   }
-  ok = isfinite(ru) && isfinite(rv) && isfinite(cost);
+  ok = finite64(ru) && finite64(rv) && finite64(cost);
   if (!unit_scale) {
     const double *sc = B.cam_scale + 9 * (size_t)c, *sp = B.pt_scale + 3 * (size_t)j;
 #pragma unroll
@@ -158,6 +160,9 @@ __device__ __forceinline__ double eval_rig(const DeviceBatch &B, int64_t o, int 
   for (int k = 0; k < 12; ++k) ok = ok && isfinite((float)ju[k]) && isfinite((float)jv[k]);
   return cost;
 }
+
+__device__ __forceinline__ bool finite_real(float v) { return isfinite(v); }
+__device__ __forceinline__ bool finite_real(double v) { return finite64(v); }
 
 // Residual + Jacobian of one observation.  Jc[k] = (d r_u, d r_v)/d cam_k,
 // Jp[k] = (d r_u, d r_v)/d X_k, r = corrected residual; scaled by the Jacobi
@@ -236,7 +241,7 @@ __device__ __forceinline__ double eval_observation(const DeviceBatch &B, int64_t
     ru *= cr.residual_scaling;
     rv *= cr.residual_scaling;
   }
-  bool ok = isfinite(ru) && isfinite(rv) && isfinite(cost);
+  bool ok = finite64(ru) && finite64(rv) && finite64(cost);
   if (!unit_scale) {
     const real *sc = reinterpret_cast<const real *>(MIXED ? (const void *)B.cam_scalef : (const void *)B.cam_scale) +
                      9 * (size_t)c;
@@ -256,12 +261,12 @@ __device__ __forceinline__ double eval_observation(const DeviceBatch &B, int64_t
 #pragma unroll
   for (int k = 0; k < 9; ++k) {
     Jc[k] = mk2(ju[k], jv[k]);
-    ok = ok && isfinite(ju[k]) && isfinite(jv[k]);
+    ok = ok && finite_real(ju[k]) && finite_real(jv[k]);
   }
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
     Jp[k] = mk2(ju[9 + k], jv[9 + k]);
-    ok = ok && isfinite(ju[9 + k]) && isfinite(jv[9 + k]);
+    ok = ok && finite_real(ju[9 + k]) && finite_real(jv[9 + k]);
   }
   r = mk2((real)ru, (real)rv);
   bad = !ok;
@@ -386,7 +391,7 @@ __device__ __forceinline__ double eval_observation_df(const DeviceBatch &B, int6
     ru *= cr.residual_scaling;
     rv *= cr.residual_scaling;
   }
-  bool ok = isfinite(ru) && isfinite(rv) && isfinite(cost);
+  bool ok = finite64(ru) && finite64(rv) && finite64(cost);
   const float2 *sc = B.cam_scaledf + 9 * (size_t)c;
   const float2 *sp = B.pt_scaledf + 3 * (size_t)j;
 #pragma unroll
@@ -445,7 +450,7 @@ __global__ void __launch_bounds__(kChunkCap, !NORMS ? 3 : 1) k_eval_chunk(Device
   // G64: per observation its FP64 J_c^T r (9, at its camera-sorted slot) and
   // J_p^T r (3, at its position)
   __shared__ DF gsm[G64 ? kChunkCap : 1][12];
-  __shared__ double red[kChunkCap / 32];
+  __shared__ double red[2 * (kChunkCap / 32) + 1];
   const int t = threadIdx.x;
   for (int ch = blockIdx.x; ch < B.nchunks; ch += gridDim.x) {
     const ChunkInfo ci = B.chunk[ch];
@@ -515,59 +520,58 @@ __global__ void __launch_bounds__(kChunkCap, !NORMS ? 3 : 1) k_eval_chunk(Device
         B.seg_grad[9 * (size_t)slot9 + q] = df_value(a);
       }
     }
+    // the points' sums, a thread per (point, entry): C (6) and g (3), each over
+    // the point's observations in order (a thread per point ran nine chains of
+    // FP64 additions one after the other)
     double gmax = 0.0, xn2 = 0.0;
-    if (t < ci.pt_count) {
-      const int jj = ci.pt_begin + t;
+    constexpr int kEntries = NORMS ? 3 : 9;
+    for (int i = t; i < ci.pt_count * kEntries; i += blockDim.x) {
+      const int e = i / ci.pt_count, p = i - e * ci.pt_count, jj = ci.pt_begin + p;
       const int b0 = B.pt_obs_begin[jj] - ci.obs_begin, b1 = B.pt_obs_begin[jj + 1] - ci.obs_begin;
-      Acc acc[9];
-#pragma unroll
-      for (int q = 0; q < 9; ++q) acc[q].init();
-      DF g64[3] = {df_zero(), df_zero(), df_zero()};
-      for (int k = b0; k < b1; ++k) {
-#pragma unroll
-        for (int q = 0; q < (G64 ? 6 : 9); ++q) acc[q].add(sm[k][q]);
-        if (G64) {
-#pragma unroll
-          for (int q = 0; q < 3; ++q) g64[q] = df_add(g64[q], gsm[k][9 + q]);
-        }
+      const int q = NORMS ? (e == 0 ? 0 : e == 1 ? 3 : 5) : e;
+      double v = 0.0;
+      if (G64 && q >= 6) {
+        DF g = df_zero();
+        for (int k = b0; k < b1; ++k) g = df_add(g, gsm[k][3 + q]);
+        v = df_value(g);
+      } else {
+        Acc acc;
+        acc.init();
+        for (int k = b0; k < b1; ++k) acc.add(sm[k][q]);
+        v = q < 6 ? (double)acc.rvalue() : acc.value();
       }
       if (NORMS) {
-        B.pt_colnorm[3 * (size_t)jj + 0] = (double)acc[0].rvalue();
-        B.pt_colnorm[3 * (size_t)jj + 1] = (double)acc[3].rvalue();
-        B.pt_colnorm[3 * (size_t)jj + 2] = (double)acc[5].rvalue();
+        B.pt_colnorm[3 * (size_t)jj + e] = v;
+      } else if (q < 6) {
+        B.pt_C[6 * (size_t)jj + q] = v;
       } else {
-#pragma unroll
-        for (int q = 0; q < 6; ++q) B.pt_C[6 * (size_t)jj + q] = (double)acc[q].rvalue();
-        if (B.pt_used[jj]) {
-          const double *x = B.pt_param[parity] + 4 * (size_t)jj;
-#pragma unroll
-          for (int q = 0; q < 3; ++q) {
-            const double gq = G64 ? df_value(g64[q]) : acc[6 + q].value();
-            B.pt_g[3 * (size_t)jj + q] = gq;
-            const double gu = gq / B.pt_scale[3 * (size_t)jj + q];
-            gmax = fmax(gmax, fabs(x[q] - (x[q] - gu)));
-            xn2 += x[q] * x[q];
-          }
-        } else {
-#pragma unroll
-          for (int q = 0; q < 3; ++q) B.pt_g[3 * (size_t)jj + q] = 0.0;
+        const bool used = B.pt_used[jj] != 0;
+        B.pt_g[3 * (size_t)jj + q - 6] = used ? v : 0.0;
+        if (used) {
+          const double x = B.pt_param[parity][4 * (size_t)jj + q - 6];
+          const double gu = v / B.pt_scale[3 * (size_t)jj + q - 6];
+          gmax = max_nonneg(gmax, abs_or_0(x - (x - gu)));
         }
       }
     }
+    if (!NORMS && t < ci.pt_count && B.pt_used[ci.pt_begin + t]) {
+      const double *x = B.pt_param[parity] + 4 * (size_t)(ci.pt_begin + t);
+#pragma unroll
+      for (int q = 0; q < 3; ++q) xn2 += x[q] * x[q];
+    }
     if (!NORMS) {
-      // the mixed form's later evaluations form no cost (eval_observation_df)
-      const bool with_cost = !G64 || (L->iteration == 0 && !L->resumed);
-      const double cs = with_cost ? block_sum(cost, red) : 0.0;
-      const double gm = block_max(gmax, red);
-      const double xs = block_sum(xn2, red);
-      const double bd = block_max(bad ? 1.0 : 0.0, red);
+      // (the mixed form's later evaluations form no cost: eval_observation_df
+      // returns 0)
+      double gm;
+      bool bd;
+      const double sum = block_sums2_max(cost, xn2, gmax, bad, red, &gm, &bd);
+      double *cs_out = B.chunk_scal + (size_t)kChunkScal * ch;
       if (t == 0) {
-        double *cs_out = B.chunk_scal + (size_t)kChunkScal * ch;
-        cs_out[kCS_COST] = cs;
+        cs_out[kCS_COST] = sum;
         cs_out[kCS_GMAX] = gm;
-        cs_out[kCS_XN2] = xs;
-        cs_out[kCS_BAD] = bd;
+        cs_out[kCS_BAD] = bd ? 1.0 : 0.0;
       }
+      if (t == 32) cs_out[kCS_XN2] = sum;
     }
     __syncthreads();
   }
@@ -576,6 +580,36 @@ __global__ void __launch_bounds__(kChunkCap, !NORMS ? 3 : 1) k_eval_chunk(Device
 // ---------------------------------------------------------------------------
 // K1c: one CTA per camera.
 constexpr int kCamThreads = 128;
+
+// A camera's J_c^T J_c (45) and J_c^T r (9) from `tot` (shared memory) to its
+// record, with max |g| and |x|^2, by the CTA's first 64 threads (call from
+// all): a thread per entry, the divisions side by side.
+__device__ __forceinline__ void camera_results(const DeviceBatch &B, int c, int t, const double *tot, int parity) {
+  __shared__ unsigned long long gm;
+  const bool used = B.cam_used[c] != 0;
+  const double *x = B.cam_param[parity] + 9 * (size_t)c;
+  if (t == 0) gm = 0ull;
+  __syncthreads();
+  if (t < 45) {
+    B.cam_B[45 * (size_t)c + t] = tot[t];
+  } else if (t < 54) {
+    const int q = t - 45;
+    const double gq = used ? tot[t] : 0.0;
+    B.cam_g[9 * (size_t)c + q] = gq;
+    if (used) {
+      const double gu = gq / B.cam_scale[9 * (size_t)c + q];
+      atomicMax(&gm, (unsigned long long)__double_as_longlong(abs_or_0(x[q] - (x[q] - gu))));
+    }
+  }
+  __syncthreads();
+  if (t == 0) {
+    double xn2 = 0.0;
+    if (used)
+      for (int q = 0; q < 9; ++q) xn2 += x[q] * x[q];
+    B.cam_scal[(size_t)kCamScal * c + kCC_GMAX] = __longlong_as_double((long long)gm);
+    B.cam_scal[(size_t)kCamScal * c + kCC_XN2] = xn2;
+  }
+}
 
 template <bool MIXED, bool NORMS>
 __global__ void __launch_bounds__(kCamThreads) k_eval_camera(DeviceBatch B) {
@@ -661,26 +695,10 @@ __global__ void __launch_bounds__(kCamThreads) k_eval_camera(DeviceBatch B) {
     part[0][t] = s;  // each t reads its own column only before writing it
   }
   __syncthreads();
-  if (t == 0) {
-    if (NORMS) {
-      for (int q = 0; q < 9; ++q) B.cam_colnorm[9 * (size_t)c + q] = part[0][q];
-    } else {
-      for (int q = 0; q < 45; ++q) B.cam_B[45 * (size_t)c + q] = part[0][q];
-      double gmax = 0.0, xn2 = 0.0;
-      const bool used = B.cam_used[c] != 0;
-      const double *x = B.cam_param[L->parity] + 9 * (size_t)c;
-      for (int q = 0; q < 9; ++q) {
-        const double gq = used ? part[0][45 + q] : 0.0;
-        B.cam_g[9 * (size_t)c + q] = gq;
-        if (used) {
-          const double gu = gq / B.cam_scale[9 * (size_t)c + q];
-          gmax = fmax(gmax, fabs(x[q] - (x[q] - gu)));
-          xn2 += x[q] * x[q];
-        }
-      }
-      B.cam_scal[(size_t)kCamScal * c + kCC_GMAX] = gmax;
-      B.cam_scal[(size_t)kCamScal * c + kCC_XN2] = xn2;
-    }
+  if (NORMS) {
+    if (t < 9) B.cam_colnorm[9 * (size_t)c + t] = part[0][t];
+  } else {
+    camera_results(B, c, t, part[0], L->parity);
   }
 }
 
@@ -694,10 +712,18 @@ __global__ void __launch_bounds__(kCamThreads) k_eval_camera(DeviceBatch B) {
 // thread, shared memory); the camera's last piece to finish (a counter per
 // camera, reset by it) adds the pieces' sums in piece order and writes the
 // camera's values.  Every sum has a fixed order.
-constexpr int kPieceThreads = 64;
+// The entries of an observation are split between two threads (27 of the 54
+// each: the first three rows of J_c^T J_c and of J_c^T r, and the rest), so a
+// piece keeps all four sub-partitions' FP64 pipes busy.  With the points'
+// sums spread over threads (K1), comparisons and maxima by integers and the
+// CTA's sums in one pass, an evaluation (K1 + K1c) went from 68 to 52 us on a
+// window of 3,360 observations, from 49 to 35 on 14,000 and from 217 to 181
+// on 295,000 (walk, 250 cameras).
+constexpr int kPieceLanes = 64;
+constexpr int kPieceThreads = 2 * kPieceLanes;
 
 __global__ void __launch_bounds__(kPieceThreads) k_eval_camera_pieces(DeviceBatch B) {
-  __shared__ double part[kPieceThreads][55];
+  __shared__ double part[kPieceLanes][55];
   __shared__ double tot[54];
   __shared__ int last;
   const int piece = blockIdx.x, t = threadIdx.x;
@@ -716,28 +742,43 @@ __global__ void __launch_bounds__(kPieceThreads) k_eval_camera_pieces(DeviceBatc
   const int k0 = B.cam_piece_begin[c], npc = B.cam_piece_begin[c + 1] - k0;
   const int e1 = B.cam_obs_begin[c + 1];
   const int o0 = B.cam_obs_begin[c] + (piece - k0) * kCamPieceObs, o1 = min(o0 + kCamPieceObs, e1);
-  double acc[54];
+  auto sums = [&](auto first, int ln) {
+    constexpr int A0 = decltype(first)::value ? 0 : 3, A1 = decltype(first)::value ? 3 : 9;
+    double acc[27];
 #pragma unroll
-  for (int q = 0; q < 54; ++q) acc[q] = 0.0;
-  for (int k = o0 + t; k < o1; k += kPieceThreads) {
-    const int64_t o = B.cam_obs_list[k];
-    double2 J[9];
+    for (int q = 0; q < 27; ++q) acc[q] = 0.0;
+    for (int k = o0 + ln; k < o1; k += kPieceLanes) {
+      const int64_t o = B.cam_obs_list[k];
+      double2 J[9];
 #pragma unroll
-    for (int q = 0; q < 9; ++q) J[q] = jload<double2>(B.jac, B.no, q, o);
-    const double2 r = jload<double2>(B.jac, B.no, 12, o);
+      for (int q = A0; q < 9; ++q) J[q] = jload<double2>(B.jac, B.no, q, o);
+      const double2 r = jload<double2>(B.jac, B.no, 12, o);
+      int i = 0;
 #pragma unroll
-    for (int a = 0; a < 9; ++a) {
+      for (int a = A0; a < A1; ++a) {
 #pragma unroll
-      for (int b = a; b < 9; ++b) acc[sym9(a, b)] = fma(J[a].y, J[b].y, fma(J[a].x, J[b].x, acc[sym9(a, b)]));
-      acc[45 + a] = fma(J[a].y, r.y, fma(J[a].x, r.x, acc[45 + a]));
+        for (int b = a; b < 9; ++b, ++i) acc[i] = fma(J[a].y, J[b].y, fma(J[a].x, J[b].x, acc[i]));
+        acc[i] = fma(J[a].y, r.y, fma(J[a].x, r.x, acc[i]));
+        ++i;
+      }
     }
-  }
+    int i = 0;
 #pragma unroll
-  for (int q = 0; q < 54; ++q) part[t][q] = acc[q];
+    for (int a = A0; a < A1; ++a) {
+#pragma unroll
+      for (int b = a; b < 9; ++b, ++i) part[ln][sym9(a, b)] = acc[i];
+      part[ln][45 + a] = acc[i];
+      ++i;
+    }
+  };
+  if (t < kPieceLanes)
+    sums(std::true_type(), t);
+  else
+    sums(std::false_type(), t - kPieceLanes);
   __syncthreads();
   double s = 0.0;
   if (t < 54)
-    for (int i = 0; i < kPieceThreads; ++i) s += part[i][t];
+    for (int i = 0; i < kPieceLanes; ++i) s += part[i][t];
   if (npc > 1) {
     // the piece's sums to the camera's slots; the last piece adds them up
     if (t < 54) B.piece_part[54 * (size_t)piece + t] = s;
@@ -754,23 +795,7 @@ __global__ void __launch_bounds__(kPieceThreads) k_eval_camera_pieces(DeviceBatc
   }
   if (t < 54) tot[t] = s;
   __syncthreads();
-  if (t == 0) {
-    for (int q = 0; q < 45; ++q) B.cam_B[45 * (size_t)c + q] = tot[q];
-    double gmax = 0.0, xn2 = 0.0;
-    const bool used = B.cam_used[c] != 0;
-    const double *x = B.cam_param[L->parity] + 9 * (size_t)c;
-    for (int q = 0; q < 9; ++q) {
-      const double gq = used ? tot[45 + q] : 0.0;
-      B.cam_g[9 * (size_t)c + q] = gq;
-      if (used) {
-        const double gu = gq / B.cam_scale[9 * (size_t)c + q];
-        gmax = fmax(gmax, fabs(x[q] - (x[q] - gu)));
-        xn2 += x[q] * x[q];
-      }
-    }
-    B.cam_scal[(size_t)kCamScal * c + kCC_GMAX] = gmax;
-    B.cam_scal[(size_t)kCamScal * c + kCC_XN2] = xn2;
-  }
+  camera_results(B, c, t, tot, L->parity);
 }
 
 void launch_eval_jacobian(const DeviceBatch &b, bool mixed, bool norms, cudaStream_t s) {
@@ -1020,14 +1045,19 @@ __global__ void __launch_bounds__(kChunkCap) k_cost_chunk(DeviceBatch B) {
         ru = pr.ru, rv = pr.rv;
       }
       cost = block_cost(B.opt.loss, B.opt.loss_scale, ru, rv);
-      bad = !(isfinite(ru) && isfinite(rv) && isfinite(cost));
+      bad = !(finite64(ru) && finite64(rv) && finite64(cost));
     }
-    const double cs = block_sum(cost, red);
-    const double bd = block_max(bad ? 1.0 : 0.0, red);
+    // block_sum's additions; the barrier carries bad
+    cost = warp_sum(cost);
+    if ((t & 31) == 0) red[t >> 5] = cost;
+    const bool bd = __syncthreads_or(bad ? 1 : 0) != 0;
     if (t == 0) {
+      double cs = 0.0;
+      for (int w = 0; w < kChunkCap / 32; ++w) cs += red[w];
       B.chunk_scal[(size_t)kChunkScal * ch + kCS_COST] = cs;
-      B.chunk_scal[(size_t)kChunkScal * ch + kCS_BAD] = bd;
+      B.chunk_scal[(size_t)kChunkScal * ch + kCS_BAD] = bd ? 1.0 : 0.0;
     }
+    __syncthreads();
   }
 }
 

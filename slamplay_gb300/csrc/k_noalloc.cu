@@ -40,10 +40,16 @@ namespace {
 constexpr int kNoAllocMaxCameras = 16384;
 constexpr int kNoAllocMaxObservations = 1 << 24;
 constexpr int kNoAllocThreads = 256;
+// partials (256 observations each) from which a warp takes a whole one: 8 of
+// them per CTA then still give every SM two CTAs.  A warp per 32 against a
+// warp per 256 observations: 29 us against 43 at 608 partials, 42 / 43 at
+// 1,216, 62 / 57 at 2,432, 105 / 96 at 4,864, 343 / 315 at 19,456.
+constexpr int kNoAllocWideBlocks = 2432;
 constexpr int kNoAllocMaxBlocks = kNoAllocMaxObservations / kNoAllocThreads;
 constexpr size_t kNoAllocScratchDoubles = (size_t)kNoAllocMaxCameras * kCamTable + kNoAllocMaxBlocks;  // ~6.3 MB
 
 static __device__ __align__(256) double g_noalloc_scratch[kNoAllocScratchDoubles];
+static __device__ uint32_t g_noalloc_done;  // CTAs of the call that are done
 
 constexpr int kMaxDevices = 64;
 std::mutex g_setup_mu;
@@ -54,48 +60,100 @@ gba_status fail(gba_status st, const std::string &msg);
 // Per-camera table (R, t, f, k1, k2) of the rotation the residual uses.
 __global__ void k_na_tables(const double *cameras, int nc, double *tables) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c == 0) g_noalloc_done = 0u;  // whatever an earlier call left
   if (c >= nc) return;
   camera_table_entry(cameras + 9 * (size_t)c, tables + (size_t)kCamTable * c);
 }
 
-// Per observation: residual (pred - observed) and the block's cost partial.
-// Out-of-range indices give NaN residuals (and a NaN cost) instead of a read
-// outside the arrays.
+// Per observation: residual (pred - observed) and the block's cost partial; the
+// last CTA to finish adds the partials up (a fixed order: the same result
+// for the same problem).  Out-of-range indices give NaN residuals (and a NaN
+// cost) instead of a read outside the arrays.
+// A cost partial is the sum of 256 observations: each 32 by a butterfly over
+// a warp's lanes, the eight results in order.  What bounds the kernel is the
+// FP64 pipe (one warp instruction per 64 clocks per SM sub-partition), about
+// 28 instructions per 32 observations and, a warp per 32, 6 more for the
+// sums.  W = 8: a warp takes all 256 and runs the eight butterflies at once
+// (each level adds only what its lanes keep: 9 additions instead of 40), for
+// problems that still fill the GPU that way; W = 1: a warp per 32.  5M
+// observations of 1,800 cameras: 393 us with a warp per 32, FP64 comparisons
+// and conversions in the reciprocal and a second kernel for the partials; 327
+// us now (the 28 instructions alone: 290 us).
+template <int W>
 __global__ void __launch_bounds__(kNoAllocThreads)
     k_na_residuals(gba_device_problem p, const double *tables, int loss, double loss_scale, double *residuals,
-                   double *partials) {
-  __shared__ double red[kNoAllocThreads / 32];
-  const int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  double cost = 0.0;
-  if (o < p.num_observations) {
-    const int c = p.camera_index[o], j = p.point_index[o];
-    double ru = __longlong_as_double(0x7ff8000000000000LL), rv = ru;
-    if (c >= 0 && c < p.num_cameras && j >= 0 && j < p.num_points) {
-      const double X[3] = {p.points[3 * (size_t)j], p.points[3 * (size_t)j + 1], p.points[3 * (size_t)j + 2]};
-      const double2 uv = make_double2(p.observations[2 * o], p.observations[2 * o + 1]);
-      Proj pr;
-      project(tables + (size_t)kCamTable * c, X, uv, pr);
-      ru = pr.ru;
-      rv = pr.rv;
+                   double *partials, int nblocks, double *cost_out) {
+  constexpr int kWarps = kNoAllocThreads / 32;
+  __shared__ double red[kWarps][8];
+  __shared__ int last;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned full = 0xffffffffu;
+  // the warp's W runs of 32 observations
+  const int64_t o0 = W == 8 ? 256 * ((int64_t)blockIdx.x * kWarps + warp) : 256 * (int64_t)blockIdx.x + 32 * warp;
+  double cost[W];
+#pragma unroll
+  for (int w = 0; w < W; ++w) {
+    const int64_t o = o0 + 32 * w + lane;
+    cost[w] = 0.0;
+    if (o < p.num_observations) {
+      const int c = p.camera_index[o], j = p.point_index[o];
+      double ru = __longlong_as_double(0x7ff8000000000000LL), rv = ru;
+      if (c >= 0 && c < p.num_cameras && j >= 0 && j < p.num_points) {
+        const double X[3] = {p.points[3 * (size_t)j], p.points[3 * (size_t)j + 1], p.points[3 * (size_t)j + 2]};
+        const double2 uv = make_double2(p.observations[2 * o], p.observations[2 * o + 1]);
+        Proj pr;
+        project(tables + (size_t)kCamTable * c, X, uv, pr);
+        ru = pr.ru;
+        rv = pr.rv;
+      }
+      if (residuals) {
+        residuals[2 * o] = ru;
+        residuals[2 * o + 1] = rv;
+      }
+      cost[w] = block_cost(loss, loss_scale, ru, rv);
     }
-    if (residuals) {
-      residuals[2 * o] = ru;
-      residuals[2 * o + 1] = rv;
-    }
-    cost = block_cost(loss, loss_scale, ru, rv);
   }
-  const double s = block_sum(cost, red);
-  if (threadIdx.x == 0) partials[blockIdx.x] = s;
+  if constexpr (W == 8) {
+    // level 16: lanes 0-15 keep runs 0-3, 16-31 runs 4-7; level 8: two each;
+    // level 4: one; every lane after xor s holds its run's butterfly value
+    double a[4], b[2];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      a[i] = (lane < 16 ? cost[i] : cost[4 + i]) + __shfl_xor_sync(full, lane < 16 ? cost[4 + i] : cost[i], 16);
+    const bool h = (lane & 8) == 0;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) b[i] = (h ? a[i] : a[2 + i]) + __shfl_xor_sync(full, h ? a[2 + i] : a[i], 8);
+    const bool q = (lane & 4) == 0;
+    double v = (q ? b[0] : b[1]) + __shfl_xor_sync(full, q ? b[1] : b[0], 4);
+    v += __shfl_xor_sync(full, v, 2);
+    v += __shfl_xor_sync(full, v, 1);
+    if ((lane & 3) == 0) red[warp][lane >> 2] = v;
+    __syncthreads();
+    const int blk = blockIdx.x * kWarps + (int)threadIdx.x;
+    if (threadIdx.x < kWarps && blk < nblocks) {
+      double s = 0.0;
+      for (int w = 0; w < 8; ++w) s += red[threadIdx.x][w];
+      partials[blk] = s;
+    }
+  } else {
+    const double v = warp_sum(cost[0]);
+    if (lane == 0) red[warp][0] = v;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      double s = 0.0;
+      for (int w = 0; w < kWarps; ++w) s += red[w][0];
+      partials[blockIdx.x] = s;
+    }
+  }
+  if (!last_block_done(&g_noalloc_done, gridDim.x, &last)) return;
+  double s = 0.0;
+  for (int i = threadIdx.x; i < nblocks; i += kNoAllocThreads) s += __ldcg(partials + i);
+  s = block_sum(s, &red[0][0]);
+  if (threadIdx.x == 0) *cost_out = s;
 }
 
-// Fixed-order sum of the partials (same result for the same problem).
-__global__ void __launch_bounds__(kNoAllocThreads) k_na_reduce(const double *partials, int n, double *cost) {
-  __shared__ double red[kNoAllocThreads / 32];
-  double s = 0.0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) s += partials[i];
-  s = block_sum(s, red);
-  if (threadIdx.x == 0) *cost = s;
-}
+// The cost of a problem without observations.
+__global__ void k_na_zero(double *cost) { *cost = 0.0; }
 
 }  // namespace
 
@@ -152,10 +210,14 @@ extern "C" gba_status gba_evaluate_noalloc(const gba_device_problem *p, int32_t 
   double *partials = scratch + (size_t)kNoAllocMaxCameras * kCamTable;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int nblocks = (p->num_observations + kNoAllocThreads - 1) / kNoAllocThreads;
-  if (p->num_cameras > 0) k_na_tables<<<(p->num_cameras + 127) / 128, 128, 0, s>>>(p->cameras, p->num_cameras, tables);
-  if (nblocks > 0)
-    k_na_residuals<<<nblocks, kNoAllocThreads, 0, s>>>(*p, tables, loss, loss_scale, residuals, partials);
-  k_na_reduce<<<1, kNoAllocThreads, 0, s>>>(partials, nblocks, cost);
+  k_na_tables<<<p->num_cameras / 128 + 1, 128, 0, s>>>(p->cameras, p->num_cameras, tables);
+  if (nblocks >= kNoAllocWideBlocks)
+    k_na_residuals<8><<<(nblocks + 7) / 8, kNoAllocThreads, 0, s>>>(*p, tables, loss, loss_scale, residuals, partials,
+                                                                   nblocks, cost);
+  else if (nblocks > 0)
+    k_na_residuals<1><<<nblocks, kNoAllocThreads, 0, s>>>(*p, tables, loss, loss_scale, residuals, partials, nblocks, cost);
+  else
+    k_na_zero<<<1, 1, 0, s>>>(cost);
   e = cudaGetLastError();
   if (e != cudaSuccess) return fail(GBA_ERR_CUDA, std::string("kernel launch: ") + cudaGetErrorString(e));
   return GBA_OK;

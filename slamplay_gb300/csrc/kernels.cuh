@@ -320,6 +320,55 @@ __device__ __forceinline__ double block_sum(double v, double *red) {
   __syncthreads();
   return red[0];
 }
+// Whether a double is finite, and the larger of two that are neither
+// negative nor NaN, by integer instructions (an FP64 comparison would hold
+// the FP64 pipe for 64 clocks a warp).
+__device__ __forceinline__ bool finite64(double v) { return (__double2hiint(v) & 0x7ff00000) != 0x7ff00000; }
+__device__ __forceinline__ double max_nonneg(double a, double b) {
+  return __longlong_as_double(max(__double_as_longlong(a), __double_as_longlong(b)));
+}
+// |v|, 0 for a NaN (what fmax(0, |v|) gives).
+__device__ __forceinline__ double abs_or_0(double v) {
+  const long long b = __double_as_longlong(v) & 0x7fffffffffffffffLL;
+  return __longlong_as_double(b > 0x7ff0000000000000LL ? 0LL : b);
+}
+
+// The CTA's sums of a and b (block_sum's additions for each: the same bits)
+// and maximum of g (neither negative nor NaN), and whether any thread has
+// bad, in one pass: both butterflies at once (lanes 0-15 end with a, 16-31
+// with b), the warps' sums added in order by a thread for each.  `red` needs
+// 2 * blockDim / 32 + 1 doubles.  The sums are valid in threads 0 (a) and 32
+// (b) as their returned value, the maximum and bad in every thread.  At
+// least two warps; contains barriers: call from all threads, `red` free
+// before the call.
+__device__ __forceinline__ double block_sums2_max(double a, double b, double g, bool bad, double *red, double *gmax,
+                                                  bool *any_bad) {
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const bool lo = lane < 16;
+  double v = (lo ? a : b) + __shfl_xor_sync(full, lo ? b : a, 16);
+  v += __shfl_xor_sync(full, v, 8);
+  v += __shfl_xor_sync(full, v, 4);
+  v += __shfl_xor_sync(full, v, 2);
+  v += __shfl_xor_sync(full, v, 1);
+  const unsigned hi = (unsigned)__double2hiint(g);
+  const unsigned mh = __reduce_max_sync(full, hi);
+  const unsigned ml = __reduce_max_sync(full, hi == mh ? (unsigned)__double2loint(g) : 0u);
+  unsigned long long *gm = reinterpret_cast<unsigned long long *>(red + 2 * nw);
+  if (threadIdx.x == 0) *gm = 0ull;
+  if ((lane & 15) == 0) red[(lane >> 4) * nw + warp] = v;
+  *any_bad = __syncthreads_or(bad ? 1 : 0) != 0;
+  if (lane == 0) atomicMax(gm, ((unsigned long long)mh << 32) | ml);
+  double s = 0.0;
+  if (threadIdx.x == 0 || threadIdx.x == 32) {
+    const double *r = red + (threadIdx.x == 0 ? 0 : nw);
+    for (int w = 0; w < nw; ++w) s += r[w];
+  }
+  __syncthreads();
+  *gmax = __longlong_as_double((long long)*gm);
+  return s;
+}
+
 __device__ __forceinline__ double block_max(double v, double *red) {
   v = warp_max(v);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
