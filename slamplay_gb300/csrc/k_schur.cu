@@ -13,7 +13,8 @@
 // observation a (9x3, formed by the point kernel K3a), the block of cameras
 // (i, k) is -sum over the points both see of F_a F_b^T.
 //
-//  K3c k_schur_form   one CTA per block on or above the diagonal (k >= i):
+//  K3c k_schur_form (FP64), k_schur_form_mixed
+//                     one CTA per block on or above the diagonal (k >= i):
 //                     the F rows of 64 pairs per round staged in shared
 //                     memory (the next round's loads in flight while this
 //                     one is summed); the sum over the block's pairs, in a
@@ -51,34 +52,21 @@ __device__ __forceinline__ void pdl_launch_dependents_s() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-// 16-byte vector of the working precision
-template <bool MIXED>
-struct Vec16;
-template <>
-struct Vec16<true> {
-  typedef float4 type;
-};
-template <>
-struct Vec16<false> {
-  typedef double2 type;
-};
-
 }  // namespace
 
 // ---------------------------------------------------------------------------
-// K3c
-template <bool MIXED>
+// K3c of the FP64 form: the FP64 pipe bounds it (243 FMAs a pair, one warp
+// instruction per 64 clocks per sub-partition: 92 % of that on 250 cameras).
 __global__ void __launch_bounds__(kFormThreads) k_schur_form(DeviceBatch B) {
-  typedef typename Prec<MIXED>::real real;
-  typedef typename Acc<MIXED>::type Acc;
-  typedef typename Vec16<MIXED>::type vec;
+  typedef double real;
+  typedef double2 vec;
   constexpr int kVec = (int)(sizeof(vec) / sizeof(real));
   constexpr int kRowVecs = kObsF / kVec;  // 16-byte loads per F row
   constexpr int kRoundVecs = kFormPairs * 2 * kRowVecs;
   constexpr int kPer = (kRoundVecs + kFormThreads - 1) / kFormThreads;  // loads per thread per round
   static_assert(kObsF % kVec == 0, "F rows are whole 16-byte vectors");
   __shared__ __align__(16) real Fs[kFormPairs][2][kObsF];  // F of the row's and the column's observation
-  __shared__ Acc part[kFormSub][81];
+  __shared__ double part[kFormSub][81];
   const int ub = blockIdx.x, t = threadIdx.x;
   const int blk = B.sblk_up[ub];
   const int p0 = B.sblk_pair[ub], p1 = B.sblk_pair[ub + 1];
@@ -116,8 +104,7 @@ __global__ void __launch_bounds__(kFormThreads) k_schur_form(DeviceBatch B) {
   // sub-lane `sub` of entry (i, k) sums the pairs sub, sub + kFormSub, ...
   // of every round, in order
   const int sub = t / 81, en = t - 81 * sub, ei = en / 9, ek = en - 9 * ei;
-  Acc acc;
-  acc.init();
+  double acc = 0.0;
   load_round(p0);
   store_round(p0);
   __syncthreads();
@@ -128,10 +115,8 @@ __global__ void __launch_bounds__(kFormThreads) k_schur_form(DeviceBatch B) {
     if (sub < kFormSub)
       for (int u = sub; u < n; u += kFormSub) {
         const real *fa = &Fs[u][0][3 * ei], *fb = &Fs[u][1][3 * ek];
-        if constexpr (MIXED)
-          acc.add(fa[0] * fb[0] + fa[1] * fb[1] + fa[2] * fb[2]);
-        else  // FP64: one FMA chain through the accumulator (three FP64 operations a pair, not four)
-          acc.s = fma(fa[2], fb[2], fma(fa[1], fb[1], fma(fa[0], fb[0], acc.s)));
+        // one FMA chain through the accumulator (three FP64 operations a pair, not four)
+        acc = fma(fa[2], fb[2], fma(fa[1], fb[1], fma(fa[0], fb[0], acc)));
       }
     __syncthreads();  // the stage is reused
     if (more) store_round(g + kFormPairs);
@@ -140,10 +125,10 @@ __global__ void __launch_bounds__(kFormThreads) k_schur_form(DeviceBatch B) {
   if (sub < kFormSub) part[sub][en] = acc;
   __syncthreads();
   if (t < 81) {
-    Acc s = part[0][t];
+    double s = part[0][t];
 #pragma unroll
-    for (int j = 1; j < kFormSub; ++j) s.merge(part[j][t]);
-    const real v = -(real)s.rvalue();
+    for (int j = 1; j < kFormSub; ++j) s += part[j][t];
+    const real v = -s;
     real *vals = reinterpret_cast<real *>(B.sblk_val);
     const int i = t / 9, k = t - 9 * i;
     vals[81 * (size_t)blk + t] = v;
@@ -152,109 +137,228 @@ __global__ void __launch_bounds__(kFormThreads) k_schur_form(DeviceBatch B) {
   }
 }
 
+// K3c of the mixed form.  What bounded the form above there were its
+// shared-memory loads, six per entry and pair: a lane here sums three entries
+// of a column (four loads per entry and pair), three rows' thirds times three
+// columns times the three interleaved runs on 27 lanes of three warps, with
+// the same additions in the same order, the next step's rows loaded while
+// one is added.  All four warps copy the F rows, 16 pairs of a round each,
+// asynchronously, a round ahead.  Before and after, per launch: 882 and 535 us
+// on 68,000 blocks of 107 pairs, 323 and 213 on 192 windows of 5-40 cameras,
+// 122 and 87 on 250 cameras, 38 and 33 on one window of 8 cameras (blocks of
+// up to 1,300 pairs: the chain of one block's steps bounds it).  A warp per
+// block with 3x3 tiles (two loads per entry and pair) took 431 us on the
+// 68,000 blocks but 104 on 250 cameras and 74 on the one window.
+constexpr int kTileWarps = 4;
+constexpr int kTilePairs = 16;  // pairs of a round a warp copies
+constexpr int kTileStages = 2;
+static_assert(kFormPairs == kTileWarps * kTilePairs && kFormSub == 3, "stages of a round");
+static_assert(kTilePairs * 2 == 32 && kObsF == 28, "a lane per row index, seven 16-byte copies a row");
+
+__global__ void __launch_bounds__(32 * kTileWarps) k_schur_form_mixed(DeviceBatch B) {
+  __shared__ __align__(16) float Fs[kTileStages][kFormPairs][2][kObsF];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int ub = blockIdx.x, blk = B.sblk_up[ub];
+  const int p0 = B.sblk_pair[ub], p1 = B.sblk_pair[ub + 1];
+  if (!B.lm[B.cam_problem[B.sblk_col[blk]]].active) return;  // uniform
+  const float *F = reinterpret_cast<const float *>(B.obs_F);
+  const int *pairs = reinterpret_cast<const int *>(B.spair);
+  const int w0 = kTilePairs * warp;  // this warp's pairs of a round
+  // lane l: the observation of the warp's pair l / 2, the row's (even) or the column's
+  auto load_index = [&](int g) { return g + w0 + (lane >> 1) < p1 ? pairs[2 * (size_t)(g + w0) + lane] : 0; };
+  // copies the rows of the warp's pairs of round g (none beyond p1)
+  auto stage_rows = [&](int g, int st, int ob) {
+    const int rows = 2 * (p1 - g - w0);
+    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&Fs[st][w0][0][0]);
+#pragma unroll
+    for (int u = 0; u < 7; ++u) {
+      const int i = lane + 32 * u, row = i / 7, e = i - 7 * row;
+      const int o = __shfl_sync(0xffffffffu, ob, row);
+      if (row < rows)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16u * (uint32_t)i),
+                     "l"(F + (size_t)kObsF * o + 4 * e)
+                     : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  const int sub = lane / 9, tile = lane - 9 * sub, ti = tile / 3, kc = 3 * warp + tile - 3 * ti;
+  const int last = min(sub, kFormSub - 1);  // (lanes 27-31 repeat a run's pairs and drop the result)
+  KahanF acc[3];
+#pragma unroll
+  for (int e = 0; e < 3; ++e) acc[e].init();
+  struct Rows {
+    float a[9], b[3];
+  };
+  auto load_rows = [&](int st, int r) {
+    Rows f;
+#pragma unroll
+    for (int e = 0; e < 9; ++e) f.a[e] = Fs[st][r][0][9 * ti + e];
+#pragma unroll
+    for (int e = 0; e < 3; ++e) f.b[e] = Fs[st][r][1][3 * kc + e];
+    return f;
+  };
+  auto add_rows = [&](const Rows &f) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+      acc[i].add(f.a[3 * i] * f.b[0] + f.a[3 * i + 1] * f.b[1] + f.a[3 * i + 2] * f.b[2]);
+  };
+#pragma unroll
+  for (int r = 0; r < kTileStages - 1; ++r) stage_rows(p0 + kFormPairs * r, r, load_index(p0 + kFormPairs * r));
+  int ob = load_index(p0 + kFormPairs * (kTileStages - 1));
+  for (int g = p0, st = 0; g < p1; g += kFormPairs) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kTileStages - 2) : "memory");
+    __syncthreads();  // the round has landed; every warp is done with the one before
+    stage_rows(g + kFormPairs * (kTileStages - 1), st == 0 ? kTileStages - 1 : st - 1, ob);
+    ob = load_index(g + kFormPairs * kTileStages);
+    if (warp < 3) {
+      const int n = min(kFormPairs, p1 - g);
+      int done = 0;
+      if (n >= kFormSub) {
+        Rows f = load_rows(st, last);
+#pragma unroll 4
+        for (done = kFormSub; done + kFormSub <= n; done += kFormSub) {
+          const Rows nf = load_rows(st, done + last);
+          add_rows(f);
+          f = nf;
+        }
+        add_rows(f);
+      }
+      if (done + sub < n) add_rows(load_rows(st, done + sub));
+    }
+    st = st == kTileStages - 1 ? 0 : st + 1;
+  }
+  __syncthreads();  // the stages are reused
+  KahanF *part = reinterpret_cast<KahanF *>(&Fs[0][0][0][0]);
+  if (warp < 3 && sub < kFormSub)
+#pragma unroll
+    for (int i = 0; i < 3; ++i) part[81 * sub + 9 * (3 * ti + i) + kc] = acc[i];
+  __syncthreads();
+  // the three runs of each entry combined in order, stored with the transpose
+  const int e = threadIdx.x;
+  if (e < 81) {
+    KahanF s = part[e];
+#pragma unroll
+    for (int j = 1; j < kFormSub; ++j) s.merge(part[81 * j + e]);
+    const float v = -s.rvalue();
+    float *vals = reinterpret_cast<float *>(B.sblk_val);
+    const int tr = B.sblk_tr[blk];
+    vals[81 * (size_t)blk + e] = v;
+    if (tr != blk) vals[81 * (size_t)tr + 9 * (e % 9) + e / 9] = v;
+  }
+}
+
 void launch_schur_form(const DeviceBatch &b, bool mixed, cudaStream_t s) {
   if (!b.explicit_schur || b.nup == 0) return;
   if (mixed)
-    k_schur_form<true><<<b.nup, kFormThreads, 0, s>>>(b);
+    k_schur_form_mixed<<<b.nup, 32 * kTileWarps, 0, s>>>(b);
   else
-    k_schur_form<false><<<b.nup, kFormThreads, 0, s>>>(b);
+    k_schur_form<<<b.nup, kFormThreads, 0, s>>>(b);
 }
 
 // ---------------------------------------------------------------------------
 // K4a'
 constexpr int kSpmvThreads = 9 * 32;
-constexpr int kSpmvPrefetch = 2;  // blocks per lane whose values load before the wait
+constexpr int kSpmvStage = 96;  // blocks of a camera staged at a time (at most)
 
-template <bool MIXED>
-__global__ void __launch_bounds__(kSpmvThreads) k_schur_spmv(DeviceBatch B) {
-  typedef typename Prec<MIXED>::real real;
-  __shared__ double pqs[9];
+// Mixed form.  A lane that reads its block's row from memory touches a
+// 128-byte line of its own with every load, and so do its reads of the
+// direction: the L1's lines per load, not bytes, bounded the kernel.  So the
+// camera's blocks, contiguous in memory, are copied into shared memory (16
+// bytes a copy, issued before the wait), the direction at their columns is
+// formed once for the nine rows, and both are read from there, an odd stride
+// between lanes (81 and 9 words: no bank conflicts).  `cap` (a multiple of
+// 32, at most kSpmvStage): blocks the stage holds; longer rows take rounds.
+// The rows' FP64 values are formed by one warp for all nine (a warp each
+// would queue on the FP64 pipes: 54 instead of 14 instructions a camera).
+// 1,800 cameras with 76 blocks each: 32.4 us with reads from memory, 26.7 now.
+__global__ void __launch_bounds__(kSpmvThreads) k_schur_spmv(DeviceBatch B, int cap) {
+  extern __shared__ __align__(16) float sv_smem[];  // [81 cap + 4] blocks, [9 cap] direction
+  __shared__ DF rows[9];
   const int c = blockIdx.x, t = threadIdx.x;
   const int q = t >> 5, lane = t & 31;
-  const int prob = B.cam_problem[c];
   const int r0 = B.sblk_row[c], nb = B.sblk_row[c + 1] - r0;
+  float *sv = sv_smem, *sp = sv_smem + 81 * cap + 4;
   // virtual block v of the row: v < nb the off-diagonal block r0 + v, v = nb
   // the diagonal block; lane l takes v = l, l + 32, ...
-  const real *vals = reinterpret_cast<const real *>(B.sblk_val);
-  const real *diag = reinterpret_cast<const real *>(B.cam_Sii) + 81 * (size_t)c + 9 * q;
-  real pre[kSpmvPrefetch][9];
-  int pcol[kSpmvPrefetch];
-#pragma unroll
-  for (int u = 0; u < kSpmvPrefetch; ++u) {
-    const int v = lane + 32 * u;
-    pcol[u] = -1;
-#pragma unroll
-    for (int cc = 0; cc < 9; ++cc) pre[u][cc] = 0;
-    if (v <= nb) {
-      const real *row = v < nb ? vals + 81 * (size_t)(r0 + v) + 9 * q : diag;
-      pcol[u] = v < nb ? B.sblk_col[r0 + v] : c;
-#pragma unroll
-      for (int cc = 0; cc < 9; ++cc) pre[u][cc] = row[cc];
+  const float *vals = reinterpret_cast<const float *>(B.sblk_val) + 81 * (size_t)r0;
+  const int off = r0 & 3;  // the stage keeps the source's place in its 16 bytes
+  const uint32_t sv0 = (uint32_t)__cvta_generic_to_shared(sv);
+  auto stage = [&](int v0) {  // blocks [v0, v0 + cap); v0 a multiple of 32
+    const int n = min(cap, nb - v0);
+    if (n > 0) {
+      const int chunks = (off + 81 * n + 3) >> 2;
+      const float *src = vals - off + 81 * (size_t)v0;
+      for (int i = t; i < chunks; i += kSpmvThreads)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(sv0 + 16u * (uint32_t)i), "l"(src + 4 * (size_t)i)
+                     : "memory");
     }
+  };
+  const LMState *L = B.lm + B.cam_problem[c];
+  // (a PCG that has ended does not start again before the next camera-side
+  // kernel, so the early look only ever skips work; past the L1, which would
+  // keep the state of before the wait)
+  const bool hint = __ldcg(&L->active) && __ldcg(&L->pcg_active);
+  float diag = 0.f;
+  if (hint) {
+    stage(0);
+    if (t < 81) diag = (reinterpret_cast<const float *>(B.cam_Sii) + 81 * (size_t)c)[t];
   }
   pdl_wait_s();
   pdl_launch_dependents_s();
-  const LMState *L = B.lm + prob;
-  if (!(L->active && L->pcg_active)) return;  // uniform over the CTA
-  const int k = L->pcg_iterations;
-  const double beta = L->beta;
-  const real *zv = reinterpret_cast<const real *>(MIXED ? (const void *)B.pcg_zf : (const void *)B.pcg_z);
-  const real *pvv = reinterpret_cast<const real *>(MIXED ? (const void *)B.pcg_pf : (const void *)B.pcg_p);
-  // p_k of a camera coordinate: the FP64 form evaluates the camera kernel's
-  // expression, the mixed form the same recurrence in FP32 on the FP32
-  // copies (as the implicit mat-vec)
-  auto pdir = [&](size_t idx) -> real {
-    const real z = zv[idx];
+  if (!hint || !__ldcg(&L->pcg_active)) {  // uniform over the CTA
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    return;
+  }
+  const int k = __ldcg(&L->pcg_iterations);
+  const float beta = (float)__ldcg(&L->beta);
+  // p_k of a camera coordinate: the camera kernel's recurrence in FP32 on the
+  // FP32 copies (as the implicit mat-vec)
+  auto pdir = [&](size_t idx) -> float {
+    const float z = B.pcg_zf[idx];
     if (k == 0) return z;
-    if (MIXED) return (real)__fmaf_rn((float)beta, (float)pvv[idx], (float)z);
-    return (real)fma(beta, (double)pvv[idx], (double)z);
+    return __fmaf_rn(beta, B.pcg_pf[idx], z);
   };
-  auto row_dot = [&](const real *row, int col) -> real {
-    real s = 0;
-#pragma unroll
-    for (int cc = 0; cc < 9; ++cc) s += row[cc] * pdir(9 * (size_t)col + cc);
-    return s;
-  };
-  // the lane's blocks in order: FP64 sums in the FP64 form, double-float in
-  // the mixed form
-  DF af = df_zero();
-  double ad = 0.0;
-#pragma unroll
-  for (int u = 0; u < kSpmvPrefetch; ++u)
-    if (pcol[u] >= 0) {
-      const real s = row_dot(pre[u], pcol[u]);
-      if (MIXED)
-        af = df_add(af, DF{(float)s, 0.f});
-      else
-        ad += (double)s;
+  DF af = df_zero();  // the lane's blocks in order
+  for (int v0 = 0; v0 <= nb; v0 += cap) {
+    const int n = min(cap, nb + 1 - v0);
+    if (v0 > 0) {
+      __syncthreads();  // the stage is reused
+      stage(v0);
     }
-  for (int v = lane + 32 * kSpmvPrefetch; v <= nb; v += 32) {
-    const real *row = v < nb ? vals + 81 * (size_t)(r0 + v) + 9 * q : diag;
-    const real s = row_dot(row, v < nb ? B.sblk_col[r0 + v] : c);
-    if (MIXED)
-      af = df_add(af, DF{(float)s, 0.f});
-    else
-      ad += (double)s;
+    for (int e = t; e < 9 * n; e += kSpmvThreads) {
+      const int v = e / 9, col = v0 + v < nb ? B.sblk_col[r0 + v0 + v] : c;
+      sp[e] = pdir(9 * (size_t)col + (e - 9 * v));
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    if (nb - v0 < cap) {  // uniform; after the round's copies, which may share their last 16 bytes with it
+      if (t < 81) sv[off + 81 * (nb - v0) + t] = diag;
+      __syncthreads();
+    }
+    for (int v = lane; v < n; v += 32) {
+      const float *row = sv + off + 81 * v + 9 * q, *pp = sp + 9 * v;
+      float s = 0.f;
+#pragma unroll
+      for (int cc = 0; cc < 9; ++cc) s += row[cc] * pp[cc];
+      af = df_add(af, DF{s, 0.f});
+    }
   }
   // the row's sum over the lanes (butterfly: a fixed order)
-  double qv;
-  if (MIXED) {
-    af = df_warp_sum(af);
-    qv = df_value(af);
-  } else {
-    qv = warp_sum(ad);
-  }
-  if (lane == 0) {
-    const size_t i = 9 * (size_t)c + q;
-    B.pcg_q[i] = qv;
-    pqs[q] = (double)pdir(i) * qv;
-  }
+  af = df_warp_sum(af);
+  if (lane == 0) rows[q] = af;
   __syncthreads();
-  if (t == 0) {
+  if (t < 32) {
+    double pq = 0.0;
+    if (t < 9) {
+      const size_t i = 9 * (size_t)c + t;
+      const double qv = df_value(rows[t]);
+      B.pcg_q[i] = qv;
+      pq = (double)pdir(i) * qv;
+    }
     double s = 0.0;
 #pragma unroll
-    for (int r = 0; r < 9; ++r) s += pqs[r];
-    B.spmv_red[c] = s;
+    for (int r = 0; r < 9; ++r) s += __shfl_sync(0xffffffffu, pq, r);
+    if (t == 0) B.spmv_red[c] = s;
   }
 }
 
@@ -357,7 +461,11 @@ cudaError_t launch_schur_spmv(const DeviceBatch &b, bool mixed, cudaStream_t s, 
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pdl ? 1 : 0;
-  if (mixed) return cudaLaunchKernelEx(&cfg, k_schur_spmv<true>, b);
+  if (mixed) {
+    const int cap = std::min((b.sblk_max + 31) / 32 * 32, kSpmvStage);
+    cfg.dynamicSmemBytes = sizeof(float) * (90 * (size_t)cap + 4);
+    return cudaLaunchKernelEx(&cfg, k_schur_spmv, b, cap);
+  }
   size_t smem = 0;
   int stage = 0;
   const int rpp = spmv64_rows(b.sblk_max, &smem, &stage);
