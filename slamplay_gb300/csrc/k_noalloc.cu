@@ -74,11 +74,10 @@ __global__ void k_na_tables(const double *cameras, int nc, double *tables) {
 // FP64 pipe (one warp instruction per 64 clocks per SM sub-partition), about
 // 28 instructions per 32 observations and, a warp per 32, 6 more for the
 // sums.  W = 8: a warp takes all 256 and runs the eight butterflies at once
-// (each level adds only what its lanes keep: 9 additions instead of 40), for
-// problems that still fill the GPU that way; W = 1: a warp per 32.  5M
-// observations of 1,800 cameras: 393 us with a warp per 32, FP64 comparisons
-// and conversions in the reciprocal and a second kernel for the partials; 327
-// us now (the 28 instructions alone: 290 us).
+// (9 additions instead of 40), for problems that still fill the GPU that way;
+// W = 1: a warp per 32.  5M observations of 1,800 cameras: 393 us with a warp
+// per 32, FP64 comparisons and conversions in the reciprocal and a second
+// kernel for the partials; 327 us now (the 28 instructions alone: 290 us).
 template <int W>
 __global__ void __launch_bounds__(kNoAllocThreads)
     k_na_residuals(gba_device_problem p, const double *tables, int loss, double loss_scale, double *residuals,
@@ -87,7 +86,6 @@ __global__ void __launch_bounds__(kNoAllocThreads)
   __shared__ double red[kWarps][8];
   __shared__ int last;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const unsigned full = 0xffffffffu;
   // the warp's W runs of 32 observations
   const int64_t o0 = W == 8 ? 256 * ((int64_t)blockIdx.x * kWarps + warp) : 256 * (int64_t)blockIdx.x + 32 * warp;
   double cost[W];
@@ -114,19 +112,7 @@ __global__ void __launch_bounds__(kNoAllocThreads)
     }
   }
   if constexpr (W == 8) {
-    // level 16: lanes 0-15 keep runs 0-3, 16-31 runs 4-7; level 8: two each;
-    // level 4: one; every lane after xor s holds its run's butterfly value
-    double a[4], b[2];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-      a[i] = (lane < 16 ? cost[i] : cost[4 + i]) + __shfl_xor_sync(full, lane < 16 ? cost[4 + i] : cost[i], 16);
-    const bool h = (lane & 8) == 0;
-#pragma unroll
-    for (int i = 0; i < 2; ++i) b[i] = (h ? a[i] : a[2 + i]) + __shfl_xor_sync(full, h ? a[2 + i] : a[i], 8);
-    const bool q = (lane & 4) == 0;
-    double v = (q ? b[0] : b[1]) + __shfl_xor_sync(full, q ? b[1] : b[0], 4);
-    v += __shfl_xor_sync(full, v, 2);
-    v += __shfl_xor_sync(full, v, 1);
+    const double v = warp_sum8(cost);
     if ((lane & 3) == 0) red[warp][lane >> 2] = v;
     __syncthreads();
     const int blk = blockIdx.x * kWarps + (int)threadIdx.x;

@@ -483,18 +483,22 @@ static_assert(kPcgThreads % 32 == 0, "the block reductions combine whole warps")
 
 // Two CTAs per SM (56 registers a thread, some spilled): a problem's camera
 // blocks run in one wave instead of two on 1,800 cameras (20.1 instead of
-// 22.7 us per PCG iteration; FP64 batches of configuration 3 +4.7 %).
+// 22.7 us per PCG iteration; FP64 batches of configuration 3 +4.7 %).  Its
+// time is a chain of FP64 sums: with those of p.q eight warps at a time, the
+// blocks' values by a warp each and what the state alone gives taken before
+// the wait, 15.1 us instead of 19.5 (1,800 cameras, mixed, explicit
+// complement).
 template <bool MIXED>
 __global__ void __launch_bounds__(kPcgThreads, 2) k_pcg_camera(DeviceBatch B) {
   typedef typename Prec<MIXED>::real real;
   typedef typename Acc<MIXED>::type Acc;
-  __shared__ Acc psub[kPcgSub][kPcgCoords];  // sub-lane sums of the partials
+  __shared__ __align__(16) Acc psub[kPcgSub][kPcgCoords];  // sub-lane sums of the partials
   __shared__ double pv[kPcgCoords];          // p_k of the block, for (B + Dc^2) p
   __shared__ real rv[kPcgCoords];            // r_{k+1} of the block, for M r
   __shared__ double red[kPcgWarps];
   __shared__ DF dfred[kPcgWarps];
   __shared__ double red3[kPcgWarps][3];
-  __shared__ double sc[2];
+  __shared__ double sc[4];                   // p.q, alpha; 1 / r_k.z_k and the residual limit squared
   __shared__ double chs[kPcgChunkSums];  // the explicit FP64 form's p.q chunk sums
   __shared__ int flag, sgood;
   constexpr int kLeadWarps = (kPcgCoords + 31) / 32;  // the warps holding sub-lane 0
@@ -539,6 +543,12 @@ __global__ void __launch_bounds__(kPcgThreads, 2) k_pcg_camera(DeviceBatch B) {
     z = B.pcg_z[i];
     v = B.pcg_v[i];
     p_old = B.pcg_p[i];  // used when k > 0
+  }
+  // what the last block will need of the state, off its serial path
+  if (t == kPcgThreads - 1 && live) {
+    const double lim = B.opt.pcg_tolerance * L->r0_norm;
+    sc[2] = recip_nr(rz_k);
+    sc[3] = lim * lim;
   }
   pdl_wait();  // the partials and the chunk values come from the mat-vec kernel
   double pq = 0.0, qex = 0.0;
@@ -596,7 +606,7 @@ __global__ void __launch_bounds__(kPcgThreads, 2) k_pcg_camera(DeviceBatch B) {
         for (int uu = 0; uu < kBatch; ++uu)
           if (sg + uu * kPcgSub < s1) a.add(pp[uu]);
       }
-      psub[sub][m] = a;
+      if (!ex) psub[sub][m] = a;
     }
     // p.q over the CTA (fixed order); thread 0 forms alpha once.  The FP64
     // form with the explicit complement sums the cameras' values in chunks
@@ -615,10 +625,30 @@ __global__ void __launch_bounds__(kPcgThreads, 2) k_pcg_camera(DeviceBatch B) {
       psf = df_warp_sum(psf);
       if ((t & 31) == 0) dfred[t >> 5] = psf;
     } else {
+      // (a warp whose threads have no value skips the addition of zeros)
 #pragma unroll
-      for (int j = 0; j < kCv; ++j) psm += cvl[j];
-      psm = warp_sum(psm);
-      if ((t & 31) == 0) red[t >> 5] = psm;
+      for (int j = 0; j < kCv; ++j)
+        if (j == 0 || (t & ~31) + j * kPcgThreads < n) psm += cvl[j];
+      if (MIXED) {
+        // explicit complement: the warps' butterflies eight at a time by the
+        // first warps, from psub's place (no partials), so that the FP64
+        // pipes get 27 additions of them instead of 90
+        double *lanes = reinterpret_cast<double *>(&psub[0][0]);
+        static_assert(!MIXED || sizeof(psub) >= sizeof(double) * kPcgThreads, "a value per thread");
+        lanes[t] = psm;
+        __syncthreads();
+        if (t < 32 * ((kPcgWarps + 7) / 8)) {
+          double v8[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) v8[j] = 8 * (t >> 5) + j < kPcgWarps ? lanes[32 * (8 * (t >> 5) + j) + (t & 31)] : 0.0;
+          const double s8 = warp_sum8(v8);
+          const int w = 8 * (t >> 5) + ((t & 31) >> 2);
+          if ((t & 3) == 0 && w < kPcgWarps) red[w] = s8;
+        }
+      } else {
+        psm = warp_sum(psm);
+        if ((t & 31) == 0) red[t >> 5] = psm;
+      }
     }
     __syncthreads();  // also publishes psub
     if (t == 0 && !(ex && !MIXED)) {
@@ -651,12 +681,14 @@ __global__ void __launch_bounds__(kPcgThreads, 2) k_pcg_camera(DeviceBatch B) {
     __syncthreads();
     double rz = 0.0, rr = 0.0, qx = 0.0;
     if (lead) {
-      // the sub-lane sums in order (compensated in the mixed form)
-      Acc comb = psub[0][m];
+      double qv = qex;
+      if (!ex) {
+        // the sub-lane sums in order (compensated in the mixed form)
+        Acc comb = psub[0][m];
 #pragma unroll
-      for (int j = 1; j < kPcgSub; ++j) comb.merge(psub[j][m]);
-      const double psum = comb.value();
-      const double qv = ex ? qex : a_times(arow, pv + 9 * lc, q) - psum;
+        for (int j = 1; j < kPcgSub; ++j) comb.merge(psub[j][m]);
+        qv = a_times(arow, pv + 9 * lc, q) - comb.value();
+      }
       x = fma(alpha, p, x);
       r = fma(-alpha, qv, r);
       rv[m] = (real)r;
@@ -692,54 +724,59 @@ __global__ void __launch_bounds__(kPcgThreads, 2) k_pcg_camera(DeviceBatch B) {
   // latency-bound loads and stores above
   pdl_launch_dependents();
   if (live && last_block_done(B.prob_counter + 4 * prob + kPC_UPDATE, (uint32_t)pi.cam_block_count, &flag)) {
-    // the blocks' values in block order: strided over the lanes of warp 0,
-    // then a butterfly (an order fixed by the block count)
-    if (t < 32) {
-      double a3[3] = {0.0, 0.0, 0.0};
-      if (good) {
-        for (int b = t; b < pi.cam_block_count; b += 32) {
-          const double *bv = B.blk_red + 3 * (size_t)(pi.cam_block_begin + b);
-          a3[0] += __ldcg(bv), a3[1] += __ldcg(bv + 1), a3[2] += __ldcg(bv + 2);
-        }
-        warp_sum3(a3[0], a3[1], a3[2]);
+    // the blocks' values in block order: strided over the lanes of a warp
+    // each, then a butterfly (an order fixed by the block count)
+    if (good && t < 96) {
+      const double *bv = B.blk_red + 3 * (size_t)pi.cam_block_begin + (t >> 5);
+      double a = 0.0;
+      for (int b = t & 31; b < pi.cam_block_count; b += 32 * 4) {
+        double v4[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v4[j] = b + 32 * j < pi.cam_block_count ? __ldcg(bv + 3 * (size_t)(b + 32 * j)) : 0.0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if ((b & ~31) + 32 * j < pi.cam_block_count) a += v4[j];
       }
-      if (t == 0) {
-        // the stopping test on (x_{k+1}, r_{k+1}) and beta_{k+1}, without
-        // FP64 division or square root (long sequences on GB300's FP64 pipe)
-        const double rz1 = a3[0], rr1 = a3[1], qk = -a3[2];  // Q(x) = x'Sx - 2 v'x = -x.(v + r)
-        const DeviceOptions &o = B.opt;
-        const int k1 = k + 1;  // completed iterations
-        bool stop = !good;     // no update: the PCG ends with x_k (a failed solve if k = 0)
-        if (good) {
-          if (o.pcg_criterion == GBA_PCG_QUADRATIC_MODEL) {
-            // zeta = k1 (Q_k1 - Q_k) / Q_k1 < eta, multiplied through by Q_k1
-            const double lhs = k1 * (qk - L->q0), rhs = o.eta * qk;
-            const bool below = qk > 0.0 ? lhs < rhs : (qk < 0.0 ? lhs > rhs : L->q0 > 0.0);
-            if (below && k1 >= o.min_pcg_iterations) stop = true;
-          } else {
-            const double lim = o.pcg_tolerance * L->r0_norm;  // |r| <= tol |r_0|
-            if (rr1 <= lim * lim && k1 >= o.min_pcg_iterations) stop = true;
-          }
-          if (k1 >= o.max_pcg_iterations) stop = true;
-          if (!(rz1 != 0.0 && isfinite(rz1))) stop = true;
-          L->pcg_iterations = k1;
-          L->beta = rz1 * recip_nr(rz_k);
-          L->rz = rz1;
-          L->rr = rr1;
-          L->q0 = qk;
-          L->pq = pq;
-        } else if (k == 0) {
-          L->linear_ok = 0;  // S not positive definite along the first direction
+      a = warp_sum(a);
+      if ((t & 31) == 0) red3[0][t >> 5] = a;
+    }
+    __syncthreads();
+    if (t == 0) {
+      const double a3[3] = {good ? red3[0][0] : 0.0, good ? red3[0][1] : 0.0, good ? red3[0][2] : 0.0};
+      // the stopping test on (x_{k+1}, r_{k+1}) and beta_{k+1}, without
+      // FP64 division or square root (long sequences on GB300's FP64 pipe)
+      const double rz1 = a3[0], rr1 = a3[1], qk = -a3[2];  // Q(x) = x'Sx - 2 v'x = -x.(v + r)
+      const DeviceOptions &o = B.opt;
+      const int k1 = k + 1;  // completed iterations
+      bool stop = !good;     // no update: the PCG ends with x_k (a failed solve if k = 0)
+      if (good) {
+        if (o.pcg_criterion == GBA_PCG_QUADRATIC_MODEL) {
+          // zeta = k1 (Q_k1 - Q_k) / Q_k1 < eta, multiplied through by Q_k1
+          const double lhs = k1 * (qk - L->q0), rhs = o.eta * qk;
+          const bool below = qk > 0.0 ? lhs < rhs : (qk < 0.0 ? lhs > rhs : L->q0 > 0.0);
+          if (below && k1 >= o.min_pcg_iterations) stop = true;
+        } else {
+          if (rr1 <= sc[3] && k1 >= o.min_pcg_iterations) stop = true;
         }
-        if (stop) {
-          L->pcg_active = 0;
-          atomicSub(B.status + 3, 1);
-        }
-        if (B.num_problems == 1) {
-          // the only problem decides the loop: no grid-wide count needed
-          B.status[2] = stop ? 0 : 1;
-          if (B.use_cond && B.pcg_cond) cudaGraphSetConditional((cudaGraphConditionalHandle)B.pcg_cond, stop ? 0u : 1u);
-        }
+        if (k1 >= o.max_pcg_iterations) stop = true;
+        if (!(rz1 != 0.0 && isfinite(rz1))) stop = true;
+        L->pcg_iterations = k1;
+        L->beta = rz1 * sc[2];
+        L->rz = rz1;
+        L->rr = rr1;
+        L->q0 = qk;
+        L->pq = pq;
+      } else if (k == 0) {
+        L->linear_ok = 0;  // S not positive definite along the first direction
+      }
+      if (stop) {
+        L->pcg_active = 0;
+        atomicSub(B.status + 3, 1);
+      }
+      if (B.num_problems == 1) {
+        // the only problem decides the loop: no grid-wide count needed
+        B.status[2] = stop ? 0 : 1;
+        if (B.use_cond && B.pcg_cond) cudaGraphSetConditional((cudaGraphConditionalHandle)B.pcg_cond, stop ? 0u : 1u);
       }
     }
   } else if (!live && B.num_problems == 1 && blockIdx.x == 0 && t == 0) {

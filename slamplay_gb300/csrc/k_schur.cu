@@ -24,7 +24,8 @@
 //                     (k, i).  The diagonal blocks B + Dc^2 - sum F_a F_a^T
 //                     come from K3b; a camera that sees a point twice has a
 //                     block (i, i) here for the cross terms.
-//  K4a' k_schur_spmv  one CTA per camera, one warp per row of its 9x9
+//  K4a' k_schur_spmv  (FP64: k_schur_spmv64) one CTA per camera, or
+//                     cameras in turn, one warp per row of its 9x9
 //                     blocks, the lanes over the row's blocks (the last
 //                     one the diagonal block): q = S p_k with p_k = z_k +
 //                     beta_k p_{k-1} formed on the fly exactly as the
@@ -259,107 +260,223 @@ void launch_schur_form(const DeviceBatch &b, bool mixed, cudaStream_t s) {
 // K4a'
 constexpr int kSpmvThreads = 9 * 32;
 constexpr int kSpmvStage = 96;  // blocks of a camera staged at a time (at most)
+constexpr int kSpmvCtas = 3;    // resident CTAs per SM
+constexpr int kSpmvKeep = 8;    // cameras whose row sums a CTA keeps before it writes them
 
 // Mixed form.  A lane that reads its block's row from memory touches a
 // 128-byte line of its own with every load, and so do its reads of the
-// direction: the L1's lines per load, not bytes, bounded the kernel.  So the
+// direction: the L1's lines per load, not bytes, bounded the kernel.  So a
 // camera's blocks, contiguous in memory, are copied into shared memory (16
-// bytes a copy, issued before the wait), the direction at their columns is
-// formed once for the nine rows, and both are read from there, an odd stride
-// between lanes (81 and 9 words: no bank conflicts).  `cap` (a multiple of
-// 32, at most kSpmvStage): blocks the stage holds; longer rows take rounds.
-// The rows' FP64 values are formed by one warp for all nine (a warp each
-// would queue on the FP64 pipes: 54 instead of 14 instructions a camera).
-// 1,800 cameras with 76 blocks each: 32.4 us with reads from memory, 26.7 now.
-__global__ void __launch_bounds__(kSpmvThreads) k_schur_spmv(DeviceBatch B, int cap) {
-  extern __shared__ __align__(16) float sv_smem[];  // [81 cap + 4] blocks, [9 cap] direction
-  __shared__ DF rows[9];
-  const int c = blockIdx.x, t = threadIdx.x;
-  const int q = t >> 5, lane = t & 31;
-  const int r0 = B.sblk_row[c], nb = B.sblk_row[c + 1] - r0;
-  float *sv = sv_smem, *sp = sv_smem + 81 * cap + 4;
-  // virtual block v of the row: v < nb the off-diagonal block r0 + v, v = nb
-  // the diagonal block; lane l takes v = l, l + 32, ...
-  const float *vals = reinterpret_cast<const float *>(B.sblk_val) + 81 * (size_t)r0;
-  const int off = r0 & 3;  // the stage keeps the source's place in its 16 bytes
-  const uint32_t sv0 = (uint32_t)__cvta_generic_to_shared(sv);
-  auto stage = [&](int v0) {  // blocks [v0, v0 + cap); v0 a multiple of 32
-    const int n = min(cap, nb - v0);
-    if (n > 0) {
-      const int chunks = (off + 81 * n + 3) >> 2;
-      const float *src = vals - off + 81 * (size_t)v0;
-      for (int i = t; i < chunks; i += kSpmvThreads)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(sv0 + 16u * (uint32_t)i), "l"(src + 4 * (size_t)i)
+// bytes a copy), the direction at their columns is formed once for the nine
+// rows, and both are read from there, an odd stride between lanes (81 and 9
+// words: no bank conflicts).  A camera needs a chain of loads (row, columns,
+// direction, blocks), so a CTA takes every gridDim-th camera: the blocks of the next two cameras, the direction of the
+// next and the columns of the one after are on their way while one is summed.
+// The first two cameras' blocks are copied before the wait.  `cap` (a
+// multiple of 32, at most kSpmvStage): blocks a stage holds; longer rows take
+// rounds.  The rows' FP64 values are formed together for up to kSpmvKeep
+// cameras (a warp for each row would queue on the FP64 pipes).  1,800 cameras
+// of 74 blocks: 32.4 us reading from memory, 26.4 staged with a CTA per
+// camera, 28.5 so pipelined with every warp reading the problem's state, 21.6
+// now; instruction issue bounds it (some 600 a warp and camera).
+__global__ void __launch_bounds__(kSpmvThreads, kSpmvCtas) k_schur_spmv(DeviceBatch B, int cap) {
+  extern __shared__ __align__(16) float sv_smem[];  // two stages of [81 cap + 4] blocks, [9 cap] direction
+  __shared__ float dg[81], own[kSpmvKeep][9];       // the diagonal block; the cameras' own direction
+  __shared__ DF rows[kSpmvKeep][9];
+  __shared__ double pqs[kSpmvKeep][9];
+  __shared__ int kcam[kSpmvKeep];
+  constexpr int kCols = 9 * kSpmvStage / kSpmvThreads;  // the direction's entries a thread forms
+  const int t = threadIdx.x, q = t >> 5, lane = t & 31;
+  float *sp = sv_smem + 2 * (81 * cap + 4);
+  const uint32_t sv0 = (uint32_t)__cvta_generic_to_shared(sv_smem);
+  struct Cam {
+    int c, r0, nb, prob;
+  };
+  auto cam_at = [&](int i) {  // the CTA's i-th camera
+    Cam m = {(int)(blockIdx.x + i * gridDim.x), 0, -1, -1};
+    if (m.c < B.nc) {
+      m.r0 = B.sblk_row[m.c];
+      m.nb = B.sblk_row[m.c + 1] - m.r0;
+      m.prob = B.cam_problem[m.c];
+    }
+    return m;
+  };
+  // The state of the cameras' problems: one thread reads it for the CTA (a
+  // line that every warp of the GPU asks for is served by one slice of the
+  // L2, a request a clock), past the L1, which would keep that of before the
+  // wait.  Before the wait a PCG that is seen ended has ended, so an early
+  // look only skips work.
+  struct State {
+    int live, k;
+    float beta;
+  };
+  __shared__ State state[4];  // of the CTA's i-th camera: i mod 4
+  State ns = {0, 0, 0.f};     // thread 0: the state read last, of problem nsp
+  int nsp = -1;
+  auto read_state = [&](const Cam &m) {
+    if (t == 0 && m.prob != nsp) {
+      nsp = m.prob;
+      ns = State{0, 0, 0.f};
+      if (nsp >= 0) {
+        const LMState *L = B.lm + nsp;
+        const int active = __ldcg(&L->active), pcg = __ldcg(&L->pcg_active), k = __ldcg(&L->pcg_iterations);
+        const double beta = __ldcg(&L->beta);
+        ns = State{active && pcg, k, (float)beta};
+      }
+    }
+  };
+  // blocks [v0, v0 + cap) of a camera's row, at their place in their 16 bytes
+  auto stage = [&](const Cam &m, int st, int v0, bool live) {
+    if (live) {
+      const int n = min(cap, m.nb - v0), off = m.r0 & 3;
+      const float *src = reinterpret_cast<const float *>(B.sblk_val) + 81 * (size_t)(m.r0 + v0) - off;
+      const uint32_t dst = sv0 + 4u * (uint32_t)(st * (81 * cap + 4));
+      for (int i = t; i < (n > 0 ? (off + 81 * n + 3) >> 2 : 0); i += kSpmvThreads)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16u * (uint32_t)i), "l"(src + 4 * (size_t)i)
                      : "memory");
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  const LMState *L = B.lm + B.cam_problem[c];
-  // (a PCG that has ended does not start again before the next camera-side
-  // kernel, so the early look only ever skips work; past the L1, which would
-  // keep the state of before the wait)
-  const bool hint = __ldcg(&L->active) && __ldcg(&L->pcg_active);
-  float diag = 0.f;
-  if (hint) {
-    stage(0);
-    if (t < 81) diag = (reinterpret_cast<const float *>(B.cam_Sii) + 81 * (size_t)c)[t];
-  }
-  pdl_wait_s();
-  pdl_launch_dependents_s();
-  if (!hint || !__ldcg(&L->pcg_active)) {  // uniform over the CTA
-    asm volatile("cp.async.wait_all;" ::: "memory");
-    return;
-  }
-  const int k = __ldcg(&L->pcg_iterations);
-  const float beta = (float)__ldcg(&L->beta);
+  // the cameras whose direction this thread forms entries of (the row's
+  // blocks in order, the diagonal block's, the camera itself, last)
+  auto columns = [&](const Cam &m, int v0, int (&col)[kCols]) {
+#pragma unroll
+    for (int j = 0; j < kCols; ++j) {
+      const int v = (t + j * kSpmvThreads) / 9;
+      col[j] = -1;
+      if (v < min(cap, m.nb + 1 - v0)) col[j] = v0 + v < m.nb ? B.sblk_col[m.r0 + v0 + v] : m.c;
+    }
+  };
   // p_k of a camera coordinate: the camera kernel's recurrence in FP32 on the
   // FP32 copies (as the implicit mat-vec)
-  auto pdir = [&](size_t idx) -> float {
-    const float z = B.pcg_zf[idx];
-    if (k == 0) return z;
-    return __fmaf_rn(beta, B.pcg_pf[idx], z);
+  auto load_zp = [&](const int (&col)[kCols], float (&z)[kCols], float (&p)[kCols]) {
+#pragma unroll
+    for (int j = 0; j < kCols; ++j) {
+      const int e = t + j * kSpmvThreads;
+      z[j] = p[j] = 0.f;
+      if (col[j] >= 0) {
+        const size_t idx = 9 * (size_t)col[j] + (e - 9 * (e / 9));
+        z[j] = B.pcg_zf[idx];
+        p[j] = B.pcg_pf[idx];  // used when k > 0
+      }
+    }
   };
-  DF af = df_zero();  // the lane's blocks in order
-  for (int v0 = 0; v0 <= nb; v0 += cap) {
-    const int n = min(cap, nb + 1 - v0);
-    if (v0 > 0) {
-      __syncthreads();  // the stage is reused
-      stage(v0);
-    }
-    for (int e = t; e < 9 * n; e += kSpmvThreads) {
-      const int v = e / 9, col = v0 + v < nb ? B.sblk_col[r0 + v0 + v] : c;
-      sp[e] = pdir(9 * (size_t)col + (e - 9 * v));
-    }
-    asm volatile("cp.async.wait_all;" ::: "memory");
-    __syncthreads();
-    if (nb - v0 < cap) {  // uniform; after the round's copies, which may share their last 16 bytes with it
-      if (t < 81) sv[off + 81 * (nb - v0) + t] = diag;
-      __syncthreads();
-    }
-    for (int v = lane; v < n; v += 32) {
-      const float *row = sv + off + 81 * v + 9 * q, *pp = sp + 9 * v;
-      float s = 0.f;
-#pragma unroll
-      for (int cc = 0; cc < 9; ++cc) s += row[cc] * pp[cc];
-      af = df_add(af, DF{s, 0.f});
-    }
-  }
-  // the row's sum over the lanes (butterfly: a fixed order)
-  af = df_warp_sum(af);
-  if (lane == 0) rows[q] = af;
+  const float *diag = reinterpret_cast<const float *>(B.cam_Sii);
+
+  Cam m0 = cam_at(0), m1 = cam_at(1), m2 = cam_at(2);
+  read_state(m0);
+  if (t == 0) state[0] = ns;
+  read_state(m1);
+  if (t == 0) state[1] = ns;
   __syncthreads();
-  if (t < 32) {
-    double pq = 0.0;
-    if (t < 9) {
-      const size_t i = 9 * (size_t)c + t;
-      const double qv = df_value(rows[t]);
-      B.pcg_q[i] = qv;
-      pq = (double)pdir(i) * qv;
+  stage(m0, 0, 0, state[0].live);
+  stage(m1, 1, 0, state[1].live);
+  int col1[kCols], col2[kCols];
+  columns(m0, 0, col1);
+  float d0 = m0.c < B.nc && t < 81 ? diag[81 * (size_t)m0.c + t] : 0.f;
+  __syncthreads();  // the early states are read
+  nsp = -1;
+  pdl_wait_s();
+  pdl_launch_dependents_s();
+  float z0[kCols], p0[kCols], zo = 0.f, po = 0.f;
+  load_zp(col1, z0, p0);
+  if (m0.c < B.nc && t < 9) zo = B.pcg_zf[9 * (size_t)m0.c + t], po = B.pcg_pf[9 * (size_t)m0.c + t];
+  columns(m1, 0, col1);
+  read_state(m0);
+  if (t == 0) state[0] = ns;
+  read_state(m1);
+  if (t == 0) state[1] = ns;
+  read_state(m2);
+  if (t == 0) state[2] = ns;
+  __syncthreads();
+  int kept = 0;
+  // the kept cameras' rows and their shares of p.q
+  auto write_kept = [&](int n) {
+    __syncthreads();
+    if (t < 9 * n) {
+      const int i = t / 9, r = t - 9 * i;
+      const double qv = df_value(rows[i][r]);
+      B.pcg_q[9 * (size_t)kcam[i] + r] = qv;
+      pqs[i][r] = (double)own[i][r] * qv;
     }
-    double s = 0.0;
+    __syncthreads();
+    if (t < n) {
+      double s = 0.0;
 #pragma unroll
-    for (int r = 0; r < 9; ++r) s += __shfl_sync(0xffffffffu, pq, r);
-    if (t == 0) B.spmv_red[c] = s;
+      for (int r = 0; r < 9; ++r) s += pqs[t][r];
+      B.spmv_red[kcam[t]] = s;
+    }
+  };
+  for (int i = 0; m0.c < B.nc; ++i) {
+    if (t == 0 && i > 0) state[(i + 2) & 3] = ns;
+    const int k = state[i & 3].k;
+    const float beta = state[i & 3].beta;
+    const bool live = state[i & 3].live;
+    auto pdir = [&](float z, float p) { return k == 0 ? z : __fmaf_rn(beta, p, z); };
+#pragma unroll
+    for (int j = 0; j < kCols; ++j) {
+      const int e = t + j * kSpmvThreads;
+      if (e < 9 * cap) sp[e] = pdir(z0[j], p0[j]);
+    }
+    if (t < 81) dg[t] = d0;
+    if (t < 9) own[kept][t] = pdir(zo, po);
+    // the next camera's direction, the columns after it, the row after those
+    if (m1.c < B.nc) {
+      load_zp(col1, z0, p0);
+      if (t < 9) zo = B.pcg_zf[9 * (size_t)m1.c + t], po = B.pcg_pf[9 * (size_t)m1.c + t];
+      if (t < 81) d0 = diag[81 * (size_t)m1.c + t];
+    }
+    columns(m2, 0, col2);
+    Cam m3 = cam_at(i + 3);
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncthreads();
+    const int st = i & 1;
+    if (live) {
+      const float *sv = sv_smem + st * (81 * cap + 4) + (m0.r0 & 3);
+      DF af = df_zero();  // the lane's blocks in order
+      for (int v0 = 0;;) {
+        const int n = min(cap, m0.nb + 1 - v0);
+        for (int v = lane; v < n; v += 32) {
+          const float *row = (v0 + v < m0.nb ? sv + 81 * v : dg) + 9 * q, *pp = sp + 9 * v;
+          float s = 0.f;
+#pragma unroll
+          for (int cc = 0; cc < 9; ++cc) s += row[cc] * pp[cc];
+          af = df_add(af, DF{s, 0.f});
+        }
+        if ((v0 += cap) > m0.nb) break;
+        // a row longer than the stage: its next round, in line
+        __syncthreads();
+        stage(m0, st, v0, true);
+        int col[kCols];
+        float z[kCols], p[kCols];
+        columns(m0, v0, col);
+        load_zp(col, z, p);
+#pragma unroll
+        for (int j = 0; j < kCols; ++j) {
+          const int e = t + j * kSpmvThreads;
+          if (e < 9 * cap) sp[e] = pdir(z[j], p[j]);
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
+      }
+      // the row's sum over the lanes (butterfly: a fixed order)
+      af = df_warp_sum(af);
+      if (lane == 0) rows[kept][q] = af;
+      if (t == 0) kcam[kept] = m0.c;
+    }
+    __syncthreads();  // the stage is free
+    stage(m2, st, 0, state[(i + 2) & 3].live);
+    read_state(m3);
+    if (live && ++kept == kSpmvKeep) {
+      write_kept(kept);
+      kept = 0;
+    }
+    m0 = m1, m1 = m2, m2 = m3;
+#pragma unroll
+    for (int j = 0; j < kCols; ++j) col1[j] = col2[j];
   }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  if (kept > 0) write_kept(kept);
 }
 
 // K4a' of the FP64 form: one CTA per camera; the direction p_k = z_k +
@@ -463,7 +580,14 @@ cudaError_t launch_schur_spmv(const DeviceBatch &b, bool mixed, cudaStream_t s, 
   cfg.numAttrs = pdl ? 1 : 0;
   if (mixed) {
     const int cap = std::min((b.sblk_max + 31) / 32 * 32, kSpmvStage);
-    cfg.dynamicSmemBytes = sizeof(float) * (90 * (size_t)cap + 4);
+    const size_t bytes = sizeof(float) * (2 * (81 * (size_t)cap + 4) + 9 * (size_t)cap);
+    int sms = 0, dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess) e = raise_smem_limit((const void *)k_schur_spmv, bytes);
+    if (e != cudaSuccess) return e;
+    cfg.gridDim = dim3((unsigned)std::min(b.nc, kSpmvCtas * sms));
+    cfg.dynamicSmemBytes = bytes;
     return cudaLaunchKernelEx(&cfg, k_schur_spmv, b, cap);
   }
   size_t smem = 0;

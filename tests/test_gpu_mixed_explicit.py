@@ -30,26 +30,45 @@ def _dense(nc, npt, seed):
     return BALProblem.from_arrays(nc, npt, ci, pi, obs, b.parameters())
 
 
+def _scale(d):
+    with Solver() as s:
+        _, J, _ = s.evaluate(d)
+    sq = (J * J).sum(axis=1)
+    cam, pt = np.zeros((d.num_cameras(), 9)), np.zeros((d.num_points(), 3))
+    np.add.at(cam, d.camera_index(), sq[:, :9])
+    np.add.at(pt, d.point_index(), sq[:, 9:])
+    return 1.0 + np.sqrt(np.concatenate([cam.ravel(), pt.ravel()]))
+
+
 def _step_error(d, persistent):
     opts = dict(pcg_tolerance=1e-8, max_linear_solver_iterations=500)
     with Solver(precision="mixed", schur="explicit", persistent_pcg=persistent, **opts) as s:
         step, _, _ = s.compute_step(d, 1.0)
-        _, J, _ = s.evaluate(d)
     want, _, _, ok = O.compute_step(O.Problem.from_bal(d), 1.0, linear_solver="pcg_schur", pcg_tolerance=1e-12,
                                     max_linear_solver_iterations=1000)
     assert ok
-    nc, npt = d.num_cameras(), d.num_points()
-    sq = (J * J).sum(axis=1)
-    cam, pt = np.zeros((nc, 9)), np.zeros((npt, 3))
-    np.add.at(cam, d.camera_index(), sq[:, :9])
-    np.add.at(pt, d.point_index(), sq[:, 9:])
-    scale = 1.0 + np.sqrt(np.concatenate([cam.ravel(), pt.ravel()]))
+    scale = _scale(d)
     return np.linalg.norm(scale * (step - want)) / np.linalg.norm(scale * want)
 
 
 @pytest.mark.parametrize("npt", [1, 2, 3, 4, 63, 64, 65, 66, 67, 129, 191])
 def test_formation_pair_counts(npt):
     assert _step_error(_dense(4, npt, 40 + npt), 1) <= 1e-4
+
+
+@pytest.mark.parametrize("nc", [455, 460, 1000, 3700])
+def test_product_cameras_per_cta(nc):
+    """Up to eight and more cameras a CTA, one after the other: the PCG's
+    iterates depend on every row, so a wrong or missing one shows in the
+    step (FP32 blocks against the implicit FP64 step; the bound above)."""
+    b = BALProblem.synthetic(1, seed=nc, num_cameras=nc, num_points=4 * nc)
+    opts = dict(pcg_tolerance=1e-8, max_linear_solver_iterations=500)
+    with Solver(precision="mixed", schur="explicit", persistent_pcg=0, **opts) as s:
+        step, _, _ = s.compute_step(b, 1.0)
+    with Solver(schur="implicit", **opts) as s:
+        want, _, _ = s.compute_step(b, 1.0)
+    scale = _scale(b)
+    assert np.linalg.norm(scale * (step - want)) <= 1e-4 * np.linalg.norm(scale * want)
 
 
 @pytest.mark.parametrize("nc", [3, 31, 32, 33, 95, 96, 97, 193])
