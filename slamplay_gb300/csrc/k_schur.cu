@@ -44,9 +44,8 @@ namespace gba {
 
 namespace {
 
-constexpr int kFormThreads = 256;
-constexpr int kFormPairs = 64;  // pairs staged per round
-constexpr int kFormSub = 3;     // sub-lanes per block entry (243 of the 256 threads)
+constexpr int kFormPairs = 64;  // pairs per round
+constexpr int kFormSub = 3;     // sub-lanes (interleaved runs) per block entry
 
 __device__ __forceinline__ void pdl_wait_s() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents_s() {
@@ -56,85 +55,84 @@ __device__ __forceinline__ void pdl_launch_dependents_s() {
 }  // namespace
 
 // ---------------------------------------------------------------------------
-// K3c of the FP64 form: the FP64 pipe bounds it (243 FMAs a pair, one warp
-// instruction per 64 clocks per sub-partition: 92 % of that on 250 cameras).
-__global__ void __launch_bounds__(kFormThreads) k_schur_form(DeviceBatch B) {
-  typedef double real;
-  typedef double2 vec;
-  constexpr int kVec = (int)(sizeof(vec) / sizeof(real));
-  constexpr int kRowVecs = kObsF / kVec;  // 16-byte loads per F row
-  constexpr int kRoundVecs = kFormPairs * 2 * kRowVecs;
-  constexpr int kPer = (kRoundVecs + kFormThreads - 1) / kFormThreads;  // loads per thread per round
-  static_assert(kObsF % kVec == 0, "F rows are whole 16-byte vectors");
-  __shared__ __align__(16) real Fs[kFormPairs][2][kObsF];  // F of the row's and the column's observation
-  __shared__ double part[kFormSub][81];
-  const int ub = blockIdx.x, t = threadIdx.x;
-  const int blk = B.sblk_up[ub];
+// K3c of the FP64 form, two CTAs a block (entries 0-40 and 41-80).  The FP64
+// pipe bounds it: 243 FMAs a pair at one warp instruction per 64 clocks per
+// sub-partition, dependent or not.  With four warps a CTA a lone block's
+// three runs go at the chain's own speed (eight warps for all 81 entries on
+// one SM take twice as long), and many blocks fill the GPU as before.  Every
+// warp copies the F rows of eight of 32 pairs, asynchronously, the next 32's
+// in flight while one is summed.  One CTA of eight warps a block, and now: 43
+// and 27 us (rig window, blocks of up to 500 pairs), 53 and 41 (23 cameras),
+// 520 and 430 (48 windows), 488 and 454 (250 cameras, 883,000 pairs; the
+// FMAs alone 342).
+constexpr int kForm64Warps = 4;
+constexpr int kForm64Pairs = 32;
+constexpr int kForm64Split = 41;  // entries of the first CTA
+static_assert(kFormPairs == 2 * kForm64Pairs && kForm64Split * kFormSub <= 32 * kForm64Warps, "rounds and threads");
+
+__global__ void __launch_bounds__(32 * kForm64Warps) k_schur_form(DeviceBatch B) {
+  __shared__ __align__(16) double Fs[2][kForm64Pairs][2][kObsF];
+  __shared__ double part[kFormSub][kForm64Split];
+  constexpr int kWarpPairs = kForm64Pairs / kForm64Warps, kRowVecs = kObsF / 2;
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  const int ub = blockIdx.x >> 1, blk = B.sblk_up[ub];
   const int p0 = B.sblk_pair[ub], p1 = B.sblk_pair[ub + 1];
-  const LMState *L = B.lm + B.cam_problem[B.sblk_col[blk]];
-  if (!L->active) return;  // uniform
-  const real *F = reinterpret_cast<const real *>(B.obs_F);
-  // a round's F rows: every load issued before any is stored (one L2 round
-  // trip per round), the next round's loaded while this one is summed
-  vec buf[kPer];
-  auto load_round = [&](int g) {
-    const int n = min(kFormPairs, p1 - g);
-#pragma unroll
-    for (int u = 0; u < kPer; ++u) {
-      const int i = t + u * kFormThreads;
-      if (i < n * 2 * kRowVecs) {
-        const int pr = i / (2 * kRowVecs), r = i - 2 * kRowVecs * pr;
-        const int side = r / kRowVecs, e = r - kRowVecs * side;
-        const int2 ob = B.spair[g + pr];
-        buf[u] = reinterpret_cast<const vec *>(F + (size_t)kObsF * (side ? ob.y : ob.x))[e];
-      }
-    }
+  if (!B.lm[B.cam_problem[B.sblk_col[blk]]].active) return;  // uniform
+  const double *F = reinterpret_cast<const double *>(B.obs_F);
+  const int *pairs = reinterpret_cast<const int *>(B.spair);
+  const int w0 = kWarpPairs * warp;
+  // lane l < 16: the observation of the warp's pair l / 2, the row's (even) or the column's
+  auto load_index = [&](int g) {
+    return lane < 2 * kWarpPairs && g + w0 + (lane >> 1) < p1 ? pairs[2 * (size_t)(g + w0) + lane] : 0;
   };
-  auto store_round = [&](int g) {
-    const int n = min(kFormPairs, p1 - g);
+  auto stage_rows = [&](int g, int st, int ob) {
+    const int rows = 2 * (p1 - g - w0);
+    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&Fs[st][w0][0][0]);
 #pragma unroll
-    for (int u = 0; u < kPer; ++u) {
-      const int i = t + u * kFormThreads;
-      if (i < n * 2 * kRowVecs) {
-        const int pr = i / (2 * kRowVecs), r = i - 2 * kRowVecs * pr;
-        const int side = r / kRowVecs, e = r - kRowVecs * side;
-        *reinterpret_cast<vec *>(&Fs[pr][side][kVec * e]) = buf[u];
-      }
+    for (int u = 0; u < 2 * kWarpPairs * kRowVecs / 32; ++u) {
+      const int i = lane + 32 * u, row = i / kRowVecs, e = i - kRowVecs * row;
+      const int o = __shfl_sync(0xffffffffu, ob, row);
+      if (row < rows)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16u * (uint32_t)i),
+                     "l"(F + (size_t)kObsF * o + 2 * e)
+                     : "memory");
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  // sub-lane `sub` of entry (i, k) sums the pairs sub, sub + kFormSub, ...
-  // of every round, in order
-  const int sub = t / 81, en = t - 81 * sub, ei = en / 9, ek = en - 9 * ei;
+  // sub-lane `sub` of entry (i, k) sums the pairs sub, sub + kFormSub, ... of
+  // every round of 64, in order: one FMA chain through the accumulator (three
+  // FP64 operations a pair, not four)
+  const int e0 = (blockIdx.x & 1) * kForm64Split, cnt = min(kForm64Split, 81 - e0);
+  const int sub = t / cnt, en = e0 + t - cnt * sub, ei = en / 9, ek = en - 9 * ei;
   double acc = 0.0;
-  load_round(p0);
-  store_round(p0);
-  __syncthreads();
-  for (int g = p0; g < p1; g += kFormPairs) {
-    const int n = min(kFormPairs, p1 - g);
-    const bool more = g + kFormPairs < p1;
-    if (more) load_round(g + kFormPairs);
+  stage_rows(p0, 0, load_index(p0));
+  int ob = load_index(p0 + kForm64Pairs);
+  int u = sub;  // the run's next pair of the round
+  for (int g = p0, it = 0; g < p1; g += kForm64Pairs, ++it) {
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();  // these pairs have landed; every warp is done with the ones before
+    stage_rows(g + kForm64Pairs, (it & 1) ^ 1, ob);
+    ob = load_index(g + 2 * kForm64Pairs);
+    const int base = kForm64Pairs * (it & 1), lim = base + min(kForm64Pairs, p1 - g);
     if (sub < kFormSub)
-      for (int u = sub; u < n; u += kFormSub) {
-        const real *fa = &Fs[u][0][3 * ei], *fb = &Fs[u][1][3 * ek];
-        // one FMA chain through the accumulator (three FP64 operations a pair, not four)
+#pragma unroll 4
+      for (; u < lim; u += kFormSub) {
+        const double *fa = &Fs[it & 1][u - base][0][3 * ei], *fb = &Fs[it & 1][u - base][1][3 * ek];
         acc = fma(fa[2], fb[2], fma(fa[1], fb[1], fma(fa[0], fb[0], acc)));
       }
-    __syncthreads();  // the stage is reused
-    if (more) store_round(g + kFormPairs);
-    __syncthreads();
+    if (it & 1) u = sub;
   }
-  if (sub < kFormSub) part[sub][en] = acc;
+  if (sub < kFormSub) part[sub][en - e0] = acc;
   __syncthreads();
-  if (t < 81) {
+  if (t < cnt) {
     double s = part[0][t];
 #pragma unroll
     for (int j = 1; j < kFormSub; ++j) s += part[j][t];
-    const real v = -s;
-    real *vals = reinterpret_cast<real *>(B.sblk_val);
-    const int i = t / 9, k = t - 9 * i;
-    vals[81 * (size_t)blk + t] = v;
-    const int tr = B.sblk_tr[blk];
-    if (tr != blk) vals[81 * (size_t)tr + 9 * k + i] = v;
+    const double v = -s;
+    double *vals = reinterpret_cast<double *>(B.sblk_val);
+    const int e = e0 + t, tr = B.sblk_tr[blk];
+    vals[81 * (size_t)blk + e] = v;
+    if (tr != blk) vals[81 * (size_t)tr + 9 * (e % 9) + e / 9] = v;
   }
 }
 
@@ -253,7 +251,7 @@ void launch_schur_form(const DeviceBatch &b, bool mixed, cudaStream_t s) {
   if (mixed)
     k_schur_form_mixed<<<b.nup, 32 * kTileWarps, 0, s>>>(b);
   else
-    k_schur_form<<<b.nup, kFormThreads, 0, s>>>(b);
+    k_schur_form<<<2 * b.nup, 32 * kForm64Warps, 0, s>>>(b);
 }
 
 // ---------------------------------------------------------------------------

@@ -61,16 +61,18 @@ struct PointSchurSmem {
 
 // Lower Cholesky factor of a symmetric 3x3 (packed 00 01 02 11 12 22):
 // l00 l10 l11 l20 l21 l22, zero where a pivot is not positive.
-__device__ __forceinline__ void chol3(const double *A, double *L) {
-  const double l00 = A[0] > 0.0 ? sqrt(A[0]) : 0.0;
-  const double i00 = l00 > 0.0 ? recip_nr(l00) : 0.0;
+// inv: the reciprocals of the first two pivots (zero for a zero pivot).
+__device__ __forceinline__ void chol3(const double *A, double *L, double inv[2]) {
+  const double l00 = positive64(A[0]) ? sqrt(A[0]) : 0.0;
+  const double i00 = positive64(l00) ? recip_nr(l00) : 0.0;
   const double l10 = A[1] * i00, l20 = A[2] * i00;
   const double d1 = A[3] - l10 * l10;
-  const double l11 = d1 > 0.0 ? sqrt(d1) : 0.0;
-  const double i11 = l11 > 0.0 ? recip_nr(l11) : 0.0;
+  const double l11 = positive64(d1) ? sqrt(d1) : 0.0;
+  const double i11 = positive64(l11) ? recip_nr(l11) : 0.0;
   const double l21 = (A[4] - l20 * l10) * i11;
   const double d2 = A[5] - l20 * l20 - l21 * l21;
-  const double l22 = d2 > 0.0 ? sqrt(d2) : 0.0;
+  const double l22 = positive64(d2) ? sqrt(d2) : 0.0;
+  inv[0] = i00, inv[1] = i11;
   L[0] = l00, L[1] = l10, L[2] = l11, L[3] = l20, L[4] = l21, L[5] = l22;
 }
 
@@ -142,8 +144,8 @@ __global__ void __launch_bounds__(kChunkCap, MIXED ? 4 : 1) k_point_schur(Device
       B.pt_t[3 * (size_t)j + 2] = t2;
       sm.tp[t][0] = (real)t0, sm.tp[t][1] = (real)t1, sm.tp[t][2] = (real)t2;
       if (B.explicit_schur) {
-        double Lc[6];
-        chol3(Ci, Lc);
+        double Lc[6], inv[2];
+        chol3(Ci, Lc, inv);
 #pragma unroll
         for (int q = 0; q < 6; ++q) sm.lc[t][q] = (real)Lc[q];
       }
@@ -240,13 +242,16 @@ __global__ void __launch_bounds__(kChunkCap, MIXED ? 4 : 1) k_point_schur(Device
 // (W C^-1 W^T = F F^T), and of the reduced rhs, sum_obs F_a . u
 // (J_c^T J_p t = F L^-1 t): three FMAs an entry and observation where the
 // general kernel's J_c^T A J_c takes seven, GB300's FP64 pipe being what
-// bounds this kernel.
+// bounds this kernel: comparisons are integer instructions, the damping has
+// a thread per diagonal entry, the two kinds of sums share one loop.  Without
+// these 47 us on small problems, 234 on 48 windows and 241 on 250 cameras
+// (295,000 observations); 32, 163 and 171 with them.
 struct PointSchurEx64Smem {
   double F[kChunkCap][27];  // F by slot
-  double ci[kChunkCap][6];  // C^-1 by chunk point
+  double us[kChunkCap][3];  // L^-1 t by slot
   double u[kChunkCap][3];   // L^-1 t by chunk point
   double lc[kChunkCap][6];  // L by chunk point
-  int spt[kChunkCap];       // chunk point of each slot
+  double cd[kChunkCap][3];  // the damped diagonal of C by chunk point
 };
 
 __global__ void __launch_bounds__(kChunkCap) k_point_schur_ex64(DeviceBatch B) {
@@ -268,17 +273,22 @@ __global__ void __launch_bounds__(kChunkCap) k_point_schur_ex64(DeviceBatch B) {
       for (int q = 0; q < 3; ++q) Jp[q] = jload<double2>(B.jac, B.no, 9 + q, o);
       slot = B.obs_slot[o];
       lp = B.obs_pt[o] - ci.pt_begin;
-      sm.spt[slot] = lp;
     }
+    // the damping's divisions and square roots, a thread for each diagonal
+    // entry: the points alone would keep one or two of the four
+    // sub-partitions busy
+    for (int i = t; i < 3 * ci.pt_count; i += kChunkCap) {
+      const int pt = i / 3, q = i - 3 * pt;
+      const double c = B.pt_C[6 * (size_t)(ci.pt_begin + pt) + (q == 0 ? 0 : 2 * q + 1)];
+      sm.cd[pt][q] = c + lm_d2(c, L->radius, B.opt);
+    }
+    __syncthreads();
     if (t < ci.pt_count) {
       const int j = ci.pt_begin + t;
-      const double radius = L->radius;
       double C[6];
 #pragma unroll
       for (int q = 0; q < 6; ++q) C[q] = B.pt_C[6 * (size_t)j + q];
-      C[0] += lm_d2(C[0], radius, B.opt);
-      C[3] += lm_d2(C[3], radius, B.opt);
-      C[5] += lm_d2(C[5], radius, B.opt);
+      C[0] = sm.cd[t][0], C[3] = sm.cd[t][1], C[5] = sm.cd[t][2];
       double Ci[6];
       if (!spd_inverse3(C, Ci)) {
         L->linear_ok = 0;  // benign race: every writer stores 0
@@ -290,7 +300,6 @@ __global__ void __launch_bounds__(kChunkCap) k_point_schur_ex64(DeviceBatch B) {
       for (int q = 0; q < 6; ++q) {
         cio[q] = Ci[q];
         B.pt_Cinv64[6 * (size_t)j + q] = Ci[q];
-        sm.ci[t][q] = Ci[q];
       }
       const double *g = B.pt_g + 3 * (size_t)j;
       const double g0 = g[0], g1 = g[1], g2 = g[2];
@@ -300,16 +309,14 @@ __global__ void __launch_bounds__(kChunkCap) k_point_schur_ex64(DeviceBatch B) {
       B.pt_t[3 * (size_t)j + 0] = t0;
       B.pt_t[3 * (size_t)j + 1] = t1;
       B.pt_t[3 * (size_t)j + 2] = t2;
-      double Lc[6];
-      chol3(Ci, Lc);
+      double Lc[6], inv[2];
+      chol3(Ci, Lc, inv);
 #pragma unroll
       for (int q = 0; q < 6; ++q) sm.lc[t][q] = Lc[q];
       // u = L^-1 t (forward substitution; a zero pivot gives a zero component)
-      const double i00 = Lc[0] > 0.0 ? recip_nr(Lc[0]) : 0.0;
-      const double i11 = Lc[2] > 0.0 ? recip_nr(Lc[2]) : 0.0;
-      const double i22 = Lc[5] > 0.0 ? recip_nr(Lc[5]) : 0.0;
-      const double u0 = t0 * i00;
-      const double u1 = (t1 - Lc[1] * u0) * i11;
+      const double i22 = positive64(Lc[5]) ? recip_nr(Lc[5]) : 0.0;
+      const double u0 = t0 * inv[0];
+      const double u1 = (t1 - Lc[1] * u0) * inv[1];
       const double u2 = (t2 - Lc[3] * u0 - Lc[4] * u1) * i22;
       sm.u[t][0] = u0, sm.u[t][1] = u1, sm.u[t][2] = u2;
     }
@@ -340,6 +347,8 @@ __global__ void __launch_bounds__(kChunkCap) k_point_schur_ex64(DeviceBatch B) {
       F[27] = 0.0;
 #pragma unroll
       for (int e = 0; e < 27; ++e) sm.F[slot][e] = F[e];
+#pragma unroll
+      for (int e = 0; e < 3; ++e) sm.us[slot][e] = sm.u[lp][e];
       double2 *dst = reinterpret_cast<double2 *>(reinterpret_cast<double *>(B.obs_F) +
                                                  (size_t)kObsF * B.obs_fpos[ci.obs_begin + t]);
 #pragma unroll
@@ -355,21 +364,16 @@ __global__ void __launch_bounds__(kChunkCap) k_point_schur_ex64(DeviceBatch B) {
         b1 = (sg + 1 < ci.seg_count) ? B.seg_pos[ci.seg_begin + sg + 1] : ci.obs_count;
         sl = B.seg_slot[ci.seg_begin + sg];
       }
+      // F_a . F_b of entry (a, b), or F_a . u: one loop for both (a warp
+      // holds lanes of both kinds and would run two, one after the other)
+      int a = en - 45, b = 0;
+      if (en < 45) sym9_pair(en, a, b);
+      const double *fa = sm.F[b0] + 3 * a, *fb = en < 45 ? sm.F[b0] + 3 * b : sm.us[b0];
+      const int step = en < 45 ? 27 : 3;
       double acc = 0.0;
-      if (en < 45) {
-        int a, b;
-        sym9_pair(en, a, b);
-        for (int k = b0; k < b1; ++k) {
-          const double *fa = sm.F[k] + 3 * a, *fb = sm.F[k] + 3 * b;
-          acc = fma(fa[2], fb[2], fma(fa[1], fb[1], fma(fa[0], fb[0], acc)));
-        }
-      } else {
-        const int a = en - 45;
-        for (int k = b0; k < b1; ++k) {
-          const double *fa = sm.F[k] + 3 * a, *u = sm.u[sm.spt[k]];
-          acc = fma(fa[2], u[2], fma(fa[1], u[1], fma(fa[0], u[0], acc)));
-        }
-      }
+#pragma unroll 4
+      for (int k = b0; k < b1; ++k, fa += 27, fb += step)
+        acc = fma(fa[2], fb[2], fma(fa[1], fb[1], fma(fa[0], fb[0], acc)));
       part[54 * (size_t)sl + en] = acc;
     }
     __syncthreads();

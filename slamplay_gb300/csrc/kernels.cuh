@@ -343,6 +343,11 @@ __device__ __forceinline__ bool finite64(double v) { return (__double2hiint(v) &
 __device__ __forceinline__ double max_nonneg(double a, double b) {
   return __longlong_as_double(max(__double_as_longlong(a), __double_as_longlong(b)));
 }
+// v > 0 (false for a NaN).
+__device__ __forceinline__ bool positive64(double v) {
+  const long long b = __double_as_longlong(v);
+  return b > 0 && b <= 0x7ff0000000000000LL;
+}
 // |v|, 0 for a NaN (what fmax(0, |v|) gives).
 __device__ __forceinline__ double abs_or_0(double v) {
   const long long b = __double_as_longlong(v) & 0x7fffffffffffffffLL;
@@ -825,7 +830,7 @@ __device__ __forceinline__ bool spd_inverse3(const double *C, double *Ci) {
   const double m12 = b * c - a * e;
   const double m22 = a * d - b * b;
   const double det = a * m00 + b * m01 + c * m02;
-  if (!(a > 0.0) || !(m22 > 0.0) || !(det > 0.0)) return false;
+  if (!positive64(a) || !positive64(m22) || !positive64(det)) return false;
   const double id = recip_nr(det);
   Ci[0] = m00 * id;
   Ci[1] = m01 * id;
@@ -833,7 +838,7 @@ __device__ __forceinline__ bool spd_inverse3(const double *C, double *Ci) {
   Ci[3] = m11 * id;
   Ci[4] = m12 * id;
   Ci[5] = m22 * id;
-  return isfinite(Ci[0]) && isfinite(Ci[3]) && isfinite(Ci[5]);
+  return finite64(Ci[0]) && finite64(Ci[3]) && finite64(Ci[5]);
 }
 
 // ---------------------------------------------------------------------------
