@@ -873,7 +873,7 @@ __device__ void finish_lm_body(const DeviceBatch &B, bool count_body) {
 
 // K7: one CTA per problem.
 __global__ void __launch_bounds__(256) k_post_eval(DeviceBatch B, int count_body) {
-  __shared__ double red[8 * 6];
+  __shared__ double red[257 * 6];
   const int p = blockIdx.x;
   LMState *L = B.lm + p;
   if (L->active && L->need_jacobian) {

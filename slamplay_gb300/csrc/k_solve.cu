@@ -600,7 +600,7 @@ __global__ void __launch_bounds__(kChunkCap) k_back_substitute(DeviceBatch B) {
   __shared__ real yseg[kChunkCap][9];
   __shared__ real W[kChunkCap][3];
   __shared__ real ypt[kChunkCap][3];
-  __shared__ double red[kChunkCap / 32];
+  __shared__ double red[2 * (kChunkCap / 32) + 1];
   const int t = threadIdx.x;
   for (int ch = blockIdx.x; ch < B.nchunks; ch += gridDim.x) {
     const ChunkInfo ci = B.chunk[ch];
@@ -674,12 +674,11 @@ __global__ void __launch_bounds__(kChunkCap) k_back_substitute(DeviceBatch B) {
       // above, camera part in K5b); only |m|^2 / 2 comes from the FP32 copies
       model += MIXED ? (m0 * m0 + m1 * m1) / 2.0 : m0 * (ru + m0 / 2.0) + m1 * (rv + m1 / 2.0);
     }
-    const double ms = block_sum(model, red);
-    const double ss = block_sum(s2, red);
-    if (t == 0) {
-      B.chunk_scal[(size_t)kChunkScal * ch + kCS_MODEL] = ms;
-      B.chunk_scal[(size_t)kChunkScal * ch + kCS_STEP2] = ss;
-    }
+    double gmax;
+    bool any;
+    const double sum = block_sums2_max(model, s2, 0.0, false, red, &gmax, &any);
+    if (t == 0) B.chunk_scal[(size_t)kChunkScal * ch + kCS_MODEL] = sum;
+    if (t == 32) B.chunk_scal[(size_t)kChunkScal * ch + kCS_STEP2] = sum;
   }
 }
 
@@ -742,7 +741,7 @@ __device__ void decide_g2o(const DeviceBatch &B, int p, LMState *L, int it, int 
 }
 
 __global__ void __launch_bounds__(256) k_decide(DeviceBatch B) {
-  __shared__ double red[8 * 6];
+  __shared__ double red[257 * 6];
   const int p = blockIdx.x;
   LMState *L = B.lm + p;
   if (!L->active) return;

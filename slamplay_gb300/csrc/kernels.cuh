@@ -422,40 +422,54 @@ __device__ __forceinline__ double block_range_max(const double *a, int begin, in
   return block_max(s, red);
 }
 
-// N range reductions in one pass (one round of loads, one set of barriers):
-// value j is the sum, or with is_max[j] the maximum (from 0), of a[j][i *
+// N range reductions in one pass (one round of loads, one set of barriers) by
+// a CTA of 256 threads: value j is the sum, or with is_max[j] the maximum
+// (from 0, of values that are not negative; a NaN counts as 0), of a[j][i *
 // stride[j]] over i in [begin[j], end[j]), each in exactly the order of its
-// own block_range_sum / block_range_max (so the same bits).  The totals are
-// valid in thread 0.  `red` needs (blockDim / 32) * N doubles.
+// own block_range_sum (so the same bits): the strided sums, the eight warps'
+// butterflies by one warp for each value, the warps' sums in order.  (Six
+// values with a butterfly of every warp for each and thread 0 adding the
+// warps' sums: 108 FP64 instructions one after the other on a sub-partition,
+// 17 now.)  The totals are valid in thread 0.  `red` needs 257 * N doubles.
 template <int N>
 __device__ __forceinline__ void block_range_multi(const double *const (&a)[N], const int (&begin)[N],
                                                   const int (&end)[N], const int (&stride)[N],
                                                   const bool (&is_max)[N], double (&out)[N], double *red) {
-  double v[N];
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
 #pragma unroll
   for (int j = 0; j < N; ++j) {
-    v[j] = 0.0;
+    double v = 0.0;
 #pragma unroll 8
-    for (int i = begin[j] + threadIdx.x; i < end[j]; i += blockDim.x) {
+    for (int i = begin[j] + t; i < end[j]; i += 256) {
       const double x = __ldcg(a[j] + (size_t)i * stride[j]);
-      v[j] = is_max[j] ? fmax(v[j], x) : v[j] + x;
+      v = is_max[j] ? max_nonneg(v, abs_or_0(x)) : v + x;
     }
+    red[256 * j + t] = v;
   }
-#pragma unroll
-  for (int j = 0; j < N; ++j) v[j] = is_max[j] ? warp_max(v[j]) : warp_sum(v[j]);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   __syncthreads();
-  if (lane == 0)
 #pragma unroll
-    for (int j = 0; j < N; ++j) red[N * warp + j] = v[j];
-  __syncthreads();
-  if (threadIdx.x == 0)
+  for (int j = 0; j < N; ++j)
+    if (warp == j) {
+      double v8[8], s = 0.0;
 #pragma unroll
-    for (int j = 0; j < N; ++j) {
-      double s = 0.0;
-      for (int w = 0; w < nw; ++w) s = is_max[j] ? fmax(s, red[N * w + j]) : s + red[N * w + j];
-      out[j] = s;
+      for (int w = 0; w < 8; ++w) v8[w] = red[256 * j + 32 * w + lane];
+      if (is_max[j]) {
+#pragma unroll
+        for (int w = 0; w < 8; ++w) s = max_nonneg(s, v8[w]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s = max_nonneg(s, __shfl_xor_sync(0xffffffffu, s, o));
+      } else {
+        const double b = warp_sum8(v8);
+#pragma unroll
+        for (int w = 0; w < 8; ++w) s += __shfl_sync(0xffffffffu, b, 4 * w);
+      }
+      if (lane == 0) red[256 * N + j] = s;
     }
+  __syncthreads();
+  if (t == 0)
+#pragma unroll
+    for (int j = 0; j < N; ++j) out[j] = red[256 * N + j];
+  static_assert(N <= 8, "a warp for each value");
 }
 
 // "Last CTA done" detection without waiting: each CTA bumps a counter after
