@@ -166,6 +166,8 @@ static inline void atomic_min_i64(std::atomic<long long> &a, long long v) {
 
 // Loops with fewer elements than this run on the calling thread.
 constexpr long long kParMin = 32768;
+// Observations per run of a large problem's first passes.
+constexpr long long kRunObs = 16384;
 
 gba_status validate_problem(const gba_problem_view *v, std::string *err) {
   if (!v) {
@@ -269,8 +271,8 @@ static void build_schur_structure(HostBatch *hbp) {
   parallel_runs(hb.no, kParMin, [&](long long b, long long e) {
     for (long long i = b; i < e; ++i) hb.obs_fpos[hb.cam_obs_list[i]] = (int32_t)i;
   });
-  std::vector<std::vector<int32_t>> rows(nc), cnts(nc);  // per row: columns; pair counts of its upper blocks
-  std::vector<int32_t> first_up(nc, 0);                  // per row: index of its first column >= the row
+  // per row: the columns on and above the diagonal and their pair counts
+  std::vector<std::vector<int32_t>> rows(nc), cnts(nc);
   // runs of rows of about equal observation counts
   std::vector<int> rb(1, 0);
   {
@@ -287,87 +289,83 @@ static void build_schur_structure(HostBatch *hbp) {
     }
   }
   const int nruns = (int)rb.size() - 1;
-  // 1. per row: sorted co-visible cameras, pair counts of the upper blocks
+  // A point's observations are sorted by camera: those of camera c and above
+  // start at the first of the point's observations by c.
+  auto from_row = [&](int a, int c) {
+    while (a > hb.pt_obs_begin[hb.obs_pt[a]] && hb.obs_cam[a - 1] == c) --a;
+    return a;
+  };
+  // 1. per row: the sorted cameras k >= c it shares points with, and the pair counts
   const long long stamp = new_stamps();
   host_parallel(nruns, [&](int r) {
     CamScratch &s = cam_scratch(nc);
     int32_t *pairs_of = s.a.data();  // per column camera: the row's pair count
+    std::vector<int32_t> cols;
     for (int c = rb[r]; c < rb[r + 1]; ++c) {
       const long long mk = stamp | c;
-      const int a0 = hb.cam_obs_begin[c], a1 = hb.cam_obs_begin[c + 1];
-      std::vector<int32_t> &row = rows[c];
-      for (int ia = a0; ia < a1; ++ia) {
-        const int a = hb.cam_obs_list[ia], j = hb.obs_pt[a];
-        for (int b = hb.pt_obs_begin[j]; b < hb.pt_obs_begin[j + 1]; ++b) {
-          const int k = hb.obs_cam[b];
+      cols.clear();
+      for (int ia = hb.cam_obs_begin[c]; ia < hb.cam_obs_begin[c + 1]; ++ia) {
+        const int a = hb.cam_obs_list[ia], e = hb.pt_obs_begin[hb.obs_pt[a] + 1];
+        for (int b = from_row(a, c); b < e; ++b) {
           if (b == a) continue;
-          if (s.mark[k] != mk) s.mark[k] = mk, row.push_back(k), pairs_of[k] = 0;
+          const int k = hb.obs_cam[b];
+          if (s.mark[k] != mk) s.mark[k] = mk, cols.push_back(k), pairs_of[k] = 0;
           ++pairs_of[k];
         }
       }
-      std::sort(row.begin(), row.end());
-      const int nb = (int)row.size();
-      const int u0 = (int)(std::lower_bound(row.begin(), row.end(), c) - row.begin());
-      first_up[c] = u0;
-      std::vector<int32_t> &cnt = cnts[c];
-      cnt.resize(nb - u0);
-      for (int u = u0; u < nb; ++u) cnt[u - u0] = pairs_of[row[u]];
+      std::sort(cols.begin(), cols.end());
+      rows[c] = cols;
+      cnts[c].resize(cols.size());
+      for (size_t u = 0; u < cols.size(); ++u) cnts[c][u] = pairs_of[cols[u]];
     }
   });
-  // 2. prefix sums: the CSR, the upper blocks, their pair ranges
+  // 2. the CSR: a row's blocks below the diagonal are the transposes of the
+  // rows above it, which come in the order of their rows; the pair ranges
+  std::vector<int32_t> low(nc, 0);  // per row: its blocks below the diagonal
+  for (int c = 0; c < nc; ++c)
+    for (const int k : rows[c]) low[k] += k > c;
   hb.sblk_row.assign(nc + 1, 0);
-  for (int c = 0; c < nc; ++c) hb.sblk_row[c + 1] = hb.sblk_row[c] + (int32_t)rows[c].size();
-  hb.nblk = hb.sblk_row[nc];
-  hb.sblk_col.resize(hb.nblk);
   std::vector<long long> up_begin(nc + 1, 0);  // per row: its first upper block (index into sblk_up)
-  for (int c = 0; c < nc; ++c) up_begin[c + 1] = up_begin[c] + (long long)cnts[c].size();
+  for (int c = 0; c < nc; ++c) {
+    hb.sblk_row[c + 1] = hb.sblk_row[c] + low[c] + (int32_t)rows[c].size();
+    up_begin[c + 1] = up_begin[c] + (long long)rows[c].size();
+  }
+  hb.nblk = hb.sblk_row[nc];
   hb.nup = up_begin[nc];
+  hb.sblk_col.resize(hb.nblk);
+  hb.sblk_tr.resize(hb.nblk);
   hb.sblk_up.resize(hb.nup);
   hb.sblk_pair.resize(hb.nup + 1);
   hb.sblk_pair[0] = 0;
-  for (int c = 0; c < nc; ++c) {
-    std::copy(rows[c].begin(), rows[c].end(), hb.sblk_col.begin() + hb.sblk_row[c]);
-    for (size_t u = 0; u < cnts[c].size(); ++u) {
-      const long long k = up_begin[c] + (long long)u;
-      hb.sblk_up[k] = hb.sblk_row[c] + first_up[c] + (int32_t)u;
-      hb.sblk_pair[k + 1] = hb.sblk_pair[k] + cnts[c][u];
+  std::vector<int32_t> next_low(hb.sblk_row.begin(), hb.sblk_row.end() - 1);
+  for (int c = 0; c < nc; ++c)
+    for (size_t u = 0; u < rows[c].size(); ++u) {
+      const int k = rows[c][u];
+      const int32_t e = hb.sblk_row[c] + low[c] + (int32_t)u;
+      const int32_t f = k > c ? next_low[k]++ : e;  // block (k, c)
+      hb.sblk_col[e] = k, hb.sblk_tr[e] = f;
+      hb.sblk_col[f] = c, hb.sblk_tr[f] = e;
+      hb.sblk_up[up_begin[c] + (long long)u] = e;
+      hb.sblk_pair[up_begin[c] + (long long)u + 1] = hb.sblk_pair[up_begin[c] + (long long)u] + cnts[c][u];
     }
-  }
   hb.npairs = hb.sblk_pair[hb.nup];
   hb.spair.resize(2 * (size_t)hb.npairs);
   // 3. the pairs, in point order per block
   host_parallel(nruns, [&](int r) {
     CamScratch &s = cam_scratch(nc);
-    std::vector<int32_t> &pos = s.a;
-    std::vector<int32_t> next;
+    int32_t *next = s.a.data();  // per column camera: the block's next pair
     for (int c = rb[r]; c < rb[r + 1]; ++c) {
-      const std::vector<int32_t> &row = rows[c];
-      const int u0 = first_up[c], nu = (int)row.size() - u0;
-      next.resize(nu);
-      for (int u = 0; u < nu; ++u) {
-        pos[row[u0 + u]] = u;
-        next[u] = hb.sblk_pair[up_begin[c] + u];
-      }
+      for (size_t u = 0; u < rows[c].size(); ++u) next[rows[c][u]] = hb.sblk_pair[up_begin[c] + (long long)u];
       for (int ia = hb.cam_obs_begin[c]; ia < hb.cam_obs_begin[c + 1]; ++ia) {
-        const int a = hb.cam_obs_list[ia], j = hb.obs_pt[a];
-        for (int b = hb.pt_obs_begin[j]; b < hb.pt_obs_begin[j + 1]; ++b)
-          if (b != a && hb.obs_cam[b] >= c) {
-            const size_t k = (size_t)next[pos[hb.obs_cam[b]]]++;
-            hb.spair[2 * k] = hb.obs_fpos[a];
-            hb.spair[2 * k + 1] = hb.obs_fpos[b];
-          }
+        const int a = hb.cam_obs_list[ia], e = hb.pt_obs_begin[hb.obs_pt[a] + 1];
+        for (int b = from_row(a, c); b < e; ++b) {
+          if (b == a) continue;
+          const size_t k = (size_t)next[hb.obs_cam[b]]++;
+          hb.spair[2 * k] = hb.obs_fpos[a];
+          hb.spair[2 * k + 1] = hb.obs_fpos[b];
+        }
       }
     }
-  });
-  // 4. the transpose of block (c, k) is block (k, c), in row k
-  hb.sblk_tr.resize(hb.nblk);
-  host_parallel(nruns, [&](int r) {
-    for (int c = rb[r]; c < rb[r + 1]; ++c)
-      for (int e = hb.sblk_row[c]; e < hb.sblk_row[c + 1]; ++e) {
-        const int k = hb.sblk_col[e];
-        const auto b0 = hb.sblk_col.begin() + hb.sblk_row[k], b1 = hb.sblk_col.begin() + hb.sblk_row[k + 1];
-        hb.sblk_tr[e] = (int32_t)(std::lower_bound(b0, b1, c) - hb.sblk_col.begin());
-      }
   });
 }
 
@@ -403,13 +401,46 @@ gba_status prepare_batch(const gba_problem_view *views, int n, const PrepOptions
     return GBA_ERR_INVALID_ARGUMENT;
   }
   const int cap = opt.chunk_cap;
+  // The problems of a batch are checked and laid out side by side on the
+  // host threads (each then on one thread: a loop inside a task does not
+  // split again), unless one of them is so much of the batch that splitting
+  // its own loops finishes earlier.  192 windows of 12,700 observations: 44
+  // ms of set-up one after the other, 9 side by side.
+  long long most = 0, all = 0;
+  for (int p = 0; p < n; ++p) {
+    const long long no = std::max(views[p].num_observations, 0);
+    most = std::max(most, no);
+    all += no;
+  }
+  const bool side_by_side = n > 1 && (most < 2 * kRunObs || most * host_threads() <= 2 * all);
+  auto each_problem = [&](const std::function<gba_status(int, std::string *)> &fn) -> gba_status {
+    if (!side_by_side) {
+      for (int p = 0; p < n; ++p)
+        if (const gba_status st = fn(p, err); st != GBA_OK) return st;
+      return GBA_OK;
+    }
+    // the first failing problem's error, as one after the other
+    std::atomic<long long> first{n};
+    std::vector<gba_status> sts(n, GBA_OK);
+    std::vector<std::string> errs(n);
+    host_parallel(n, [&](int p) {
+      if (p > first.load(std::memory_order_relaxed)) return;
+      sts[p] = fn(p, &errs[p]);
+      if (sts[p] != GBA_OK) atomic_min_i64(first, p);
+    });
+    const long long f = first.load();
+    if (f == n) return GBA_OK;
+    *err = errs[f];
+    return sts[f];
+  };
+  gba_status st = each_problem([&](int p, std::string *e) {
+    const gba_status r = validate_problem(&views[p], e);
+    if (r != GBA_OK && n > 1) *e = fmt("problem %lld: ", p) + *e;
+    return r;
+  });
+  if (st != GBA_OK) return st;
   long long tc = 0, tp = 0, to = 0;
   for (int p = 0; p < n; ++p) {
-    const gba_status st = validate_problem(&views[p], err);
-    if (st != GBA_OK) {
-      if (n > 1) *err = fmt("problem %lld: ", p) + *err;
-      return st;
-    }
     tc += views[p].num_cameras;
     tp += views[p].num_points;
     to += views[p].num_observations;
@@ -440,27 +471,41 @@ gba_status prepare_batch(const gba_problem_view *views, int n, const PrepOptions
   hb.cam_obs_begin.assign(tc + 1, 0);
   hb.cam_obs_list.resize(to);
 
-  int cam0 = 0, pt0 = 0, obs0 = 0;
-  std::vector<int32_t> deg, key, order, inv, fill, part_deg, part_key;
-  std::vector<uint8_t> part_used;
-  for (int p = 0; p < n; ++p) {
+  {
+    int cam0 = 0, pt0 = 0, obs0 = 0, blk0 = 0;
+    for (int p = 0; p < n; ++p) {
+      ProblemInfo &pi = hb.prob[p];
+      pi.cam_begin = cam0;
+      pi.cam_count = views[p].num_cameras;
+      pi.pt_begin = pt0;
+      pi.pt_count = views[p].num_points;
+      pi.obs_begin = obs0;
+      pi.obs_count = views[p].num_observations;
+      pi.cam_block_begin = blk0;
+      pi.cam_block_count = (pi.cam_count + kPcgBlockCams - 1) / kPcgBlockCams;
+      cam0 += pi.cam_count;
+      pt0 += pi.pt_count;
+      obs0 += pi.obs_count;
+      blk0 += pi.cam_block_count;
+    }
+    hb.camblk.resize(blk0);
+  }
+  std::vector<std::vector<ChunkInfo>> chunks(n);
+  st = each_problem([&](int p, std::string *perr) -> gba_status {
+    std::vector<int32_t> deg, key, order, inv, fill, part_deg, part_key;
+    std::vector<uint8_t> part_used;
     const gba_problem_view &v = views[p];
     const int nc = v.num_cameras, np = v.num_points, no = v.num_observations;
+    std::vector<int32_t> pt_begin(np + 1);  // where each point's observations begin
     ProblemInfo &pi = hb.prob[p];
-    pi.cam_begin = cam0;
-    pi.cam_count = nc;
-    pi.pt_begin = pt0;
-    pi.pt_count = np;
-    pi.obs_begin = obs0;
-    pi.obs_count = no;
-    pi.chunk_begin = (int)hb.chunk.size();
+    const int cam0 = pi.cam_begin, pt0 = pi.pt_begin, obs0 = pi.obs_begin;
     // degrees, first camera of each point.  A large problem takes runs of
     // its observations on host threads, each counting into its own
     // per-point arrays (merged over the runs); the same runs then place
     // their observations in the points' ranges after the earlier runs', so
     // each point keeps its input order as in one sequential pass.
     const long long runs =
-        std::min<long long>({(long long)host_threads(), (long long)no / 16384, (1LL << 22) / std::max(1, np)});
+        std::min<long long>({(long long)host_threads(), (long long)no / kRunObs, (1LL << 22) / std::max(1, np)});
     auto run_begin = [&](long long r) { return (int)((long long)no * r / runs); };
     deg.assign(np, 0);
     key.assign(np, nc);
@@ -519,19 +564,19 @@ gba_status prepare_batch(const gba_problem_view *views, int n, const PrepOptions
         hb.pt_orig[pt0 + ji] = j;
         hb.pt_problem[pt0 + ji] = p;
         hb.pt_used[pt0 + ji] = deg[j] > 0;
-        hb.pt_obs_begin[pt0 + ji + 1] = deg[j];
+        pt_begin[ji + 1] = deg[j];
         double *x = hb.pt_param.data() + 4 * (size_t)(pt0 + ji);
         for (int q = 0; q < 3; ++q) x[q] = v.parameters[9 * (size_t)nc + 3 * (size_t)j + q];
         x[3] = 0.0;
       }
     });
-    hb.pt_obs_begin[pt0] = obs0;
-    for (int ji = 0; ji < np; ++ji) hb.pt_obs_begin[pt0 + ji + 1] += hb.pt_obs_begin[pt0 + ji];
+    pt_begin[0] = obs0;
+    for (int ji = 0; ji < np; ++ji) pt_begin[ji + 1] += pt_begin[ji];
     if (runs > 1) {
       // per (run, point): where the run's observations of the point start
       parallel_runs(np, 8192, [&](long long j0, long long j1) {
         for (long long j = j0; j < j1; ++j) {
-          int32_t base = hb.pt_obs_begin[pt0 + inv[j]];
+          int32_t base = pt_begin[inv[j]];
           for (long long r = 0; r < runs; ++r) {
             const int32_t d = part_deg[(size_t)r * np + j];
             part_deg[(size_t)r * np + j] = base;
@@ -544,14 +589,14 @@ gba_status prepare_batch(const gba_problem_view *views, int n, const PrepOptions
         for (int i = run_begin(r); i < run_begin(r + 1); ++i) hb.obs_orig[at[v.point_index[i]]++] = i;
       });
     } else {
-      fill.assign(hb.pt_obs_begin.begin() + pt0, hb.pt_obs_begin.begin() + pt0 + np + 1);
+      fill.assign(pt_begin.begin(), pt_begin.end());
       for (int i = 0; i < no; ++i) hb.obs_orig[fill[inv[v.point_index[i]]]++] = i;
     }
     // within a point: by camera, then input index (insertion sort, stable);
     // points and observations are independent (host threads)
     parallel_runs(np, 20000, [&](long long j0, long long j1) {
       for (int ji = (int)j0; ji < (int)j1; ++ji) {
-        const int b = hb.pt_obs_begin[pt0 + ji], e = hb.pt_obs_begin[pt0 + ji + 1];
+        const int b = pt_begin[ji], e = pt_begin[ji + 1];
         for (int k = b + 1; k < e; ++k) {
           const int x = hb.obs_orig[k];
           const int cx = v.camera_index[x];
@@ -575,6 +620,7 @@ gba_status prepare_batch(const gba_problem_view *views, int n, const PrepOptions
     });
     for (int c = 0; c < nc; ++c) hb.cam_problem[cam0 + c] = p;
     if (nc > 0) std::memcpy(hb.cam_param.data() + 9 * (size_t)cam0, v.parameters, sizeof(double) * 9 * (size_t)nc);
+    std::copy(pt_begin.begin(), pt_begin.end() - 1, hb.pt_obs_begin.begin() + pt0);
     // chunks of whole points (their camera orders below, for the whole batch)
     int ji = 0;
     while (ji < np) {
@@ -582,13 +628,13 @@ gba_status prepare_batch(const gba_problem_view *views, int n, const PrepOptions
       std::memset(&ci, 0, sizeof ci);
       ci.problem = p;
       ci.pt_begin = pt0 + ji;
-      ci.obs_begin = hb.pt_obs_begin[pt0 + ji];
+      ci.obs_begin = pt_begin[ji];
       int nobs = 0, npts = 0;
       while (ji < np && npts < cap) {
-        const int d = hb.pt_obs_begin[pt0 + ji + 1] - hb.pt_obs_begin[pt0 + ji];
+        const int d = pt_begin[ji + 1] - pt_begin[ji];
         if (d > cap) {
-          *err = fmt("point %lld is observed %lld times; at most %lld observations per point are supported",
-                     order[ji], d, cap);
+          *perr = fmt("point %lld is observed %lld times; at most %lld observations per point are supported",
+                      order[ji], d, cap);
           return GBA_ERR_INVALID_ARGUMENT;
         }
         if (nobs + d > cap) break;
@@ -598,23 +644,25 @@ gba_status prepare_batch(const gba_problem_view *views, int n, const PrepOptions
       }
       ci.obs_count = nobs;
       ci.pt_count = npts;
-      hb.chunk.push_back(ci);
+      chunks[p].push_back(ci);
     }
-    pi.chunk_count = (int)hb.chunk.size() - pi.chunk_begin;
     // camera blocks of the PCG kernels
-    pi.cam_block_begin = (int)hb.camblk.size();
     for (int c = 0; c < nc; c += kPcgBlockCams) {
       int4 b;
       b.x = p;
       b.y = cam0 + c;
       b.z = std::min(kPcgBlockCams, nc - c);
       b.w = 0;
-      hb.camblk.push_back(b);
+      hb.camblk[pi.cam_block_begin + c / kPcgBlockCams] = b;
     }
-    pi.cam_block_count = (int)hb.camblk.size() - pi.cam_block_begin;
-    cam0 += nc;
-    pt0 += np;
-    obs0 += no;
+    return GBA_OK;
+  });
+  if (st != GBA_OK) return st;
+  hb.pt_obs_begin[tp] = hb.no;
+  for (int p = 0; p < n; ++p) {
+    hb.prob[p].chunk_begin = (int)hb.chunk.size();
+    hb.prob[p].chunk_count = (int)chunks[p].size();
+    hb.chunk.insert(hb.chunk.end(), chunks[p].begin(), chunks[p].end());
   }
   hb.nchunks = (int)hb.chunk.size();
   hb.cam_blocks = (int)hb.camblk.size();
@@ -686,14 +734,25 @@ gba_status prepare_batch(const gba_problem_view *views, int n, const PrepOptions
     pi.seg_count = seg_off[pi.chunk_begin + pi.chunk_count] - pi.seg_begin;
   }
   // per camera: its segments (chunk order) and its observations (internal order)
-  hb.cam_seg_begin.assign(hb.nc + 1, 0);
-  for (int s = 0; s < hb.nseg; ++s) ++hb.cam_seg_begin[hb.seg_cam[s] + 1];
-  for (int c = 0; c < hb.nc; ++c) hb.cam_seg_begin[c + 1] += hb.cam_seg_begin[c];
   // each segment's partial goes to its camera-major position, so a camera's
-  // partials are contiguous for the camera reduce
+  // partials are contiguous for the camera reduce (a problem's segments are
+  // its cameras': the problems are independent)
+  hb.cam_seg_begin.assign(hb.nc + 1, 0);
   hb.seg_slot.resize(hb.nseg);
-  fill.assign(hb.cam_seg_begin.begin(), hb.cam_seg_begin.end());
-  for (int s = 0; s < hb.nseg; ++s) hb.seg_slot[s] = fill[hb.seg_cam[s]]++;
+  auto seg_slots = [&](int p) {
+    const ProblemInfo &pi = hb.prob[p];
+    std::vector<int32_t> at(pi.cam_count + 1, 0);
+    for (int s = pi.seg_begin; s < pi.seg_begin + pi.seg_count; ++s) ++at[hb.seg_cam[s] - pi.cam_begin + 1];
+    at[0] = pi.seg_begin;
+    for (int c = 0; c < pi.cam_count; ++c) {
+      hb.cam_seg_begin[pi.cam_begin + c] = at[c];
+      at[c + 1] += at[c];
+    }
+    for (int s = pi.seg_begin; s < pi.seg_begin + pi.seg_count; ++s)
+      hb.seg_slot[s] = at[hb.seg_cam[s] - pi.cam_begin]++;
+  };
+  host_parallel(n, seg_slots);
+  hb.cam_seg_begin[hb.nc] = hb.nseg;
   // explicit Schur complement: chosen by the option, AUTO when a point's
   // ordered observation pairs (sum over points of m (m - 1)) are at most
   // kExplicitPairsPerObs per observation (forming S then costs less than the
@@ -734,6 +793,7 @@ gba_status prepare_batch(const gba_problem_view *views, int n, const PrepOptions
     if (runs <= 1 || runs * tc > (1LL << 24)) {
       for (int k = 0; k < hb.no; ++k) ++hb.cam_obs_begin[hb.obs_cam[k] + 1];
       for (int c = 0; c < hb.nc; ++c) hb.cam_obs_begin[c + 1] += hb.cam_obs_begin[c];
+      std::vector<int32_t> fill;
       fill.assign(hb.cam_obs_begin.begin(), hb.cam_obs_begin.end());
       for (int k = 0; k < hb.no; ++k) hb.cam_obs_list[fill[hb.obs_cam[k]]++] = k;
     } else {
