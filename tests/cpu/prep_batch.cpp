@@ -13,7 +13,7 @@ struct Problem {
   std::vector<int32_t> cam, pt;
   std::vector<double> obs, par;
   int nc = 0, np = 0;
-  gba_problem_view view() const {
+  gba_problem_view view() {
     gba_problem_view v;
     std::memset(&v, 0, sizeof v);
     v.num_cameras = nc, v.num_points = np, v.num_observations = (int)cam.size();
@@ -47,7 +47,7 @@ int main() {
     for (double &x : p.par) x = (double)(r() % 100);
   }
   std::vector<gba_problem_view> v;
-  for (const Problem &p : pb) v.push_back(p.view());
+  for (Problem &p : pb) v.push_back(p.view());
   PrepOptions o;
   o.schur = GBA_SCHUR_EXPLICIT;
   HostBatch all;
