@@ -199,6 +199,7 @@ size_t Engine::layout(const HostBatch &hb, char *base, DeviceBatch *db, size_t *
   b.nup = (int32_t)nup;
   b.npairs = ex ? hb.npairs : 0;
   b.sblk_row = cv.take<int32_t>(ex ? nc + 1 : 0);
+  b.prob_order = cv.take<int32_t>(ex ? P : 0);
   b.sblk_max = 0;
   if (ex)
     for (size_t c = 0; c < nc; ++c) b.sblk_max = std::max(b.sblk_max, hb.sblk_row[c + 1] - hb.sblk_row[c] + 1);
@@ -417,6 +418,7 @@ gba_status Engine::upload(const HostBatch &hb, std::string *err) {
   sc.put(hdb.camblk, hb.camblk);
   if (hb.explicit_schur) {
     sc.put(hdb.sblk_row, hb.sblk_row);
+    sc.put(hdb.prob_order, hb.prob_order);
     sc.put(hdb.sblk_col, hb.sblk_col);
     sc.put(hdb.sblk_tr, hb.sblk_tr);
     sc.put(hdb.sblk_up, hb.sblk_up);

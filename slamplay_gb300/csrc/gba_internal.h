@@ -215,6 +215,7 @@ struct DeviceBatch {
   long long npairs;
   int32_t sblk_max;          // the most blocks of a row of S (the diagonal one included)
   const int32_t *sblk_row;   // nc + 1
+  const int32_t *prob_order; // the problems, those with the most blocks first
   const int32_t *sblk_col;   // nblk
   const int32_t *sblk_tr;    // nblk
   const int32_t *sblk_up;    // nup: block index

@@ -170,7 +170,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_pcg_cluster(DeviceBatch B, in
   __shared__ int s_lo, s_hi;
 
   const int rank = cs > 1 ? (int)cg::this_cluster().block_rank() : 0;
-  const int prob = blockIdx.x / cs;
+  const int prob = B.prob_order[blockIdx.x / cs];  // the longest first: the short ones fill in behind
   const int t = threadIdx.x, T = blockDim.x;
   LMState *L = B.lm + prob;
   // uniform over the cluster: every CTA reads the same state before its

@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(kC64Threads) k_pcg_cluster64(DeviceBatch B, in
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const unsigned full = 0xffffffffu;
   const int rank = cs > 1 ? (int)cg::this_cluster().block_rank() : 0;
-  const int prob = blockIdx.x / cs;
+  const int prob = B.prob_order[blockIdx.x / cs];  // the longest first: the short ones fill in behind
   LMState *L = B.lm + prob;
   // uniform over the cluster: every CTA reads the state before its first
   // barrier, and rank 0 changes it only after the last one

@@ -376,7 +376,7 @@ void HostBatch::reset() {
   P = nc = np = no = nchunks = nseg = cam_blocks = 0;
   explicit_schur = false;
   nblk = nup = npairs = 0;
-  for (auto *v : {&pt_obs_begin, &seg_cam, &cam_seg_begin, &cam_obs_begin, &cam_piece_begin, &sblk_row, &sblk_up,
+  for (auto *v : {&prob_order, &pt_obs_begin, &seg_cam, &cam_seg_begin, &cam_obs_begin, &cam_piece_begin, &sblk_row, &sblk_up,
                   &sblk_pair})
     v->clear();
   seg_pos.clear();
@@ -823,7 +823,16 @@ gba_status prepare_batch(const gba_problem_view *views, int n, const PrepOptions
     const int n = hb.cam_obs_begin[c + 1] - hb.cam_obs_begin[c];
     hb.cam_piece_begin[c + 1] = hb.cam_piece_begin[c] + std::max(1, (n + kCamPieceObs - 1) / kCamPieceObs);
   }
-  if (hb.explicit_schur) build_schur_structure(&hb);
+  if (hb.explicit_schur) {
+    build_schur_structure(&hb);
+    hb.prob_order.resize(n);
+    for (int p = 0; p < n; ++p) hb.prob_order[p] = p;
+    auto blocks = [&](int p) {
+      const ProblemInfo &pi = hb.prob[p];
+      return hb.sblk_row[pi.cam_begin + pi.cam_count] - hb.sblk_row[pi.cam_begin] + pi.cam_count;
+    };
+    std::stable_sort(hb.prob_order.begin(), hb.prob_order.end(), [&](int a, int b) { return blocks(a) > blocks(b); });
+  }
   return GBA_OK;
 }
 

@@ -40,6 +40,7 @@ struct HostBatch {
   bool explicit_schur = false;
   long long nblk = 0, nup = 0, npairs = 0;
   std::vector<int32_t> sblk_row, sblk_col, sblk_tr, sblk_up, sblk_pair;
+  std::vector<int32_t> prob_order;  // the problems, those with the most blocks first
   std::vector<int32_t> spair;     // 2 per pair: camera-major positions (obs_fpos)
   std::vector<int32_t> obs_fpos;  // observation -> its position in cam_obs_list
   // output mapping
