@@ -24,8 +24,8 @@
 //      the other warps fetch z of the columns the CTA's rows touch; then
 //      p = z + beta p.
 // Measured (us per PCG iteration, local windows and rings, grid form -> this
-// one): 7 cameras 7.6 -> 3.3, 16 cameras 7.7 -> 4.1, 23 cameras 7.9 -> 4.2,
-// 40 cameras 7.6 -> 5.8.  Batches (the PCG of one LM iteration, two-kernel
+// one): 8 cameras 5.1 -> 3.4, 16 cameras 5.6 -> 4.0, 23 cameras 5.6 -> 4.1,
+// 39 cameras 6.2 -> 5.5.  Batches (the PCG of one LM iteration, two-kernel
 // form -> this one): 16 windows of 5-40 cameras 8.3 -> 2.1 ms, 48 windows
 // 8.8 -> 2.6 ms, 200 windows 18.6 -> 8.5 ms.
 // The sums are the two-kernel form's and the grid form's, addition for
@@ -57,7 +57,7 @@ constexpr int kC64Slot = 96;  // threads per camera block in the update (3 warps
 constexpr int kC64Own = kC64Threads / kC64Slot;  // camera blocks a CTA updates, at most
 constexpr int kC64Coords = 9 * kPcgBlockCams;
 constexpr int kC64MaxBlocks = kC64MaxCams / kPcgBlockCams;
-constexpr double kC64GridClocks = 10500.0;  // estimated iteration from which one problem takes the grid form
+constexpr double kC64GridClocks = 11300.0;  // estimated iteration from which one problem takes the grid form
 constexpr int kC64Levels = 8;  // levels of the pairwise tree (rows of up to kC64MaxCams + 1 blocks)
 static_assert(kC64Coords <= kC64Slot && kC64Slot % 32 == 0, "a camera block's coordinates fit three whole warps");
 static_assert(kC64MaxBlocks <= 16, "half a warp holds one quantity of every block");
@@ -84,8 +84,8 @@ __host__ __device__ inline C64Layout c64_layout(int R, int n, int own_blocks, in
   l.qv = o, o = c64_align(o + 8 * oc);          // q of the owned coordinates (stored by the row's owner)
   l.zo = o, o = c64_align(o + 8 * oc);          // z of the owned coordinates (read by the others)
   l.uoff = o, o = c64_align(o + 4 * (9 / rows * n + 1));
-  l.pass = o, o = c64_align(o + (R > 0 ? 0 : 4 * (9 * (size_t)n + 1)));  // R = 0: each pass's first row
-  l.pcol = o, o = c64_align(o + 2 * (size_t)pairs);  // column camera of each pair
+  l.pass = o, o = c64_align(o + (R > 0 ? 0 : 4 * (9 * (size_t)n + 1)));  // R = 0: each pass's first row, its tree levels << 16
+  l.pcol = o, o = c64_align(o + (R > 0 ? 2 : 4) * (size_t)pairs);  // column camera of each pair (R = 0: c64_meta)
   l.ldst = o, o = c64_align(o + (R > 0 ? 2 * (size_t)pairs : 0));  // the tree's additions, level by level
   l.total = o;
   return l;
@@ -97,6 +97,18 @@ __host__ __device__ inline int units_below(int t, int before, int m, int U) {
   if (t <= before) return 0;
   const int r = (t - before + m - 1) / m;
   return r > U ? U : r;
+}
+
+// R = 0, what a pass needs of a pair: the column camera (8 bits), the tree
+// levels in which its block takes another's sum (5: block v takes block v + s
+// while v is a multiple of 2 s), whether it is its row's first block (1), the
+// row (among the CTA's).
+static_assert(kC64MaxCams <= 256, "a column camera in 8 bits");
+__device__ __forceinline__ uint32_t c64_meta(int col, int v, int m, int row) {
+  uint32_t mask = 0;
+  for (int l = 0; l < 5; ++l)
+    if ((v & ((2 << l) - 1)) == 0 && v + (1 << l) < m) mask |= 1u << l;
+  return (uint32_t)col | mask << 8 | (v == 0 ? 1u << 13 : 0u) | (uint32_t)row << 16;
 }
 
 // Shared memory of another CTA of the cluster.
@@ -149,7 +161,8 @@ __global__ void __launch_bounds__(kC64Threads) k_pcg_cluster64(DeviceBatch B, in
   double *zo = reinterpret_cast<double *>(c64_smem + lay.zo);
   int *uoff = reinterpret_cast<int *>(c64_smem + lay.uoff);
   int *pass_j = reinterpret_cast<int *>(c64_smem + lay.pass);
-  unsigned short *pcol = reinterpret_cast<unsigned short *>(c64_smem + lay.pcol);
+  unsigned short *pcol = reinterpret_cast<unsigned short *>(c64_smem + lay.pcol);  // R > 0
+  uint32_t *meta = reinterpret_cast<uint32_t *>(c64_smem + lay.pcol);              // R = 0
   unsigned short *ldst = reinterpret_cast<unsigned short *>(c64_smem + lay.ldst);
 
   // ---- ownership -------------------------------------------------------------
@@ -197,9 +210,10 @@ __global__ void __launch_bounds__(kC64Threads) k_pcg_cluster64(DeviceBatch B, in
     if (t == 0) {
       int c = 0, j = 0;
       while (j < nu) {
-        const int e0 = uoff[j];
-        pass_j[c++] = j++;
-        while (j < nu && uoff[j + 1] - e0 <= 32) ++j;
+        const int e0 = uoff[j], j0 = j++;
+        int m = uoff[j] - e0;  // the longest row
+        while (j < nu && uoff[j + 1] - e0 <= 32) m = max(m, uoff[j + 1] - uoff[j]), ++j;
+        pass_j[c++] = j0 | (m > 1 ? 32 - __clz(m - 1) : 0) << 16;
       }
       pass_j[c] = nu;
       s_npass = c;
@@ -232,7 +246,10 @@ __global__ void __launch_bounds__(kC64Threads) k_pcg_cluster64(DeviceBatch B, in
     int lo = c, hi = c;
     for (int v = lane; v < m; v += 32) {
       const int col = v < m - 1 ? B.sblk_col[rr0 + v] - c0 : c;
-      pcol[e0 + v] = (unsigned short)col;
+      if (R > 0)
+        pcol[e0 + v] = (unsigned short)col;
+      else
+        meta[e0 + v] = c64_meta(col, v, m, j);
       lo = min(lo, col), hi = max(hi, col);
     }
     lo = __reduce_min_sync(full, lo), hi = __reduce_max_sync(full, hi);
@@ -286,47 +303,43 @@ __global__ void __launch_bounds__(kC64Threads) k_pcg_cluster64(DeviceBatch B, in
     *(cs > 1 ? peer(q, blk_own[b]) : q) = qv;
   };
 
-  // R = 0: a pass over rows j .. j1 - 1 (pairs from e0): the lane's row and
-  // block, and the tree levels in which it takes another block's sum (block v
-  // takes block v + s while v is a multiple of 2 s)
-  auto lane_of_pass = [&](int j, int j1, int e0, int &row, int &mask) -> bool {
-    const int e = e0 + lane;
-    row = j;
-    while (row + 1 < j1 && e >= uoff[row + 1]) ++row;
-    const int v = e - uoff[row], m = uoff[row + 1] - uoff[row];
-    mask = 0;
-    for (int l = 0; l < 5; ++l)
-      if (v < m && (v & ((2 << l) - 1)) == 0 && v + (1 << l) < m) mask |= 1 << l;
-    return v < m;
+  // R = 0: a pass over rows j .. j1 - 1 (pairs from e0).  A row's sum ends in
+  // the lane of its first block (lead); the lanes then take (row, CTA) pairs:
+  // pair x = lane stores the sum of lane src into CTA x % cs
+  double *const pq_dest = cs > 1 ? peer(pqb + ua, lane & (cs - 1)) : pqb + ua;
+  struct Pass {
+    int j, e0, rows, levels, mask, lead, src;
+    const double *s, *p, *own;
+    double *dst;
+    bool in;
   };
-  auto pass_levels = [&](int j, int j1) {
-    int l = 0;
-    for (int r = j; r < j1; ++r)
-      while ((1 << l) < uoff[r + 1] - uoff[r]) ++l;
-    return l;
+  auto pass_at = [&](int ps) {
+    Pass a;
+    const int pj = pass_j[ps], j1 = pass_j[ps + 1] & 0xffff;
+    a.j = pj & 0xffff, a.levels = pj >> 16, a.rows = j1 - a.j;
+    a.e0 = uoff[a.j];
+    a.in = lane < uoff[j1] - a.e0;
+    const int e = a.in ? a.e0 + lane : a.e0, row = (int)(meta[e] >> 16);
+    a.mask = a.in ? (int)(meta[e] >> 8) & 31 : 0;
+    a.lead = a.in && (meta[e] >> 13 & 1) ? ua + row : -1;
+    a.s = sval + 9 * e, a.p = p + 9 * (int)(meta[e] & 255), a.own = p + ua + row;
+    const int rr = min(a.j + (lane >> csh), j1 - 1);
+    a.src = uoff[rr] - a.e0;
+    a.dst = lane < a.rows << csh ? pq_dest + rr : nullptr;
+    return a;
   };
-  // a row's sum ends in the lane of its first block (lead >= 0: its row);
-  // the lanes then take (row, CTA) pairs: pair x = lane stores the sum of
-  // lane src to dst
-  auto push_of_pass = [&](int j, int j1, int e0, int row, int &src, double *&dst, int &lead) {
-    lead = e0 + lane == uoff[row] ? ua + row : -1;
-    const int rr = min(j + (lane >> csh), j1 - 1);
-    src = uoff[rr] - e0;
-    dst = lane < (j1 - j) << csh ? (cs > 1 ? peer(pqb + ua + rr, lane & (cs - 1)) : pqb + ua + rr) : nullptr;
-  };
-  auto finish_pass = [&](double d, int levels, int mask, int lead, double own_p, int rows, int src, double *dst, int j,
-                         int e0) {
-    for (int l = 0; l < levels; ++l) {
+  auto finish_pass = [&](double d, const Pass &a) {
+    for (int l = 0; l < a.levels; ++l) {
       const double x = __shfl_down_sync(full, d, 1 << l);
-      d += (mask >> l) & 1 ? x : 0.0;
+      d += (a.mask >> l) & 1 ? x : 0.0;
     }
-    const double pqv = own_p * d, y = __shfl_sync(full, pqv, src);
-    if (dst) *dst = y;
-    if (lead >= 0) push_q(lead, d);
-    for (int x0 = 32; x0 < rows << csh; x0 += 32) {  // more pairs than lanes
-      const int x = x0 + lane, rr = min(j + (x >> csh), j + rows - 1);
-      const double y2 = __shfl_sync(full, pqv, uoff[rr] - e0);
-      if (x < rows << csh) *(cs > 1 ? peer(pqb + ua + rr, x & (cs - 1)) : pqb + ua + rr) = y2;
+    const double pqv = *a.own * d, y = __shfl_sync(full, pqv, a.src);
+    if (a.dst) *a.dst = y;
+    if (a.lead >= 0) push_q(a.lead, d);
+    for (int x0 = 32; x0 < a.rows << csh; x0 += 32) {  // more pairs than lanes (32 is a multiple of cs)
+      const int x = x0 + lane, rr = min(a.j + (x >> csh), a.j + a.rows - 1);
+      const double y2 = __shfl_sync(full, pqv, uoff[rr] - a.e0);
+      if (x < a.rows << csh) pq_dest[rr] = y2;
     }
   };
   // a row of more than 32 blocks (kC64MaxCams + 1 at most): runs of 32, each
@@ -338,7 +351,7 @@ __global__ void __launch_bounds__(kC64Threads) k_pcg_cluster64(DeviceBatch B, in
     for (int g = 0; g < 5; ++g) {
       if (g < nrun) {
         const int v = 32 * g + lane, e = e0 + min(v, m0 - 1);
-        const double *sr = sval + 9 * e, *pp = p + 9 * (int)pcol[e];
+        const double *sr = sval + 9 * e, *pp = p + 9 * (int)(meta[e] & 255);
         double x = 0.0;
 #pragma unroll
         for (int cc = 0; cc < 9; ++cc) x = fma(sr[cc], pp[cc], x);
@@ -351,24 +364,17 @@ __global__ void __launch_bounds__(kC64Threads) k_pcg_cluster64(DeviceBatch B, in
     if (nrun > 4) run[0] += run[4];
     const double qv = __shfl_sync(full, run[0], 0), pqv = p[ua + j] * qv;
     if (lane == 0) push_q(ua + j, qv);
-    if (lane < cs) *(cs > 1 ? peer(pqb + ua + j, lane) : pqb + ua + j) = pqv;
+    if (lane < cs) pq_dest[j] = pqv;
   };
-  int npass = 0, a_levels = 0, a_mask = 0, a_lead = -1, a_rows = 0, a_src = 0, a_j = 0, a_e0 = 0;
-  double a_s[9], *a_dst = nullptr;
-  const double *a_p = p, *a_own = p;
+  int npass = 0;
+  double a_s[9];  // the warp's first pass: its rows of S and its addresses in registers
+  Pass first = {};
   if constexpr (R == 0) {
     npass = s_npass;
     if (warp < npass) {
-      const int j1 = pass_j[warp + 1];
-      a_j = pass_j[warp], a_e0 = uoff[a_j], a_rows = j1 - a_j;
-      int row;
-      const bool in = lane_of_pass(a_j, j1, a_e0, row, a_mask);
+      first = pass_at(warp);
 #pragma unroll
-      for (int cc = 0; cc < 9; ++cc) a_s[cc] = in ? sval[9 * (a_e0 + lane) + cc] : 0.0;
-      a_p = p + 9 * (int)pcol[in ? a_e0 + lane : a_e0];
-      a_own = p + ua + row;
-      a_levels = pass_levels(a_j, j1);
-      push_of_pass(a_j, j1, a_e0, row, a_src, a_dst, a_lead);
+      for (int cc = 0; cc < 9; ++cc) a_s[cc] = first.in ? first.s[cc] : 0.0;
     }
   }
   const int blk_top = nblk > 8 ? 8 : nblk > 4 ? 4 : nblk > 2 ? 2 : nblk > 1 ? 1 : 0;  // the first butterfly level over the blocks
@@ -386,28 +392,21 @@ __global__ void __launch_bounds__(kC64Threads) k_pcg_cluster64(DeviceBatch B, in
     // ---- A. q = S p_k for the owned rows -----------------------------------
     if constexpr (R == 0) {
       if (warp < npass) {
-        // the warp's first pass, its rows of S and addresses in registers
         double d = 0.0;
 #pragma unroll
-        for (int cc = 0; cc < 9; ++cc) d = fma(a_s[cc], a_p[cc], d);
-        finish_pass(d, a_levels, a_mask, a_lead, *a_own, a_rows, a_src, a_dst, a_j, a_e0);
+        for (int cc = 0; cc < 9; ++cc) d = fma(a_s[cc], first.p[cc], d);
+        finish_pass(d, first);
       }
       for (int ps = warp + kC64Warps; ps < npass; ps += kC64Warps) {
-        const int j = pass_j[ps], j1 = pass_j[ps + 1], e0 = uoff[j], m0 = uoff[j + 1] - e0;
+        const int j = pass_j[ps] & 0xffff, m0 = uoff[j + 1] - uoff[j];
         if (m0 <= 32) {
-          int row, mask;
-          const bool in = lane_of_pass(j, j1, e0, row, mask);
-          const double *sr = sval + 9 * (in ? e0 + lane : e0), *pp = p + 9 * (int)pcol[in ? e0 + lane : e0];
+          const Pass a = pass_at(ps);
           double d = 0.0;
 #pragma unroll
-          for (int cc = 0; cc < 9; ++cc) d = fma(sr[cc], pp[cc], d);
-          int src, lead;
-          double *dst;
-          const int lv = pass_levels(j, j1);
-          push_of_pass(j, j1, e0, row, src, dst, lead);
-          finish_pass(d, lv, mask, lead, p[ua + row], j1 - j, src, dst, j, e0);
+          for (int cc = 0; cc < 9; ++cc) d = fma(a.s[cc], a.p[cc], d);
+          finish_pass(d, a);
         } else {
-          long_row(j, e0, m0);
+          long_row(j, uoff[j], m0);
         }
       }
     } else {
@@ -713,8 +712,10 @@ bool pcg_cluster64_plan(const ProblemInfo *prob, int num_problems, const int32_t
       }
     }
   // a single problem whose product keeps the cluster's 16 SMs busy for longer
-  // goes to the grid form: 159 k FMAs per iteration (75 cameras of a walk)
-  // take 8.6 us here and 8.1 us there, 44 k (40 cameras) 5.8 and 7.6 us
+  // goes to the grid form.  An iteration here and there, at the estimate in
+  // thousands of clocks: 9.7 (39 cameras of a window) 5.5 and 6.2 us, 11.0 (24
+  // cameras of a ring) 5.5 and 5.9, 11.6 (60 of a window) 6.7 and 6.5, 12.0
+  // (32 of a ring) 6.6 and 6.2, 15.9 (75 of a walk) 8.9 and 6.9
   if (plan->cs == 0 || (num_problems == 1 && plan->clocks > kC64GridClocks)) {
     *plan = Cluster64Plan();
     return false;
