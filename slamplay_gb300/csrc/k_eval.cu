@@ -141,6 +141,7 @@ __device__ __forceinline__ double eval_rig(const DeviceBatch &B, int64_t o, int 
     const Corrector cr = make_corrector(loss, B.opt.loss_scale, ru, rv);
 #pragma unroll
     for (int k = 0; k < 12; ++k) {
+      if (k >= 6 && k < 9) continue;
       const double rJ = ru * ju[k] + rv * jv[k];
       ju[k] = cr.sqrt_rho1 * (ju[k] - cr.alpha_sq_norm * ru * rJ);
       jv[k] = cr.sqrt_rho1 * (jv[k] - cr.alpha_sq_norm * rv * rJ);
@@ -152,12 +153,12 @@ __device__ __forceinline__ double eval_rig(const DeviceBatch &B, int64_t o, int 
   if (!unit_scale) {
     const double *sc = B.cam_scale + 9 * (size_t)c, *sp = B.pt_scale + 3 * (size_t)j;
 #pragma unroll
-    for (int k = 0; k < 9; ++k) ju[k] *= sc[k], jv[k] *= sc[k];
+    for (int k = 0; k < 6; ++k) ju[k] *= sc[k], jv[k] *= sc[k];
 #pragma unroll
     for (int k = 0; k < 3; ++k) ju[9 + k] *= sp[k], jv[9 + k] *= sp[k];
   }
 #pragma unroll
-  for (int k = 0; k < 12; ++k) ok = ok && isfinite((float)ju[k]) && isfinite((float)jv[k]);
+  for (int k = 0; k < 12; ++k) ok = ok && finite_as_float(ju[k]) && finite_as_float(jv[k]);
   return cost;
 }
 
@@ -308,14 +309,15 @@ __device__ __forceinline__ double eval_observation_df(const DeviceBatch &B, int6
     const double cost = eval_rig(B, o, c, j, X, false, jd, kd, rud, rvd, ok);
 #pragma unroll
     for (int k = 0; k < 12; ++k) {
-      gr[k] = df_from_double(jd[k] * rud + kd[k] * rvd);
-      const float2 jk = make_float2((float)jd[k], (float)kd[k]);
+      const bool zero = k >= 6 && k < 9;  // the poses have six parameters
+      gr[k] = zero ? df_zero() : df_from_double(jd[k] * rud + kd[k] * rvd);
+      const float2 jk = zero ? make_float2(0.f, 0.f) : make_float2(to_float(jd[k]), to_float(kd[k]));
       if (k < 9)
         Jc[k] = jk;
       else
         Jp[k - 9] = jk;
     }
-    r = make_float2((float)rud, (float)rvd);
+    r = make_float2(to_float(rud), to_float(rvd));
     bad = !ok;
     return cost;
   }

@@ -135,7 +135,31 @@ __device__ __forceinline__ DF df_prod(float a, float b) {
   const float p = __fmul_rn(a, b);
   return DF{p, __fmaf_rn(a, b, -p)};
 }
-__device__ __forceinline__ double df_value(DF a) { return (double)a.hi + (double)a.lo; }
+// Conversions by integer instructions (a conversion to or from FP64 holds the
+// FP64 pipe for 64 clocks a warp): the same values, outside the normal FP32
+// range by the hardware's conversion.
+__device__ __forceinline__ float to_float(double d) {
+  const uint32_t hi = (uint32_t)__double2hiint(d), lo = (uint32_t)__double2loint(d), ah = hi & 0x7fffffffu;
+  if (ah - 0x38100000u < 0x47ef0000u - 0x38100000u) {
+    uint32_t f = ((ah - 0x38000000u) << 3) | (lo >> 29);
+    f += (lo & 0x1fffffffu) + (f & 1u) > 0x10000000u ? 1u : 0u;  // to nearest, ties to even
+    return __uint_as_float(f | (hi & 0x80000000u));
+  }
+  if ((ah | lo) == 0u) return __uint_as_float(hi);
+  return __double2float_rn(d);
+}
+__device__ __forceinline__ double to_double(float f) {
+  const uint32_t u = __float_as_uint(f), a = u & 0x7fffffffu;
+  if (a - 0x00800000u < 0x7f800000u - 0x00800000u)
+    return __hiloint2double((int)(((a >> 3) + 0x38000000u) | (u & 0x80000000u)), (int)(u << 29));
+  if (a == 0u) return __hiloint2double((int)u, 0);
+  return (double)f;
+}
+// Whether a double is finite as a float.
+__device__ __forceinline__ bool finite_as_float(double d) {
+  return (__double_as_longlong(d) & 0x7fffffffffffffffLL) < 0x47effffff0000000LL;
+}
+__device__ __forceinline__ double df_value(DF a) { return to_double(a.hi) + to_double(a.lo); }
 // a * b for a float b, and a * b: the error-free product of the high parts
 // plus the cross terms, renormalised (about 2^-46 relative error)
 __device__ __forceinline__ DF df_mul_f(DF a, float b) {
@@ -149,8 +173,8 @@ __device__ __forceinline__ DF df_mul(DF a, DF b) {
 __device__ __forceinline__ DF df_neg(DF a) { return DF{-a.hi, -a.lo}; }
 // a double as the nearest float plus the nearest float to the remainder
 __device__ __forceinline__ DF df_from_double(double d) {
-  const float h = __double2float_rn(d);
-  return DF{h, __double2float_rn(d - (double)h)};
+  const float h = to_float(d);
+  return DF{h, to_float(d - to_double(h))};
 }
 // Sum over a warp (xor butterfly, result in every lane).
 __device__ __forceinline__ DF df_warp_sum(DF v) {
