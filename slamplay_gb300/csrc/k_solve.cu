@@ -254,10 +254,12 @@ struct PointSchurEx64Smem {
   double cd[kChunkCap][3];  // the damped diagonal of C by chunk point
 };
 
+// SPLIT: gridDim.y CTAs a chunk.
+template <bool SPLIT>
 __global__ void __launch_bounds__(kChunkCap) k_point_schur_ex64(DeviceBatch B) {
   extern __shared__ __align__(16) unsigned char k3x_smem[];
   PointSchurEx64Smem &sm = *reinterpret_cast<PointSchurEx64Smem *>(k3x_smem);
-  const int t = threadIdx.x;
+  const int t = threadIdx.x, part_y = SPLIT ? blockIdx.y : 0, parts = SPLIT ? gridDim.y : 1;
   for (int ch = blockIdx.x; ch < B.nchunks; ch += gridDim.x) {
     const ChunkInfo ci = B.chunk[ch];
     LMState *L = B.lm + ci.problem;
@@ -414,24 +416,20 @@ __device__ bool spd_inverse9_gj(double (*buf)[81]) {
   bool ok = true;
   for (int k = 0; k < 9; ++k) {
     const double p = buf[cur][10 * k];
-    if (!(p > 0.0)) ok = false;  // uniform: every thread reads the same pivot
+    if (!positive64(p)) ok = false;  // uniform: every thread reads the same pivot
     if (ok && t < 81) {
-      const double pinv = recip_nr(p);
-      double v;
-      if (i == k && j == k)
-        v = pinv;
-      else if (i == k)
-        v = buf[cur][t] * pinv;
-      else if (j == k)
-        v = -buf[cur][t] * pinv;
-      else
-        v = fma(-(buf[cur][9 * i + k] * pinv), buf[cur][9 * k + j], buf[cur][t]);
-      buf[cur ^ 1][t] = v;
+      // one product and one FMA for every entry, of which each kind of entry
+      // takes its own (the kinds share warps, and as branches each would
+      // hold the FP64 pipe in turn)
+      const double pinv = recip_nr(p), akj = buf[cur][9 * k + j];
+      const double m = (i == k ? akj : buf[cur][9 * i + k]) * pinv;
+      const double f = fma(-m, akj, buf[cur][t]);
+      buf[cur ^ 1][t] = i == k ? (j == k ? pinv : m) : (j == k ? -m : f);
     }
     __syncthreads();
     cur ^= 1;
   }
-  const bool fin = t >= 81 || isfinite(buf[cur][t]);
+  const bool fin = t >= 81 || finite64(buf[cur][t]);
   return __syncthreads_and(fin ? 1 : 0) && ok;
 }
 
@@ -446,9 +444,9 @@ __global__ void __launch_bounds__(kSchurThreads) k_camera_schur(DeviceBatch B) {
   typedef typename Prec<MIXED>::real real;
   typedef typename Acc<MIXED>::type Acc;
   __shared__ double buf[2][81];
-  __shared__ double sums[54];
+  __shared__ double sums[54], damp[9];
   __shared__ double vec[9];
-  __shared__ double red[kSchurThreads / 32];
+  __shared__ double red[2 * (kSchurThreads / 32) + 1];
   __shared__ int flag;
   const int c = blockIdx.x;
   const int p = B.cam_problem[c];
@@ -477,17 +475,18 @@ __global__ void __launch_bounds__(kSchurThreads) k_camera_schur(DeviceBatch B) {
       double sum = a[0].value();
       if (kAcc == 4) sum = (a[0].value() + a[1 % kAcc].value()) + (a[2 % kAcc].value() + a[3 % kAcc].value());
       sums[t] = sum;
+    } else if (t >= kSchurThreads - 9) {
+      // the damping's divisions and square roots, in a warp that sums nothing
+      const int a = t - (kSchurThreads - 9);
+      const double d2 = lm_d2(B.cam_B[45 * (size_t)c + sym9(a, a)], L->radius, B.opt);
+      B.cam_D2[9 * (size_t)c + a] = d2;
+      damp[a] = d2;
     }
     __syncthreads();
-    const double radius = L->radius;
     if (t < 81) {
       const int a = t / 9, b = t % 9;
       double v = B.cam_B[45 * (size_t)c + sym9(a, b)] - sums[sym9(a, b)];
-      if (a == b) {
-        const double d2 = lm_d2(B.cam_B[45 * (size_t)c + sym9(a, a)], radius, B.opt);
-        v += d2;
-        B.cam_D2[9 * (size_t)c + a] = d2;
-      }
+      if (a == b) v += damp[a];
       buf[0][t] = v;
       if (B.explicit_schur) reinterpret_cast<real *>(B.cam_Sii)[81 * (size_t)c + t] = (real)v;
     }
@@ -517,12 +516,11 @@ __global__ void __launch_bounds__(kSchurThreads) k_camera_schur(DeviceBatch B) {
       if (MIXED) B.cam_Minvf[81 * (size_t)c + t] = (float)buf[1][t];
     }
     if (MIXED && t < 45) B.cam_Bf[45 * (size_t)c + t] = (float)B.cam_B[45 * (size_t)c + t];
-    const double rzs = block_sum(rz, red);
-    const double rrs = block_sum(rr, red);
-    if (t == 0) {
-      B.cam_scal[(size_t)kCamScal * c + kCC_RZ] = rzs;
-      B.cam_scal[(size_t)kCamScal * c + kCC_RR] = rrs;
-    }
+    double gmax;
+    bool any;
+    const double sum = block_sums2_max(rz, rr, 0.0, false, red, &gmax, &any);
+    if (t == 0) B.cam_scal[(size_t)kCamScal * c + kCC_RZ] = sum;
+    if (t == 32) B.cam_scal[(size_t)kCamScal * c + kCC_RR] = sum;
     // the problem's last camera CTA starts its PCG
     const ProblemInfo pi = B.prob[p];
     if (last_block_done(B.prob_counter + 4 * p + kPC_SCHUR, (uint32_t)pi.cam_count, &flag)) {
