@@ -298,19 +298,23 @@ __global__ void __launch_bounds__(kChunkCap) k_point_schur_ex64(DeviceBatch B) {
         for (int q = 0; q < 6; ++q) Ci[q] = 0.0;
       }
       double *cio = reinterpret_cast<double *>(B.pt_Cinv) + 6 * (size_t)j;
+      if (part_y == 0) {
 #pragma unroll
-      for (int q = 0; q < 6; ++q) {
-        cio[q] = Ci[q];
-        B.pt_Cinv64[6 * (size_t)j + q] = Ci[q];
+        for (int q = 0; q < 6; ++q) {
+          cio[q] = Ci[q];
+          B.pt_Cinv64[6 * (size_t)j + q] = Ci[q];
+        }
       }
       const double *g = B.pt_g + 3 * (size_t)j;
       const double g0 = g[0], g1 = g[1], g2 = g[2];
       const double t0 = Ci[0] * g0 + Ci[1] * g1 + Ci[2] * g2;
       const double t1 = Ci[1] * g0 + Ci[3] * g1 + Ci[4] * g2;
       const double t2 = Ci[2] * g0 + Ci[4] * g1 + Ci[5] * g2;
-      B.pt_t[3 * (size_t)j + 0] = t0;
-      B.pt_t[3 * (size_t)j + 1] = t1;
-      B.pt_t[3 * (size_t)j + 2] = t2;
+      if (part_y == 0) {
+        B.pt_t[3 * (size_t)j + 0] = t0;
+        B.pt_t[3 * (size_t)j + 1] = t1;
+        B.pt_t[3 * (size_t)j + 2] = t2;
+      }
       double Lc[6], inv[2];
       chol3(Ci, Lc, inv);
 #pragma unroll
@@ -323,9 +327,10 @@ __global__ void __launch_bounds__(kChunkCap) k_point_schur_ex64(DeviceBatch B) {
       sm.u[t][0] = u0, sm.u[t][1] = u1, sm.u[t][2] = u2;
     }
     // the first (segment, entry) task of this thread: its metadata now
+    const int i0 = t + kChunkCap * part_y;
     int f_b0 = 0, f_b1 = 0, f_slot = 0;
-    if (t < ci.seg_count * 54) {
-      const int sg = t / 54;
+    if (i0 < ci.seg_count * 54) {
+      const int sg = i0 / 54;
       f_b0 = B.seg_pos[ci.seg_begin + sg];
       f_b1 = (sg + 1 < ci.seg_count) ? B.seg_pos[ci.seg_begin + sg + 1] : ci.obs_count;
       f_slot = B.seg_slot[ci.seg_begin + sg];
@@ -351,17 +356,19 @@ __global__ void __launch_bounds__(kChunkCap) k_point_schur_ex64(DeviceBatch B) {
       for (int e = 0; e < 27; ++e) sm.F[slot][e] = F[e];
 #pragma unroll
       for (int e = 0; e < 3; ++e) sm.us[slot][e] = sm.u[lp][e];
-      double2 *dst = reinterpret_cast<double2 *>(reinterpret_cast<double *>(B.obs_F) +
-                                                 (size_t)kObsF * B.obs_fpos[ci.obs_begin + t]);
+      if (part_y == 0) {
+        double2 *dst = reinterpret_cast<double2 *>(reinterpret_cast<double *>(B.obs_F) +
+                                                   (size_t)kObsF * B.obs_fpos[ci.obs_begin + t]);
 #pragma unroll
-      for (int e = 0; e < kObsF / 2; ++e) dst[e] = *reinterpret_cast<const double2 *>(&F[2 * e]);
+        for (int e = 0; e < kObsF / 2; ++e) dst[e] = *reinterpret_cast<const double2 *>(&F[2 * e]);
+      }
     }
     __syncthreads();
     double *part = reinterpret_cast<double *>(B.schur_partial);
-    for (int i = t; i < ci.seg_count * 54; i += blockDim.x) {
+    for (int i = i0; i < ci.seg_count * 54; i += kChunkCap * parts) {
       const int sg = i / 54, en = i - 54 * sg;
       int b0 = f_b0, b1 = f_b1, sl = f_slot;
-      if (i != t) {
+      if (i != i0) {
         b0 = B.seg_pos[ci.seg_begin + sg];
         b1 = (sg + 1 < ci.seg_count) ? B.seg_pos[ci.seg_begin + sg + 1] : ci.obs_count;
         sl = B.seg_slot[ci.seg_begin + sg];
@@ -386,15 +393,29 @@ size_t point_schur_smem(bool mixed) {
   return mixed ? sizeof(PointSchurSmem<float>) : sizeof(PointSchurSmem<double>);
 }
 
+// CTAs per chunk of the FP64 explicit form: while there are SMs to spare, the
+// segments' sums (the longest part of a chunk) are shared by two CTAs, each
+// of which forms the chunk's F for itself.  One, two and four a chunk: 31, 26
+// and 26 us on 14 chunks, 33, 29 and 29 on 55; two on 100 chunks 37, one 33.
+static int ex64_parts(int nchunks) {
+  int sms = 0, dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return 1;
+  return std::max(1, std::min(2, sms / std::max(nchunks, 1)));
+}
+
 void launch_point_prepare(const DeviceBatch &b, bool mixed, cudaStream_t s) {
   // without the explicit Schur complement the factor rows are not allocated
   // (more CTAs per SM in the FP64 form)
   const size_t lcb = b.explicit_schur ? 0 : kChunkCap * 6 * (mixed ? sizeof(float) : sizeof(double));
   if (mixed)
     k_point_schur<true><<<b.nchunks, kChunkCap, point_schur_smem(true) - lcb, s>>>(b);
-  else if (b.explicit_schur)
-    k_point_schur_ex64<<<b.nchunks, kChunkCap, sizeof(PointSchurEx64Smem), s>>>(b);
-  else
+  else if (b.explicit_schur) {
+    if (const int parts = ex64_parts(b.nchunks); parts > 1)
+      k_point_schur_ex64<true><<<dim3((unsigned)b.nchunks, (unsigned)parts), kChunkCap, sizeof(PointSchurEx64Smem), s>>>(b);
+    else
+      k_point_schur_ex64<false><<<b.nchunks, kChunkCap, sizeof(PointSchurEx64Smem), s>>>(b);
+  } else
     k_point_schur<false><<<b.nchunks, kChunkCap, point_schur_smem(false) - lcb, s>>>(b);
 }
 
@@ -578,7 +599,8 @@ cudaError_t raise_smem_limit(const void *func, size_t bytes) {
 void point_schur_init() {
   cudaFuncSetAttribute(k_point_schur<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)point_schur_smem(true));
   cudaFuncSetAttribute(k_point_schur<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)point_schur_smem(false));
-  cudaFuncSetAttribute(k_point_schur_ex64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PointSchurEx64Smem));
+  for (const void *f : {(const void *)k_point_schur_ex64<true>, (const void *)k_point_schur_ex64<false>})
+    cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PointSchurEx64Smem));
 }
 
 
