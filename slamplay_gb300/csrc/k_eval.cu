@@ -63,20 +63,29 @@ void launch_init_state(const DeviceBatch &b, cudaStream_t s) {
 // the mixed form to all four.  sc: the CTA's staging, the cameras' parameters
 // in sc.cam; cameras [c0, c0 + m), of which those with live[.] get a table.
 // (one thread a camera: 16-19 us a launch for up to 250 cameras FP64, 20-31
-// us mixed)
+// us mixed).  Left-multiplicative rotations take their derivatives from R and
+// rigs need none: R alone, a quarter of the instructions.
 constexpr int kCamTableCams = 32;
 constexpr int kCamTableThreads = 128;
 struct CamStage {
   double cam[kCamTableCams][9];
   double tab[kCamTableCams][45];
+  double turn[kCamTableCams][7];  // the new rotation and translation (manifold updates)
   int live[kCamTableCams];
 };
 __device__ __forceinline__ void camera_tables(const DeviceBatch &B, CamStage &sc, int c0, int m) {
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const bool bare = B.opt.so3_left || B.opt.pinhole;
   if (warp < 3 && lane < m && sc.live[lane]) {
     double *tab = sc.tab[lane];
     const double *cam = sc.cam[lane];
-    if (warp == 0)
+    if (bare && warp == 0)
+      rotation_column<0>(cam, tab);
+    else if (bare && warp == 1)
+      rotation_column<1>(cam, tab);
+    else if (bare)
+      rotation_column<2>(cam, tab);
+    else if (warp == 0)
       rotation_columns<0, 1>(cam, tab);
     else if (warp == 1)
       rotation_columns<1, 2>(cam, tab);
@@ -86,7 +95,7 @@ __device__ __forceinline__ void camera_tables(const DeviceBatch &B, CamStage &sc
   if (warp == 3 && lane < m)
     for (int k = 36; k < kCamTable; ++k) sc.tab[lane][k] = k < 42 ? sc.cam[lane][k - 33] : 0.0;
   __syncthreads();
-  if (B.opt.so3_left) {
+  if (bare) {
     if (warp == 0 && lane < m) so3_left_derivatives(sc.tab[lane]);
     __syncthreads();
   }
@@ -979,44 +988,53 @@ __global__ void __launch_bounds__(kCamTableThreads) k_candidate_cameras(DeviceBa
   const LMState *L = B.lm + B.cam_problem[c0 + min(lane, m - 1)];
   const bool live = lane < m && L->active && L->linear_ok;
   const bool used = live && B.cam_used[c] != 0;
+  // poses that move on their manifold (T <- exp(xi) T on SE3 for local-BA
+  // windows, R <- exp(dw) R otherwise): the rotation by one warp and the SE3
+  // translation by another (some 500 FP64 instructions in a row for a thread
+  // that does both)
+  const bool manifold = (B.opt.pinhole || B.opt.so3_left) && used;
+  const double *x = B.cam_param[L->parity] + 9 * (size_t)c;
+  const double *y = B.pcg_x + 9 * (size_t)c, *s9 = B.cam_scale + 9 * (size_t)c;
   if (t < 32) {
     sc.live[lane] = live;
-    if (live) {
-      const double *x = B.cam_param[L->parity] + 9 * (size_t)c;
-      double *xc = B.cam_param[L->parity ^ 1] + 9 * (size_t)c;
-      double cand[9];
-      double s2 = 0.0;
+    if (live)
       for (int q = 0; q < 9; ++q) {
-        const double step = -B.pcg_x[9 * (size_t)c + q];
-        cand[q] = used ? x[q] + step * B.cam_scale[9 * (size_t)c + q] : x[q];
+        const double step = -y[q];
+        sc.cam[lane][q] = used ? x[q] + step * s9[q] : x[q];
       }
-      if (B.opt.pinhole && used) {
-        // local-BA windows: the pose moves on SE3, T <- exp(xi) T
-        const double *y = B.pcg_x + 9 * (size_t)c, *s9 = B.cam_scale + 9 * (size_t)c;
-        const double dw[3] = {-y[0] * s9[0], -y[1] * s9[1], -y[2] * s9[2]};
-        const double du[3] = {-y[3] * s9[3], -y[4] * s9[4], -y[5] * s9[5]};
-        se3_compose_left(dw, du, x, cand);
-      } else if (B.opt.so3_left && used) {
-        const double dw[3] = {-B.pcg_x[9 * (size_t)c + 0] * B.cam_scale[9 * (size_t)c + 0],
-                              -B.pcg_x[9 * (size_t)c + 1] * B.cam_scale[9 * (size_t)c + 1],
-                              -B.pcg_x[9 * (size_t)c + 2] * B.cam_scale[9 * (size_t)c + 2]};
-        compose_left(dw, x, cand);
-      }
-      for (int q = 0; q < 9; ++q) {
-        const double d = x[q] - cand[q];
-        s2 += d * d;
-        xc[q] = cand[q];
-        sc.cam[lane][q] = cand[q];
-      }
-      B.cam_scal[(size_t)kCamScal * c + kCC_STEP2] = used ? s2 : 0.0;
+  } else if (t < 64) {
+    if (manifold) {
+      const double dw[3] = {-y[0] * s9[0], -y[1] * s9[1], -y[2] * s9[2]};
+      compose_left(dw, x, sc.turn[lane]);
     }
-  } else if (t >= 96 && live) {
+  } else if (t < 96) {
+    if (manifold && B.opt.pinhole) {
+      const double dw[3] = {-y[0] * s9[0], -y[1] * s9[1], -y[2] * s9[2]};
+      const double du[3] = {-y[3] * s9[3], -y[4] * s9[4], -y[5] * s9[5]};
+      se3_compose_translation(dw, du, x, sc.turn[lane] + 3);
+    }
+  } else if (live) {
     // the camera part of step.g (the mixed form's model cost change)
     double yg = 0.0;
     for (int q = 0; q < 9; ++q) yg += B.pcg_x[9 * (size_t)c + q] * B.cam_g[9 * (size_t)c + q];
     B.cam_scal[(size_t)kCamScal * c + kCC_YG] = used ? -yg : 0.0;
   }
   __syncthreads();
+  if (manifold && t < (B.opt.pinhole ? 64 : 32)) {
+    const int q0 = 3 * (t >> 5);
+    for (int q = q0; q < q0 + 3; ++q) sc.cam[lane][q] = sc.turn[lane][q];
+  }
+  __syncthreads();
+  if (t >= 96 && live) {
+    double *xc = B.cam_param[L->parity ^ 1] + 9 * (size_t)c;
+    double s2 = 0.0;
+    for (int q = 0; q < 9; ++q) {
+      const double cand = sc.cam[lane][q], d = x[q] - cand;
+      s2 += d * d;
+      xc[q] = cand;
+    }
+    B.cam_scal[(size_t)kCamScal * c + kCC_STEP2] = used ? s2 : 0.0;
+  }
   camera_tables(B, sc, c0, m);
 }
 

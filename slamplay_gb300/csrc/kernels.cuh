@@ -593,6 +593,14 @@ __device__ inline void rotation_columns(const double *aa_in, double *tab) {
   }
 }
 
+// Column J of R alone (the compiler drops the derivatives): the same values.
+template <int J>
+__device__ inline void rotation_column(const double *aa_in, double *tab) {
+  double t[kCamTable];
+  rotation_columns<J, J + 1>(aa_in, t);
+  tab[J] = t[J], tab[3 + J] = t[3 + J], tab[6 + J] = t[6 + J];
+}
+
 // A camera's table without the derivatives (the compiler drops them): the
 // same R as a table with them.
 __device__ inline void camera_table_entry(const double *cam, double *tab) {
@@ -755,8 +763,9 @@ __device__ __forceinline__ void aa_rotate(const double *w, const double *p, doub
 // T <- exp(xi) T on SE3 (VertexPose::oplusImpl, g2o_types.h:55-60), xi =
 // (rotation dw, translation du): R' = exp(dw) R, t' = exp(dw) t + V(dw) du,
 // V = I + (1 - cos th)/th^2 [dw]x + (th - sin th)/th^3 [dw]x^2 (series below
-// th = 1e-4).  pose = angle-axis (3), translation (3).
-__device__ inline void se3_compose_left(const double *dw, const double *du, const double *pose, double *out) {
+// th = 1e-4).  pose = angle-axis (3), translation (3).  The translation t'
+// into out; the rotation is compose_left's.
+__device__ inline void se3_compose_translation(const double *dw, const double *du, const double *pose, double *out) {
   const double th2 = dw[0] * dw[0] + dw[1] * dw[1] + dw[2] * dw[2], th = sqrt(th2);
   double a, b;
   if (th < 1e-4) {
@@ -770,14 +779,10 @@ __device__ inline void se3_compose_left(const double *dw, const double *du, cons
   }
   const double c1[3] = {dw[1] * du[2] - dw[2] * du[1], dw[2] * du[0] - dw[0] * du[2], dw[0] * du[1] - dw[1] * du[0]};
   const double c2[3] = {dw[1] * c1[2] - dw[2] * c1[1], dw[2] * c1[0] - dw[0] * c1[2], dw[0] * c1[1] - dw[1] * c1[0]};
-  double rt[3], w[3];
+  double rt[3];
   aa_rotate(dw, pose + 3, rt);
-  compose_left(dw, pose, w);
 #pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    out[i] = w[i];
-    out[3 + i] = rt[i] + (du[i] + a * c1[i] + b * c2[i]);
-  }
+  for (int i = 0; i < 3; ++i) out[i] = rt[i] + (du[i] + a * c1[i] + b * c2[i]);
 }
 
 // Ceres robust-loss rho(s) (LossFunction::Evaluate) for trivial, Huber(a),
