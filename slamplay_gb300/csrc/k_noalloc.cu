@@ -77,7 +77,9 @@ __global__ void k_na_tables(const double *cameras, int nc, double *tables) {
 // (9 additions instead of 40), for problems that still fill the GPU that way;
 // W = 1: a warp per 32.  5M observations of 1,800 cameras: 393 us with a warp
 // per 32, FP64 comparisons and conversions in the reciprocal and a second
-// kernel for the partials; 327 us now (the 28 instructions alone: 290 us).
+// kernel for the partials; 327 us now (FP64 pipe 88 % active; its instructions
+// alone: 254 us).  As fast: a grid of the resident CTAs whose warps take
+// partials in turn (329); slower: CTAs of four warps (351).
 template <int W>
 __global__ void __launch_bounds__(kNoAllocThreads)
     k_na_residuals(gba_device_problem p, const double *tables, int loss, double loss_scale, double *residuals,
