@@ -375,7 +375,7 @@ def run_gpu(args) -> None:
         roof = {"kernel": top["name"], "bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s",
                 "frac": ach / peak, "traffic": ncu_traffic(top["name"], "fp64"), "bytes_per_launch": bytes_per,
                 "avg_launch_ms": avg_ms,
-                "binding_roof": ("FP64 latency chain: grid-wide barriers and problem-wide FP64 reductions between "
+                "binding_roof": ("FP64 latency chain: exchanges between SMs and problem-wide FP64 reductions between "
                                  "the products (FP64 pipe 23% active, DRAM 0.06% of peak; "
                                  "profiles/pcg_grid_config1_fp64.md)") if top["name"] == "pcg_grid" else None,
                 "timing": "CUDA events around each launch on the solver stream, host-driven pass of the same "

@@ -72,7 +72,7 @@ __global__ void k_na_tables(const double *cameras, int nc, double *tables) {
 // A cost partial is the sum of 256 observations: each 32 by a butterfly over
 // a warp's lanes, the eight results in order.  What bounds the kernel is the
 // FP64 pipe (one warp instruction per 64 clocks per SM sub-partition), about
-// 28 instructions per 32 observations and, a warp per 32, 6 more for the
+// 32 instructions per 32 observations and, a warp per 32, 6 more for the
 // sums.  W = 8: a warp takes all 256 and runs the eight butterflies at once
 // (9 additions instead of 40), for problems that still fill the GPU that way;
 // W = 1: a warp per 32.  5M observations of 1,800 cameras: 393 us with a warp
