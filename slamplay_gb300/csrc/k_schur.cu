@@ -145,14 +145,25 @@ __global__ void __launch_bounds__(32 * kForm64Warps) k_schur_form(DeviceBatch B)
 // asynchronously, a round ahead.  Before and after, per launch: 882 and 535 us
 // on 68,000 blocks of 107 pairs, 323 and 213 on 192 windows of 5-40 cameras,
 // 122 and 87 on 250 cameras, 38 and 33 on one window of 8 cameras (blocks of
-// up to 1,300 pairs: the chain of one block's steps bounds it).  A warp per
-// block with 3x3 tiles (two loads per entry and pair) took 431 us on the
-// 68,000 blocks but 104 on 250 cameras and 74 on the one window.
+// up to 1,300 pairs: the chain of one block's steps bounds it).
 constexpr int kTileWarps = 4;
 constexpr int kTilePairs = 16;  // pairs of a round a warp copies
 constexpr int kTileStages = 2;
 static_assert(kFormPairs == kTileWarps * kTilePairs && kFormSub == 3, "stages of a round");
 static_assert(kTilePairs * 2 == 32 && kObsF == 28, "a lane per row index, seven 16-byte copies a row");
+
+// Entry e of block blk: its three runs combined in order, stored with the
+// transpose.
+__device__ __forceinline__ void store_mixed_entry(const DeviceBatch &B, const KahanF *part, int blk, int e) {
+  KahanF s = part[e];
+#pragma unroll
+  for (int j = 1; j < kFormSub; ++j) s.merge(part[81 * j + e]);
+  const float v = -s.rvalue();
+  float *vals = reinterpret_cast<float *>(B.sblk_val);
+  const int tr = B.sblk_tr[blk];
+  vals[81 * (size_t)blk + e] = v;
+  if (tr != blk) vals[81 * (size_t)tr + 9 * (e % 9) + e / 9] = v;
+}
 
 __global__ void __launch_bounds__(32 * kTileWarps) k_schur_form_mixed(DeviceBatch B) {
   __shared__ __align__(16) float Fs[kTileStages][kFormPairs][2][kObsF];
@@ -232,23 +243,128 @@ __global__ void __launch_bounds__(32 * kTileWarps) k_schur_form_mixed(DeviceBatc
 #pragma unroll
     for (int i = 0; i < 3; ++i) part[81 * sub + 9 * (3 * ti + i) + kc] = acc[i];
   __syncthreads();
-  // the three runs of each entry combined in order, stored with the transpose
-  const int e = threadIdx.x;
-  if (e < 81) {
-    KahanF s = part[e];
-#pragma unroll
-    for (int j = 1; j < kFormSub; ++j) s.merge(part[81 * j + e]);
-    const float v = -s.rvalue();
-    float *vals = reinterpret_cast<float *>(B.sblk_val);
-    const int tr = B.sblk_tr[blk];
-    vals[81 * (size_t)blk + e] = v;
-    if (tr != blk) vals[81 * (size_t)tr + 9 * (e % 9) + e / 9] = v;
-  }
+  if (threadIdx.x < 81) store_mixed_entry(B, part, blk, threadIdx.x);
 }
+
+// K3c of the mixed form when there are far more blocks than the GPU holds
+// warps: a warp per block, a lane summing a 3x3 tile (two loads per entry and
+// pair instead of four; 9 tiles times the three runs on 27 lanes), the warps
+// independent of one another.  A long block is then one warp's chain, which
+// many blocks hide and few do not.  The form above and this one, by blocks:
+// 15,000 (100 windows) 269 and 316 us, 26,000 (1,800 cameras of a walk) 103
+// and 82, 30,000 (200 windows) 445 and 431, 66,000 (1,800 cameras) 535 and
+// 421, 100,000 (a walk) 307 and 197.  A round of 64 pairs comes 16 at
+// a time, two of them ahead; the step of three pairs that crosses into the 16
+// that just landed is done first, then the stage of the 16 before is free.
+constexpr int kWarpFormBlocks = 24576;
+constexpr int kWarpFormStages = 3;
+
+__global__ void __launch_bounds__(32 * kTileWarps) k_schur_form_warp(DeviceBatch B) {
+  __shared__ __align__(16) float Fs[kTileWarps][kWarpFormStages][kTilePairs][2][kObsF];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int ub = blockIdx.x * kTileWarps + warp;
+  if (ub >= B.nup) return;
+  const int blk = B.sblk_up[ub];
+  const int p0 = B.sblk_pair[ub], p1 = B.sblk_pair[ub + 1];
+  if (!B.lm[B.cam_problem[B.sblk_col[blk]]].active) return;  // uniform over the warp
+  const float *F = reinterpret_cast<const float *>(B.obs_F);
+  const int *pairs = reinterpret_cast<const int *>(B.spair);
+  // lane l: the observation of pair g + l / 2, the row's (even) or the column's
+  auto load_index = [&](int g) { return g + (lane >> 1) < p1 ? pairs[2 * (size_t)g + lane] : 0; };
+  auto stage_rows = [&](int g, int st, int ob) {  // the rows of pairs [g, g + 16), none beyond p1
+    const int rows = 2 * (p1 - g);
+    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&Fs[warp][st][0][0][0]);
+#pragma unroll
+    for (int u = 0; u < 7; ++u) {
+      const int i = lane + 32 * u, row = i / 7, e = i - 7 * row;
+      const int o = __shfl_sync(0xffffffffu, ob, row);
+      if (row < rows)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16u * (uint32_t)i),
+                     "l"(F + (size_t)kObsF * o + 4 * e)
+                     : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  const int sub = min(lane / 9, kFormSub), tile = lane - 9 * (lane / 9), ti = tile / 3, tk = tile - 3 * ti;
+  const int last = min(sub, kFormSub - 1);  // (lanes 27-31 repeat a run's pairs and drop the result)
+  KahanF acc[9];
+#pragma unroll
+  for (int e = 0; e < 9; ++e) acc[e].init();
+  struct Rows {
+    float a[9], b[9];
+  };
+  auto load_rows = [&](int st, int r) {  // of pair r of a stage
+    Rows f;
+    const float *fa = &Fs[warp][st][r][0][9 * ti], *fb = &Fs[warp][st][r][1][9 * tk];
+#pragma unroll
+    for (int e = 0; e < 9; ++e) f.a[e] = fa[e], f.b[e] = fb[e];
+    return f;
+  };
+  auto add_rows = [&](const Rows &f) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+        acc[3 * i + k].add(f.a[3 * i] * f.b[3 * k] + f.a[3 * i + 1] * f.b[3 * k + 1] + f.a[3 * i + 2] * f.b[3 * k + 2]);
+  };
+  stage_rows(p0, 0, load_index(p0));
+  stage_rows(p0 + kTilePairs, 1, load_index(p0 + kTilePairs));
+  int ob = load_index(p0 + 2 * kTilePairs);
+  int done = 0;  // pairs summed, from the start of the current 16 (negative: left over from the 16 before)
+  int st = 0, prev = kWarpFormStages - 1;
+  for (int g = p0, it = 0; g < p1; g += kTilePairs, ++it) {
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncwarp();
+    const int n = min(kTilePairs, p1 - g);
+    if (done < 0 && done + kFormSub <= n) {
+      const int r = done + last;
+      add_rows(load_rows(r < 0 ? prev : st, r < 0 ? r + kTilePairs : r));
+      done += kFormSub;
+      __syncwarp();
+    }
+    // (a step still open here needs the stage of the 16 before, and nothing is left to copy)
+    if (done >= 0) {
+      stage_rows(g + 2 * kTilePairs, prev, ob);
+      ob = load_index(g + 3 * kTilePairs);
+    }
+    if (done >= 0 && done + kFormSub <= n) {
+      Rows f = load_rows(st, done + last);
+#pragma unroll 2
+      for (done += kFormSub; done + kFormSub <= n; done += kFormSub) {
+        const Rows nf = load_rows(st, done + last);
+        add_rows(f);
+        f = nf;
+      }
+      add_rows(f);
+    }
+    if ((it & 3) == 3 || g + kTilePairs >= p1) {  // the round's last pairs
+      const int r = done + sub;
+      if (r < n) add_rows(load_rows(r < 0 ? prev : st, r < 0 ? r + kTilePairs : r));
+      done = kTilePairs;
+    }
+    done -= kTilePairs;
+    prev = st;
+    st = st == kWarpFormStages - 1 ? 0 : st + 1;
+    __syncwarp();
+  }
+  KahanF *part = reinterpret_cast<KahanF *>(&Fs[warp][0][0][0][0]);
+  if (sub < kFormSub)
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int k = 0; k < 3; ++k) part[81 * sub + 9 * (3 * ti + i) + 3 * tk + k] = acc[3 * i + k];
+  __syncwarp();
+  for (int e = lane; e < 81; e += 32) store_mixed_entry(B, part, blk, e);
+}
+static_assert(sizeof(KahanF) * 81 * kFormSub <= sizeof(float) * kWarpFormStages * kTilePairs * 2 * kObsF,
+              "the runs fit the stages");
+static_assert(kTilePairs % 3 == 1, "two pairs at most are left over from a stage");
 
 void launch_schur_form(const DeviceBatch &b, bool mixed, cudaStream_t s) {
   if (!b.explicit_schur || b.nup == 0) return;
-  if (mixed)
+  if (mixed && b.nup >= kWarpFormBlocks)
+    k_schur_form_warp<<<(b.nup + kTileWarps - 1) / kTileWarps, 32 * kTileWarps, 0, s>>>(b);
+  else if (mixed)
     k_schur_form_mixed<<<b.nup, 32 * kTileWarps, 0, s>>>(b);
   else
     k_schur_form<<<2 * b.nup, 32 * kForm64Warps, 0, s>>>(b);

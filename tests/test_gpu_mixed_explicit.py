@@ -56,6 +56,12 @@ def test_formation_pair_counts(npt):
     assert _step_error(_dense(4, npt, 40 + npt), 1) <= 1e-4
 
 
+@pytest.mark.parametrize("npt", [1, 2, 3, 15, 16, 17, 18, 33, 49, 63, 64, 65, 81])
+def test_formation_many_blocks(npt):
+    """24,976 blocks: a warp each, 16 pairs of a round at a time."""
+    assert _step_error(_dense(224, npt, npt), 1) <= 1e-4
+
+
 @pytest.mark.parametrize("nc", [455, 460, 1000, 3700])
 def test_product_cameras_per_cta(nc):
     """Up to eight and more cameras a CTA, one after the other: the PCG's
