@@ -176,7 +176,7 @@ typedef struct gba_options {
   int32_t chunk_observations;         /* point-segment tile (obs per CTA), 0 = auto  */
   int32_t reorder_points;             /* 1 = group points by first camera (locality) */
   int32_t use_graphs;                 /* 1 = run the LM loop as one CUDA graph       */
-  int32_t pcg_unroll;                 /* PCG iterations per graph body, 0 = auto (2) */
+  int32_t pcg_unroll;                 /* PCG iterations per graph body, 0 = auto (4) */
   int32_t autotune;                   /* 1 = run gba_autotune on the first solve of a
                                          new problem-size bucket                     */
   int32_t schur;                      /* gba_schur, GBA_SCHUR_AUTO                   */
