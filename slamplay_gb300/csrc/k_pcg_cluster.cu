@@ -274,6 +274,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_pcg_cluster(DeviceBatch B, in
   const unsigned gmask = ((1u << kClSub) - 1u) << ((t & 31) & ~(kClSub - 1));
   // camera-coordinate mapping of the per-camera sums: a half-warp per camera
   const int hq = t & 15, hc = t >> 4;
+  const int wc = hc & ~1;  // the warp's first camera: a warp without one does not take issue slots from the others
   const unsigned hmask = 0xffffu << (t & 16);
   __syncthreads();
   // the thread's first triplet of S stays in registers: reading S from
@@ -368,7 +369,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_pcg_cluster(DeviceBatch B, in
     }
     __syncthreads();
     // each owned camera's p.q
-    for (int cb = 0; cb < own_n; cb += T / 16) {
+    for (int cb = 0; cb + wc < own_n; cb += T / 16) {
       const int lc = cb + hc;
       DF d = df_zero();
       if (lc < own_n && hq < 9) {
@@ -406,7 +407,7 @@ __global__ void __launch_bounds__(kClThreads, 1) k_pcg_cluster(DeviceBatch B, in
       xh[i] = x.hi, xl[i] = x.lo;
       return x;
     };
-    for (int cb = 0; cb < own_n; cb += T / 16) {
+    for (int cb = 0; cb + wc < own_n; cb += T / 16) {
       const int lc = cb + hc;
       const bool act = lc < own_n && hq < 9;
       const int i = 9 * lc + hq;
