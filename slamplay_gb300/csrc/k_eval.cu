@@ -753,8 +753,10 @@ __global__ void __launch_bounds__(kPieceThreads) k_eval_camera_pieces(DeviceBatc
   const int k0 = B.cam_piece_begin[c], npc = B.cam_piece_begin[c + 1] - k0;
   const int e1 = B.cam_obs_begin[c + 1];
   const int o0 = B.cam_obs_begin[c] + (piece - k0) * kCamPieceObs, o1 = min(o0 + kCamPieceObs, e1);
-  auto sums = [&](auto first, int ln) {
-    constexpr int A0 = decltype(first)::value ? 0 : 3, A1 = decltype(first)::value ? 3 : 9;
+  auto sums = [&](auto first, auto rig, int ln) {
+    // a rig's poses have six parameters: the other entries stay zero
+    constexpr int N = decltype(rig)::value ? 6 : 9, cut = decltype(rig)::value ? 2 : 3;
+    constexpr int A0 = decltype(first)::value ? 0 : cut, A1 = decltype(first)::value ? cut : N;
     double acc[27];
 #pragma unroll
     for (int q = 0; q < 27; ++q) acc[q] = 0.0;
@@ -762,13 +764,13 @@ __global__ void __launch_bounds__(kPieceThreads) k_eval_camera_pieces(DeviceBatc
       const int64_t o = B.cam_obs_list[k];
       double2 J[9];
 #pragma unroll
-      for (int q = A0; q < 9; ++q) J[q] = jload<double2>(B.jac, B.no, q, o);
+      for (int q = A0; q < N; ++q) J[q] = jload<double2>(B.jac, B.no, q, o);
       const double2 r = jload<double2>(B.jac, B.no, 12, o);
       int i = 0;
 #pragma unroll
       for (int a = A0; a < A1; ++a) {
 #pragma unroll
-        for (int b = a; b < 9; ++b, ++i) acc[i] = fma(J[a].y, J[b].y, fma(J[a].x, J[b].x, acc[i]));
+        for (int b = a; b < N; ++b, ++i) acc[i] = fma(J[a].y, J[b].y, fma(J[a].x, J[b].x, acc[i]));
         acc[i] = fma(J[a].y, r.y, fma(J[a].x, r.x, acc[i]));
         ++i;
       }
@@ -777,18 +779,26 @@ __global__ void __launch_bounds__(kPieceThreads) k_eval_camera_pieces(DeviceBatc
 #pragma unroll
     for (int a = A0; a < A1; ++a) {
 #pragma unroll
-      for (int b = a; b < 9; ++b, ++i) part[ln][sym9(a, b)] = acc[i];
+      for (int b = a; b < N; ++b, ++i) part[ln][sym9(a, b)] = acc[i];
       part[ln][45 + a] = acc[i];
       ++i;
     }
   };
+  const bool rig = B.opt.pinhole != 0;
   if (t < kPieceLanes)
-    sums(std::true_type(), t);
+    rig ? sums(std::true_type(), std::true_type(), t) : sums(std::true_type(), std::false_type(), t);
   else
-    sums(std::false_type(), t - kPieceLanes);
+    rig ? sums(std::false_type(), std::true_type(), t - kPieceLanes) : sums(std::false_type(), std::false_type(), t - kPieceLanes);
   __syncthreads();
   double s = 0.0;
-  if (t < 54)
+  bool none = false;
+  if (rig) {
+    int a = t - 45, b = 0;
+    if (t < 45)
+      for (a = 0, b = t; b >= 9 - a; ++a) b -= 9 - a;
+    none = a >= 6 || (t < 45 && a + b >= 6);
+  }
+  if (t < 54 && !none)
     for (int i = 0; i < kPieceLanes; ++i) s += part[i][t];
   if (npc > 1) {
     // the piece's sums to the camera's slots; the last piece adds them up

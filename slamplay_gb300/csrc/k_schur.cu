@@ -102,8 +102,21 @@ __global__ void __launch_bounds__(32 * kForm64Warps) k_schur_form(DeviceBatch B)
   // sub-lane `sub` of entry (i, k) sums the pairs sub, sub + kFormSub, ... of
   // every round of 64, in order: one FMA chain through the accumulator (three
   // FP64 operations a pair, not four)
-  const int e0 = (blockIdx.x & 1) * kForm64Split, cnt = min(kForm64Split, 81 - e0);
-  const int sub = t / cnt, en = e0 + t - cnt * sub, ei = en / 9, ek = en - 9 * ei;
+  const int half = blockIdx.x & 1, tr = B.sblk_tr[blk];
+  double *vals = reinterpret_cast<double *>(B.sblk_val);
+  auto store = [&](int i, int k, double v) {
+    vals[81 * (size_t)blk + 9 * i + k] = v;
+    if (tr != blk) vals[81 * (size_t)tr + 9 * k + i] = v;
+  };
+  // a rig's poses have six parameters: its 36 entries by the first CTA, the
+  // zeros (negated, as a sum would be) by the second
+  const bool rig = B.opt.pinhole != 0;
+  if (rig && half == 1) {
+    if (t < 81 && (t / 9 >= 6 || t % 9 >= 6)) store(t / 9, t % 9, -0.0);
+    return;
+  }
+  const int e0 = half * kForm64Split, cnt = rig ? 36 : min(kForm64Split, 81 - e0), wide = rig ? 6 : 9;
+  const int sub = t / cnt, en = e0 + t - cnt * sub, ei = en / wide, ek = en - wide * ei;
   double acc = 0.0;
   stage_rows(p0, 0, load_index(p0));
   int ob = load_index(p0 + kForm64Pairs);
@@ -128,11 +141,7 @@ __global__ void __launch_bounds__(32 * kForm64Warps) k_schur_form(DeviceBatch B)
     double s = part[0][t];
 #pragma unroll
     for (int j = 1; j < kFormSub; ++j) s += part[j][t];
-    const double v = -s;
-    double *vals = reinterpret_cast<double *>(B.sblk_val);
-    const int e = e0 + t, tr = B.sblk_tr[blk];
-    vals[81 * (size_t)blk + e] = v;
-    if (tr != blk) vals[81 * (size_t)tr + 9 * (e % 9) + e / 9] = v;
+    store((e0 + t) / wide, (e0 + t) % wide, -s);
   }
 }
 
@@ -193,6 +202,7 @@ __global__ void __launch_bounds__(32 * kTileWarps) k_schur_form_mixed(DeviceBatc
   };
   const int sub = lane / 9, tile = lane - 9 * sub, ti = tile / 3, kc = 3 * warp + tile - 3 * ti;
   const int last = min(sub, kFormSub - 1);  // (lanes 27-31 repeat a run's pairs and drop the result)
+  const int busy = B.opt.pinhole ? 2 : 3;   // a rig's poses have six parameters: columns 6-8 stay zero
   KahanF acc[3];
 #pragma unroll
   for (int e = 0; e < 3; ++e) acc[e].init();
@@ -220,7 +230,7 @@ __global__ void __launch_bounds__(32 * kTileWarps) k_schur_form_mixed(DeviceBatc
     __syncthreads();  // the round has landed; every warp is done with the one before
     stage_rows(g + kFormPairs * (kTileStages - 1), st == 0 ? kTileStages - 1 : st - 1, ob);
     ob = load_index(g + kFormPairs * kTileStages);
-    if (warp < 3) {
+    if (warp < busy) {
       const int n = min(kFormPairs, p1 - g);
       int done = 0;
       if (n >= kFormSub) {

@@ -87,9 +87,38 @@ __device__ __forceinline__ void sym9_pair(int e, int &a, int &b) {
   b = a + e;
 }
 
+// The (segment, entry) sums of a chunk: per segment the 45 entries of a
+// symmetric 9x9 and 9 of a vector or, for a rig's poses of six parameters, the
+// 21 and 6 that are not zero (K3b takes the others as zero).  Entry en: (a, b)
+// of the matrix or a of the vector (false), and its place in the segment's
+// record.
+template <bool RIG>
+constexpr int kChunkEntries = RIG ? 27 : 54;
+template <bool RIG>
+__device__ __forceinline__ bool chunk_entry(int en, int &a, int &b, int &place) {
+  if constexpr (!RIG) {
+    place = en;
+    a = en - 45, b = 0;
+    if (en < 45) sym9_pair(en, a, b);
+    return en < 45;
+  } else {
+    if (en >= 21) {
+      a = en - 21, b = 0, place = 45 + a;
+      return false;
+    }
+    int e = en, r = 6;
+    a = 0;
+    while (e >= r) e -= r, --r, ++a;
+    b = a + e;
+    place = sym9(a, b);
+    return true;
+  }
+}
+
 // (the mixed form at four CTAs per SM: 64 registers a thread)
-template <bool MIXED>
+template <bool MIXED, bool RIG>
 __global__ void __launch_bounds__(kChunkCap, MIXED ? 4 : 1) k_point_schur(DeviceBatch B) {
+  constexpr int E = kChunkEntries<RIG>;
   typedef typename Prec<MIXED>::real real;
   typedef typename Prec<MIXED>::real2 real2;
   typedef typename Acc<MIXED>::type Acc;
@@ -152,8 +181,8 @@ __global__ void __launch_bounds__(kChunkCap, MIXED ? 4 : 1) k_point_schur(Device
     }
     // the first (segment, entry) task of this thread: its metadata now
     int f_b0 = 0, f_b1 = 0, f_slot = 0;
-    if (t < ci.seg_count * 54) {
-      const int sg = t / 54;
+    if (t < ci.seg_count * E) {
+      const int sg = t / E;
       f_b0 = B.seg_pos[ci.seg_begin + sg];
       f_b1 = (sg + 1 < ci.seg_count) ? B.seg_pos[ci.seg_begin + sg + 1] : ci.obs_count;
       f_slot = B.seg_slot[ci.seg_begin + sg];
@@ -205,8 +234,8 @@ __global__ void __launch_bounds__(kChunkCap, MIXED ? 4 : 1) k_point_schur(Device
     }
     __syncthreads();
     real *part = reinterpret_cast<real *>(B.schur_partial);
-    for (int i = t; i < ci.seg_count * 54; i += blockDim.x) {
-      const int sg = i / 54, en = i - 54 * sg;
+    for (int i = t; i < ci.seg_count * E; i += blockDim.x) {
+      const int sg = i / E, en = i - E * sg;
       int b0 = f_b0, b1 = f_b1, sl = f_slot;
       if (i != t) {
         b0 = B.seg_pos[ci.seg_begin + sg];
@@ -215,9 +244,8 @@ __global__ void __launch_bounds__(kChunkCap, MIXED ? 4 : 1) k_point_schur(Device
       }
       Acc acc;
       acc.init();
-      if (en < 45) {
-        int a, b;
-        sym9_pair(en, a, b);
+      int a, b, place;
+      if (chunk_entry<RIG>(en, a, b, place)) {
         for (int k = b0; k < b1; ++k) {
           const real ua = sm.jc[k][2 * a], va = sm.jc[k][2 * a + 1];
           const real ub = sm.jc[k][2 * b], vb = sm.jc[k][2 * b + 1];
@@ -225,10 +253,9 @@ __global__ void __launch_bounds__(kChunkCap, MIXED ? 4 : 1) k_point_schur(Device
           acc.add(ua * (A00 * ub + A01 * vb) + va * (A01 * ub + A11 * vb));
         }
       } else {
-        const int a = en - 45;
         for (int k = b0; k < b1; ++k) acc.add(sm.jc[k][2 * a] * sm.ae[k][3] + sm.jc[k][2 * a + 1] * sm.ae[k][4]);
       }
-      part[54 * (size_t)sl + en] = (real)acc.rvalue();
+      part[54 * (size_t)sl + place] = (real)acc.rvalue();
     }
     __syncthreads();
   }
@@ -255,8 +282,9 @@ struct PointSchurEx64Smem {
 };
 
 // SPLIT: gridDim.y CTAs a chunk.
-template <bool SPLIT>
+template <bool SPLIT, bool RIG>
 __global__ void __launch_bounds__(kChunkCap) k_point_schur_ex64(DeviceBatch B) {
+  constexpr int E = kChunkEntries<RIG>;
   extern __shared__ __align__(16) unsigned char k3x_smem[];
   PointSchurEx64Smem &sm = *reinterpret_cast<PointSchurEx64Smem *>(k3x_smem);
   const int t = threadIdx.x, part_y = SPLIT ? blockIdx.y : 0, parts = SPLIT ? gridDim.y : 1;
@@ -329,8 +357,8 @@ __global__ void __launch_bounds__(kChunkCap) k_point_schur_ex64(DeviceBatch B) {
     // the first (segment, entry) task of this thread: its metadata now
     const int i0 = t + kChunkCap * part_y;
     int f_b0 = 0, f_b1 = 0, f_slot = 0;
-    if (i0 < ci.seg_count * 54) {
-      const int sg = i0 / 54;
+    if (i0 < ci.seg_count * E) {
+      const int sg = i0 / E;
       f_b0 = B.seg_pos[ci.seg_begin + sg];
       f_b1 = (sg + 1 < ci.seg_count) ? B.seg_pos[ci.seg_begin + sg + 1] : ci.obs_count;
       f_slot = B.seg_slot[ci.seg_begin + sg];
@@ -365,8 +393,8 @@ __global__ void __launch_bounds__(kChunkCap) k_point_schur_ex64(DeviceBatch B) {
     }
     __syncthreads();
     double *part = reinterpret_cast<double *>(B.schur_partial);
-    for (int i = i0; i < ci.seg_count * 54; i += kChunkCap * parts) {
-      const int sg = i / 54, en = i - 54 * sg;
+    for (int i = i0; i < ci.seg_count * E; i += kChunkCap * parts) {
+      const int sg = i / E, en = i - E * sg;
       int b0 = f_b0, b1 = f_b1, sl = f_slot;
       if (i != i0) {
         b0 = B.seg_pos[ci.seg_begin + sg];
@@ -375,15 +403,15 @@ __global__ void __launch_bounds__(kChunkCap) k_point_schur_ex64(DeviceBatch B) {
       }
       // F_a . F_b of entry (a, b), or F_a . u: one loop for both (a warp
       // holds lanes of both kinds and would run two, one after the other)
-      int a = en - 45, b = 0;
-      if (en < 45) sym9_pair(en, a, b);
-      const double *fa = sm.F[b0] + 3 * a, *fb = en < 45 ? sm.F[b0] + 3 * b : sm.us[b0];
-      const int step = en < 45 ? 27 : 3;
+      int a, b, place;
+      const bool mat = chunk_entry<RIG>(en, a, b, place);
+      const double *fa = sm.F[b0] + 3 * a, *fb = mat ? sm.F[b0] + 3 * b : sm.us[b0];
+      const int step = mat ? 27 : 3;
       double acc = 0.0;
 #pragma unroll 4
       for (int k = b0; k < b1; ++k, fa += 27, fb += step)
         acc = fma(fa[2], fb[2], fma(fa[1], fb[1], fma(fa[0], fb[0], acc)));
-      part[54 * (size_t)sl + en] = acc;
+      part[54 * (size_t)sl + place] = acc;
     }
     __syncthreads();
   }
@@ -408,15 +436,17 @@ void launch_point_prepare(const DeviceBatch &b, bool mixed, cudaStream_t s) {
   // without the explicit Schur complement the factor rows are not allocated
   // (more CTAs per SM in the FP64 form)
   const size_t lcb = b.explicit_schur ? 0 : kChunkCap * 6 * (mixed ? sizeof(float) : sizeof(double));
-  if (mixed)
-    k_point_schur<true><<<b.nchunks, kChunkCap, point_schur_smem(true) - lcb, s>>>(b);
-  else if (b.explicit_schur) {
-    if (const int parts = ex64_parts(b.nchunks); parts > 1)
-      k_point_schur_ex64<true><<<dim3((unsigned)b.nchunks, (unsigned)parts), kChunkCap, sizeof(PointSchurEx64Smem), s>>>(b);
-    else
-      k_point_schur_ex64<false><<<b.nchunks, kChunkCap, sizeof(PointSchurEx64Smem), s>>>(b);
-  } else
-    k_point_schur<false><<<b.nchunks, kChunkCap, point_schur_smem(false) - lcb, s>>>(b);
+  const bool rig = b.opt.pinhole != 0;
+  if (!mixed && b.explicit_schur) {
+    const int parts = ex64_parts(b.nchunks);
+    auto *f = parts > 1 ? (rig ? k_point_schur_ex64<true, true> : k_point_schur_ex64<true, false>)
+                        : (rig ? k_point_schur_ex64<false, true> : k_point_schur_ex64<false, false>);
+    f<<<dim3((unsigned)b.nchunks, (unsigned)parts), kChunkCap, sizeof(PointSchurEx64Smem), s>>>(b);
+  } else {
+    auto *f = mixed ? (rig ? k_point_schur<true, true> : k_point_schur<true, false>)
+                    : (rig ? k_point_schur<false, true> : k_point_schur<false, false>);
+    f<<<b.nchunks, kChunkCap, point_schur_smem(mixed) - lcb, s>>>(b);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -479,7 +509,11 @@ __global__ void __launch_bounds__(kSchurThreads) k_camera_schur(DeviceBatch B) {
     // interleaved accumulators, combined pairwise)
     if (t < 54) {
       const real *part = reinterpret_cast<const real *>(B.schur_partial) + t;
-      const int s0 = B.cam_seg_begin[c], s1 = B.cam_seg_begin[c + 1];
+      int ea = t - 45, eb = 0;
+      if (t < 45) sym9_pair(t, ea, eb);
+      // (a rig's poses have six parameters: no partials of the others)
+      const bool none = B.opt.pinhole && (ea >= 6 || eb >= 6);
+      const int s0 = B.cam_seg_begin[c], s1 = none ? s0 : B.cam_seg_begin[c + 1];
       constexpr int kBatch = 16;
       constexpr int kAcc = MIXED ? 1 : 4;
       Acc a[kAcc];
@@ -597,9 +631,12 @@ cudaError_t raise_smem_limit(const void *func, size_t bytes) {
 
 // Large dynamic shared memory of the point-Schur kernel (FP64 form).
 void point_schur_init() {
-  cudaFuncSetAttribute(k_point_schur<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)point_schur_smem(true));
-  cudaFuncSetAttribute(k_point_schur<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)point_schur_smem(false));
-  for (const void *f : {(const void *)k_point_schur_ex64<true>, (const void *)k_point_schur_ex64<false>})
+  for (const void *f : {(const void *)k_point_schur<true, true>, (const void *)k_point_schur<true, false>})
+    cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)point_schur_smem(true));
+  for (const void *f : {(const void *)k_point_schur<false, true>, (const void *)k_point_schur<false, false>})
+    cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)point_schur_smem(false));
+  for (const void *f : {(const void *)k_point_schur_ex64<true, true>, (const void *)k_point_schur_ex64<true, false>,
+                        (const void *)k_point_schur_ex64<false, true>, (const void *)k_point_schur_ex64<false, false>})
     cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PointSchurEx64Smem));
 }
 
