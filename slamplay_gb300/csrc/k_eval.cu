@@ -148,12 +148,23 @@ __device__ __forceinline__ double eval_rig(const DeviceBatch &B, int64_t o, int 
   const double cost = block_cost(loss, B.opt.loss_scale, ru, rv);
   if (loss != GBA_LOSS_TRIVIAL) {
     const Corrector cr = make_corrector(loss, B.opt.loss_scale, ru, rv);
+    uint32_t top = max(high_abs(ru), high_abs(rv));
+#pragma unroll
+    for (int k = 0; k < 12; ++k) top = max(top, max(high_abs(ju[k]), high_abs(jv[k])));
+    if (!no_outer<double>(cr, top)) {
+#pragma unroll
+      for (int k = 0; k < 12; ++k) {
+        if (k >= 6 && k < 9) continue;
+        const double rJ = ru * ju[k] + rv * jv[k];
+        ju[k] -= cr.alpha_sq_norm * ru * rJ;
+        jv[k] -= cr.alpha_sq_norm * rv * rJ;
+      }
+    }
 #pragma unroll
     for (int k = 0; k < 12; ++k) {
       if (k >= 6 && k < 9) continue;
-      const double rJ = ru * ju[k] + rv * jv[k];
-      ju[k] = cr.sqrt_rho1 * (ju[k] - cr.alpha_sq_norm * ru * rJ);
-      jv[k] = cr.sqrt_rho1 * (jv[k] - cr.alpha_sq_norm * rv * rJ);
+      ju[k] *= cr.sqrt_rho1;
+      jv[k] *= cr.sqrt_rho1;
     }
     ru *= cr.residual_scaling;
     rv *= cr.residual_scaling;
@@ -242,12 +253,19 @@ __device__ __forceinline__ double eval_observation(const DeviceBatch &B, int64_t
     const Corrector cr = make_corrector(loss, B.opt.loss_scale, ru, rv);
     const real s1 = (real)cr.sqrt_rho1, al = (real)cr.alpha_sq_norm;
     const real rur = (real)ru, rvr = (real)rv;
+    uint32_t top = max(high_abs(rur), high_abs(rvr));
 #pragma unroll
-    for (int k = 0; k < 12; ++k) {
-      const real rJ = rur * ju[k] + rvr * jv[k];
-      ju[k] = s1 * (ju[k] - al * rur * rJ);
-      jv[k] = s1 * (jv[k] - al * rvr * rJ);
+    for (int k = 0; k < 12; ++k) top = max(top, max(high_abs(ju[k]), high_abs(jv[k])));
+    if (!no_outer<real>(cr, top)) {
+#pragma unroll
+      for (int k = 0; k < 12; ++k) {
+        const real rJ = rur * ju[k] + rvr * jv[k];
+        ju[k] -= al * rur * rJ;
+        jv[k] -= al * rvr * rJ;
+      }
     }
+#pragma unroll
+    for (int k = 0; k < 12; ++k) ju[k] *= s1, jv[k] *= s1;
     ru *= cr.residual_scaling;
     rv *= cr.residual_scaling;
   }
@@ -393,12 +411,19 @@ __device__ __forceinline__ double eval_observation_df(const DeviceBatch &B, int6
     const Corrector cr = make_corrector(loss, B.opt.loss_scale, ru, rv);
     const DF s1 = df_from_double(cr.sqrt_rho1), al = df_from_double(cr.alpha_sq_norm);
     const DF rur = df_from_double(ru), rvr = df_from_double(rv);
+    uint32_t top = max(high_abs(rur.hi), high_abs(rvr.hi));
 #pragma unroll
-    for (int k = 0; k < 12; ++k) {
-      const DF rJ = rur * ju[k] + rvr * jv[k];
-      ju[k] = s1 * (ju[k] - al * rur * rJ);
-      jv[k] = s1 * (jv[k] - al * rvr * rJ);
+    for (int k = 0; k < 12; ++k) top = max(top, max(high_abs(ju[k].hi), high_abs(jv[k].hi)));
+    if (!no_outer<float>(cr, top)) {
+#pragma unroll
+      for (int k = 0; k < 12; ++k) {
+        const DF rJ = rur * ju[k] + rvr * jv[k];
+        ju[k] = ju[k] - al * rur * rJ;
+        jv[k] = jv[k] - al * rvr * rJ;
+      }
     }
+#pragma unroll
+    for (int k = 0; k < 12; ++k) ju[k] = s1 * ju[k], jv[k] = s1 * jv[k];
     ru *= cr.residual_scaling;
     rv *= cr.residual_scaling;
   }

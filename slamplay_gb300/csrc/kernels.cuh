@@ -846,6 +846,18 @@ __device__ __forceinline__ Corrector make_corrector(int loss, double a, double r
   return c;
 }
 
+// alpha is zero for every loss whose rho'' is not positive (Huber, Cauchy), and
+// J - 0 r r^T J is J while r r^T J does not overflow, which J and r below a
+// bound rule out.  high_abs: the high word of a magnitude; no_outer: whether
+// the outer product may be left out (one branch around all of it: predicated
+// FP64 instructions would cost what they cost executed).
+__device__ __forceinline__ uint32_t high_abs(double v) { return (uint32_t)__double2hiint(v) & 0x7fffffffu; }
+__device__ __forceinline__ uint32_t high_abs(float v) { return __float_as_uint(v) & 0x7fffffffu; }
+template <typename T>
+__device__ __forceinline__ bool no_outer(const Corrector &c, uint32_t top) {
+  return __double_as_longlong(c.alpha_sq_norm) == 0 && top < (sizeof(T) == 8 ? 0x5f300000u : 0x53800000u);  // 2^500, 2^40
+}
+
 // Loads / stores of one observation's Jacobian columns from the SoA layout:
 // column k (k = 0..8 camera, 9..11 point) as a (d/du, d/dv) pair at
 // jac[k * no + o]; the corrected residual pair at jac[12 * no + o].
