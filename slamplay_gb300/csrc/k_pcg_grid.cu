@@ -38,8 +38,8 @@
 // of a walk 8.1 -> 6.7 us, 120 8.5 -> 7.1, 170 8.9 -> 7.5, 250 9.9 -> 8.0.
 // Left out, measured no faster: the CTAs that update camera blocks summing all
 // chunks themselves (75 cameras 6.75 us as now, 250 8.4 against 8.2); slower:
-// two warps or one pipelined warp polling a slot
-// in turns (250 cameras 8.9 and 10.7 us), no copies, slots 128 bytes apart.
+// two warps or one pipelined warp polling a slot in turns (250 cameras 8.9 and
+// 10.7 us), no copies, slots 128 bytes apart.
 // Every CTA takes the same decisions from the same values.  The arithmetic
 // is the two-kernel FP64 PCG's, operation for operation (the fixed trees of
 // kernels.cuh, k_schur.cu's product and the camera kernel's reductions), so
