@@ -149,6 +149,8 @@ class Engine {
   bool pdl_ = true;        // programmatic dependent launches inside the PCG body
   ClusterPlan cl_plan_;    // cs > 0: the PCG runs as one cluster launch per LM iteration
   Cluster64Plan c64_plan_; // cs > 0: the same in the FP64 form
+  ClusterPlan cl_late_;    // cs > 0: their shapes for few running problems of a batch,
+  Cluster64Plan c64_late_; // a launch beside the first
   GridPlan gr_plan_;       // grid > 0: the PCG runs as one grid-wide launch per LM iteration
   HostBatch hb_;           // the last solve's prepared batch (storage reused)
   gba_status enqueue_pcg_one_launch(cudaStream_t s, std::string *err);

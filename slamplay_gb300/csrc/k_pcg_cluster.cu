@@ -145,7 +145,7 @@ __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.w
 // QUAD: the quadratic-model stopping test, the only reader of x.(v + r).
 template <bool QUAD>
 __global__ void __launch_bounds__(kClThreads, 1) k_pcg_cluster(DeviceBatch B, int cs, int n_max, int own_max,
-                                                            int cache_blocks) {
+                                                            int cache_blocks, int above, int upto) {
   extern __shared__ __align__(16) unsigned char cl_smem[];
   const ClLayout lay = cl_layout(n_max, own_max, cache_blocks);
   float *zf = reinterpret_cast<float *>(cl_smem + lay.zf);
@@ -170,6 +170,9 @@ __global__ void __launch_bounds__(kClThreads, 1) k_pcg_cluster(DeviceBatch B, in
   __shared__ int s_lo, s_hi;
 
   const int rank = cs > 1 ? (int)cg::this_cluster().block_rank() : 0;
+  // (the count of running PCGs that K3b left; the other shape takes this one)
+  const int running = B.status[3];
+  if (running <= above || running > upto) return;
   const int prob = B.prob_order[blockIdx.x / cs];  // the longest first: the short ones fill in behind
   const int t = threadIdx.x, T = blockDim.x;
   LMState *L = B.lm + prob;
@@ -537,7 +540,7 @@ static const void *cluster_kernel(bool quad) {
 }
 
 bool pcg_cluster_plan(const ProblemInfo *prob, int num_problems, const int32_t *sblk_row, int cams_per_cta, bool quad,
-                      ClusterPlan *plan) {
+                      int running, ClusterPlan *plan) {
   *plan = ClusterPlan();
   const void *kernel = cluster_kernel(quad);
   int n_max = 0;
@@ -590,7 +593,7 @@ bool pcg_cluster_plan(const ProblemInfo *prob, int num_problems, const int32_t *
       if (l2.total > (size_t)optin) continue;
       for (int th : {256, 512}) {
         const int occ = std::max(1, std::min(512 / th, (int)((size_t)per_sm_bytes / (l2.total + 1024))));  // (128 registers a thread)
-        const double load = (double)num_problems * c2 / sms;
+        const double load = (double)running * c2 / sms;
         const double waves = load <= occ ? 1.0 : load / occ + 0.25, share = load > 1.0 && occ > 1 ? 1.15 : 1.0;
         const double rounds = std::ceil(3.0 * o2 / (th / 8)), upd = std::ceil((double)o2 / (th / 16));
         const double est = waves * share * ((ca ? 7.5 : 32.0) * mb + 500.0 * rounds + (th == 256 ? 1100.0 : 1500.0) * upd +
@@ -645,8 +648,8 @@ cudaError_t launch_pcg_cluster(const DeviceBatch &b, const ClusterPlan &plan, cu
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (plan.quad) return cudaLaunchKernelEx(&cfg, k_pcg_cluster<true>, b, plan.cs, plan.n_max, plan.own_max, plan.cache_blocks);
-  return cudaLaunchKernelEx(&cfg, k_pcg_cluster<false>, b, plan.cs, plan.n_max, plan.own_max, plan.cache_blocks);
+  return cudaLaunchKernelEx(&cfg, plan.quad ? k_pcg_cluster<true> : k_pcg_cluster<false>, b, plan.cs, plan.n_max,
+                            plan.own_max, plan.cache_blocks, plan.above, plan.upto);
 }
 
 }  // namespace gba

@@ -128,7 +128,7 @@ __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.w
 // barrier, the shortest chain).
 template <int R, bool QUAD>
 __global__ void __launch_bounds__(kC64Threads) k_pcg_cluster64(DeviceBatch B, int cs, int n_max, int own_max,
-                                                              int pairs_max) {
+                                                              int pairs_max, int above, int upto) {
   constexpr int kRows = R > 0 ? R : 1;
   constexpr int U = 9 / kRows;  // units per camera
   extern __shared__ __align__(16) unsigned char c64_smem[];
@@ -140,6 +140,9 @@ __global__ void __launch_bounds__(kC64Threads) k_pcg_cluster64(DeviceBatch B, in
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const unsigned full = 0xffffffffu;
   const int rank = cs > 1 ? (int)cg::this_cluster().block_rank() : 0;
+  // (the count of running PCGs that K3b left; the other shape takes this one)
+  const int running = B.status[3];
+  if (running <= above || running > upto) return;
   const int prob = B.prob_order[blockIdx.x / cs];  // the longest first: the short ones fill in behind
   LMState *L = B.lm + prob;
   // uniform over the cluster: every CTA reads the state before its first
@@ -629,7 +632,7 @@ __global__ void __launch_bounds__(kC64Threads) k_pcg_cluster64(DeviceBatch B, in
 
 namespace {
 
-typedef void (*C64Kernel)(DeviceBatch, int, int, int, int);
+typedef void (*C64Kernel)(DeviceBatch, int, int, int, int, int, int);
 C64Kernel c64_kernel(int R, bool quad) {
   if (quad) return R == 9 ? k_pcg_cluster64<9, true> : R == 3 ? k_pcg_cluster64<3, true> : R == 1 ? k_pcg_cluster64<1, true> : k_pcg_cluster64<0, true>;
   return R == 9 ? k_pcg_cluster64<9, false> : R == 3 ? k_pcg_cluster64<3, false> : R == 1 ? k_pcg_cluster64<1, false> : k_pcg_cluster64<0, false>;
@@ -650,7 +653,7 @@ void c64_config(const Cluster64Plan &p, int problems, cudaLaunchConfig_t *cfg, c
 
 }  // namespace
 
-bool pcg_cluster64_plan(const ProblemInfo *prob, int num_problems, const int32_t *sblk_row, bool quad,
+bool pcg_cluster64_plan(const ProblemInfo *prob, int num_problems, const int32_t *sblk_row, bool quad, int running,
                         Cluster64Plan *plan) {
   *plan = Cluster64Plan();
   int dev = 0, sms = 0, optin = 0;
@@ -690,9 +693,9 @@ bool pcg_cluster64_plan(const ProblemInfo *prob, int num_problems, const int32_t
       const C64Layout l = c64_layout(R, n_max, own, (int)pairs);
       if (l.total + 4096 > (size_t)optin) continue;
       const double per_sm = std::max(1.0, std::floor((double)(228 * 1024) / (double)(l.total + 4096)));
-      const double waves = std::max(1.0, std::ceil((double)num_problems * cs / (sms * per_sm)));
+      const double waves = std::max(1.0, std::ceil((double)running * cs / (sms * per_sm)));
       // CTAs that share an SM share its FP64 pipe
-      const double share = std::min(per_sm, std::max(1.0, (double)num_problems * cs / sms));
+      const double share = std::min(per_sm, std::max(1.0, (double)running * cs / sms));
       double chain;
       if (R == 0) {
         const double m = (double)w_max / n_max, fit = std::max(1.0, std::floor(32.0 / m)), runs = std::ceil(m / 32.0);
@@ -742,7 +745,8 @@ cudaError_t launch_pcg_cluster64(const DeviceBatch &b, const Cluster64Plan &plan
   cudaLaunchAttribute attr[1];
   c64_config(plan, b.num_problems, &cfg, attr);
   cfg.stream = s;
-  return cudaLaunchKernelEx(&cfg, c64_kernel(plan.R, plan.quad), b, plan.cs, plan.n_max, plan.own_max, plan.pairs_max);
+  return cudaLaunchKernelEx(&cfg, c64_kernel(plan.R, plan.quad), b, plan.cs, plan.n_max, plan.own_max, plan.pairs_max,
+                            plan.above, plan.upto);
 }
 
 }  // namespace gba

@@ -44,6 +44,7 @@ struct ClusterPlan {
   bool quad = false;
   int cache_blocks = 0;  // > 0: each CTA keeps its rows of S (this many 9x9 blocks at most) in shared memory
   size_t smem = 0;
+  int above = 0, upto = 1 << 30;  // the numbers of running PCGs it is launched for: (above, upto]
 };
 // Chooses the cluster size, the block size and whether the rows of S stay
 // in shared memory, from the batch's problems (camera ranges) and the
@@ -52,8 +53,10 @@ struct ClusterPlan {
 // cams_per_cta: the cameras of a problem one CTA of its cluster takes (the
 // cluster size follows); 0 = the shortest estimated iteration.
 // quad: the quadratic-model stopping test (gba_pcg_criterion).
+// running: the problems that share the GPU (num_problems, or fewer late in a
+// batch).
 bool pcg_cluster_plan(const ProblemInfo *prob, int num_problems, const int32_t *sblk_row, int cams_per_cta, bool quad,
-                      ClusterPlan *plan);
+                      int running, ClusterPlan *plan);
 cudaError_t launch_pcg_cluster(const DeviceBatch &b, const ClusterPlan &plan, cudaStream_t s);
 // K4 cluster form of the FP64 precision: as the above, the FP64 arithmetic of
 // the two-kernel PCG addition for addition (the same bits), problems whose
@@ -66,9 +69,10 @@ struct Cluster64Plan {
   int n_max = 0, own_max = 0, pairs_max = 0;
   size_t smem = 0;
   double clocks = 0;  // estimated clocks of the largest problem's PCG iteration
+  int above = 0, upto = 1 << 30;  // the numbers of running PCGs it is launched for: (above, upto]
 };
-// quad: the quadratic-model stopping test (gba_pcg_criterion).
-bool pcg_cluster64_plan(const ProblemInfo *prob, int num_problems, const int32_t *sblk_row, bool quad,
+// quad, running: as above.
+bool pcg_cluster64_plan(const ProblemInfo *prob, int num_problems, const int32_t *sblk_row, bool quad, int running,
                         Cluster64Plan *plan);
 cudaError_t launch_pcg_cluster64(const DeviceBatch &b, const Cluster64Plan &plan, cudaStream_t s);
 // K4 grid form: the whole PCG of one problem in one launch, one CTA per SM

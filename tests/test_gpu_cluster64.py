@@ -75,3 +75,26 @@ def test_cluster64_uneven_batch_equals_alone():
         with Solver(**OPTS) as s:
             s.solve(q)
         assert np.array_equal(q.parameters(), g.parameters())
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_late_shape_equals_alone(precision):
+    """Thirty problems that end at different LM iterations: once few of them
+    run, a launch of another shape takes over; each problem keeps the bits of
+    its own solve, with the graph and with the host-driven loop."""
+    probs = [BALProblem.synthetic(3, index=i, seed=11, num_cameras=5 + i, num_points=200 + 40 * i) for i in range(30)]
+    opts = dict(max_num_iterations=30, schur="explicit", pcg_tolerance=1e-6, max_linear_solver_iterations=60,
+                precision=precision)
+    runs = []
+    for graphs in (1, 0):
+        gs = [p.copy() for p in probs]
+        with Solver(use_graphs=graphs, **opts) as s:
+            sums = s.batch_solve(gs)
+        runs.append(gs)
+    its = sorted(x.num_iterations for x in sums)
+    assert its[0] < its[-1]
+    for p, a, b in zip(probs, *runs):
+        q = p.copy()
+        with Solver(**opts) as s:
+            s.solve(q)
+        assert np.array_equal(q.parameters(), a.parameters()) and np.array_equal(q.parameters(), b.parameters())
