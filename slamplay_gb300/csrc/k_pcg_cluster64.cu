@@ -372,10 +372,12 @@ __global__ void __launch_bounds__(kC64Threads) k_pcg_cluster64(DeviceBatch B, in
   int npass = 0;
   double a_s[9];  // the warp's first pass: its rows of S and its addresses in registers
   Pass first = {};
+  int rest = warp;  // the passes from memory start here (a first pass that is a row of more than 32 blocks among them)
   if constexpr (R == 0) {
     npass = s_npass;
     if (warp < npass) {
       first = pass_at(warp);
+      if (uoff[first.j + 1] - first.e0 <= 32) rest = warp + kC64Warps;
 #pragma unroll
       for (int cc = 0; cc < 9; ++cc) a_s[cc] = first.in ? first.s[cc] : 0.0;
     }
@@ -394,13 +396,13 @@ __global__ void __launch_bounds__(kC64Threads) k_pcg_cluster64(DeviceBatch B, in
   for (;;) {
     // ---- A. q = S p_k for the owned rows -----------------------------------
     if constexpr (R == 0) {
-      if (warp < npass) {
+      if (rest > warp) {
         double d = 0.0;
 #pragma unroll
         for (int cc = 0; cc < 9; ++cc) d = fma(a_s[cc], first.p[cc], d);
         finish_pass(d, first);
       }
-      for (int ps = warp + kC64Warps; ps < npass; ps += kC64Warps) {
+      for (int ps = rest; ps < npass; ps += kC64Warps) {
         const int j = pass_j[ps] & 0xffff, m0 = uoff[j + 1] - uoff[j];
         if (m0 <= 32) {
           const Pass a = pass_at(ps);
