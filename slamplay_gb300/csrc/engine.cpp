@@ -486,21 +486,11 @@ gba_status Engine::upload(const HostBatch &hb, std::string *err) {
   // current batch shape + pointers + options + PCG form = graph key
   DeviceBatch k = db_;
   cur_key_.assign(reinterpret_cast<const char *>(&k), reinterpret_cast<const char *>(&k) + sizeof k);
-  cur_key_.push_back(cl_plan_.cs);
-  cur_key_.push_back(cl_plan_.threads);
-  cur_key_.push_back(cl_plan_.cache_blocks);
-  cur_key_.push_back(cl_late_.cs);
-  cur_key_.push_back(cl_late_.threads);
-  cur_key_.push_back(cl_late_.cache_blocks);
-  cur_key_.push_back(c64_plan_.cs);
-  cur_key_.push_back(c64_plan_.R);
-  cur_key_.push_back(c64_plan_.pairs_max);
-  cur_key_.push_back(c64_late_.cs);
-  cur_key_.push_back(c64_late_.R);
-  cur_key_.push_back(c64_late_.pairs_max);
-  cur_key_.push_back(gr_plan_.grid);
-  cur_key_.push_back(gr_plan_.cap_cols);
-  cur_key_.push_back(gr_plan_.cap_pairs);
+  cl_plan_.append_to(&cur_key_);
+  cl_late_.append_to(&cur_key_);
+  c64_plan_.append_to(&cur_key_);
+  c64_late_.append_to(&cur_key_);
+  gr_plan_.append_to(&cur_key_);
   return GBA_OK;
 }
 

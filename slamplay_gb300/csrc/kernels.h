@@ -4,6 +4,8 @@
 
 #include <cuda_runtime.h>
 
+#include <vector>
+
 #include "gba_internal.h"
 
 namespace gba {
@@ -45,6 +47,12 @@ struct ClusterPlan {
   int cache_blocks = 0;  // > 0: each CTA keeps its rows of S (this many 9x9 blocks at most) in shared memory
   size_t smem = 0;
   int above = 0, upto = 1 << 30;  // the numbers of running PCGs it is launched for: (above, upto]
+  // What a captured launch carries of the plan: each field is part of the
+  // graph's key (batches of equal totals may split them over their problems in
+  // another way, and the shared memory is laid out by the largest problem).
+  void append_to(std::vector<long long> *key) const {
+    key->insert(key->end(), {cs, n_max, own_max, threads, quad, cache_blocks, (long long)smem, above, upto});
+  }
 };
 // Chooses the cluster size, the block size and whether the rows of S stay
 // in shared memory, from the batch's problems (camera ranges) and the
@@ -70,6 +78,9 @@ struct Cluster64Plan {
   size_t smem = 0;
   double clocks = 0;  // estimated clocks of the largest problem's PCG iteration
   int above = 0, upto = 1 << 30;  // the numbers of running PCGs it is launched for: (above, upto]
+  void append_to(std::vector<long long> *key) const {
+    key->insert(key->end(), {cs, R, quad, n_max, own_max, pairs_max, (long long)smem, above, upto});
+  }
 };
 // quad, running: as above.
 bool pcg_cluster64_plan(const ProblemInfo *prob, int num_problems, const int32_t *sblk_row, bool quad, int running,
@@ -83,6 +94,9 @@ struct GridPlan {
   int cap_pairs = 0;   // (row, block) pairs of one pass of the product
   bool quad = false;
   size_t smem = 0;
+  void append_to(std::vector<long long> *key) const {
+    key->insert(key->end(), {grid, cap_cols, cap_pairs, quad, (long long)smem});
+  }
 };
 // Sizes the launch from the problem's explicit-complement structure
 // (sblk_row, nc + 1, and sblk_col); false when the form does not apply (a
