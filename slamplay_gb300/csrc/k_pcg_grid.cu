@@ -28,9 +28,12 @@
 // costs the store's way to L2 and one read, no barrier, no fence and no
 // second read; the slots alternate between two sets by iteration parity, and
 // a set is only written again after every reader of its values has published
-// what depends on them.  One exchange from every CTA to every CTA would be
-// 152 x 152 readers of the same lines (5 us, measured), so the p.q goes in
-// two hops, over the CTAs that sum a chunk of 32 cameras, and what every CTA
+// what depends on them.  A CTA that owns nothing to publish therefore leaves
+// (a row pair can cost more than a CTA's share: 20 of the 150 CTAs of a
+// 30-camera walk own no unit, block or chunk).  One exchange from every CTA
+// to every CTA would be 152 x 152 readers of the same lines (5 us, measured),
+// so the p.q goes in two hops, over the CTAs that sum a chunk of 32 cameras,
+// and what every CTA
 // reads is published in kGridCopies copies.  A hop costs 0.4-1.3 us, most of
 // it the lines' way between the SMs and the two dies' L2.  Measured per PCG
 // iteration, against two grid-wide counter barriers with the values read
@@ -191,17 +194,7 @@ __host__ __device__ inline GridSmem grid_smem(int n, int cap_cols, int cap_pairs
   return l;
 }
 
-// The units of a CTA: a camera's rows in the pairs (0,1) (2,3) (4,5) (6,7)
-// and row 8, the first level of the camera's p.q sum.  A row costs the
-// camera's blocks m (off-diagonal + diagonal), a pair 2 m; the units are cut
-// into P runs of about equal cost.  Units of a camera that start before the
-// cost bound t, the rows before the camera costing `before` in all.
-__host__ __device__ inline int units5_below(long long t, long long before, long long m) {
-  if (t <= before) return 0;
-  const long long r = (t - before + 2 * m - 1) / (2 * m);
-  return r > 5 ? 5 : (int)r;
-}
-// First row of unit u (5 per camera).
+// First row of unit u (5 per camera; kernels.h has the CTAs' shares).
 __host__ __device__ inline int unit_row(int u) { return 9 * (u / 5) + 2 * (u % 5); }
 
 // A tree step does two levels of the pairwise tree, s and 2 s: entry i (a
@@ -273,7 +266,7 @@ __global__ void __launch_bounds__(kGThreads, 1) k_pcg_grid(DeviceBatch B, int ca
   const int r0 = B.sblk_row[c0];
   {
     const long long wtot = (long long)(B.sblk_row[c0 + n] - r0) + n;
-    const long long ta = ((long long)w * 9 * wtot + P - 1) / P, tb = ((long long)(w + 1) * 9 * wtot + P - 1) / P;
+    const long long ta = grid_bound(w, P, wtot), tb = grid_bound(w + 1, P, wtot);
     int a = 0, b = 0;
     for (int c = t; c < n; c += kGThreads) {
       const long long before = (long long)(B.sblk_row[c0 + c] - r0) + c;
@@ -286,9 +279,13 @@ __global__ void __launch_bounds__(kGThreads, 1) k_pcg_grid(DeviceBatch B, int ca
   }
   // update: camera blocks in P equal runs
   const int nblk = pi.cam_block_count;
-  const int kb0 = (int)((long long)w * nblk / P), kb1 = (int)((long long)(w + 1) * nblk / P);
+  const int kb0 = grid_run(w, P, nblk), kb1 = grid_run(w + 1, P, nblk);
+  // the chunks of 32 cameras whose p.q this CTA sums
+  const int nch = (n + 31) / 32;
+  const int ch0 = grid_run(w, P, nch), ch1 = grid_run(w + 1, P, nch);
   __syncthreads();
   const int ua = s_ua, nu = s_ub - ua;
+  if (!grid_takes_part(nu, kb1 - kb0, ch1 - ch0)) return;  // (uniform; CTA 0 owns the first unit)
   const int ra = unit_row(ua), own_rows = nu > 0 ? unit_row(ua + nu) - ra : 0;  // rows of the problem (local)
   const double *vals = reinterpret_cast<const double *>(B.sblk_val);
   const double *Sii = reinterpret_cast<const double *>(B.cam_Sii);
@@ -305,14 +302,11 @@ __global__ void __launch_bounds__(kGThreads, 1) k_pcg_grid(DeviceBatch B, int ca
   // the slots' two sets (by iteration parity): per row q, per coordinate z
   // and p, per unit p.q (by unit of the camera), and in kGridCopies copies
   // per chunk its p.q and per block its three sums
-  const int nch = (n + 31) / 32;
   const size_t n9 = 9 * (size_t)n;
   const size_t set = 3 * n9 + 5 * (size_t)n + kGridCopies * (3 * (size_t)nblk + (size_t)nch);
   GridSlot *const sl_q = B.grid_slots, *const sl_z = sl_q + n9, *const sl_p = sl_z + n9, *const sl_pq = sl_p + n9,
                   *const sl_c = sl_pq + 5 * (size_t)n, *const sl_b = sl_c + kGridCopies * (size_t)nch;
   const int copy = w % kGridCopies;  // the copy this CTA reads
-  // the chunks whose p.q this CTA sums
-  const int ch0 = (int)((long long)w * nch / P), ch1 = (int)((long long)(w + 1) * nch / P);
   const unsigned long long launch_tag = (unsigned long long)B.grid_ctl[kGridLaunch] << 32;
   // (the failure test waits for a tag that nothing writes)
   const unsigned long long miss = B.opt.grid_wait_test ? 1ull << 31 : 0ull;
@@ -802,7 +796,7 @@ bool pcg_grid_plan(int num_problems, bool mixed, bool explicit_schur, int nc, co
   int c = 0, j = 0;  // the next unit: camera, unit of the camera
   long long before = 0;
   for (int r = 0; r < grid; ++r) {
-    const long long tb = ((long long)(r + 1) * 9 * wtot + grid - 1) / grid;
+    const long long tb = grid_bound(r + 1, grid, wtot);
     long long pairs = 0;
     int cols = 0;
     while (c < nc) {

@@ -98,6 +98,24 @@ struct GridPlan {
     key->insert(key->end(), {grid, cap_cols, cap_pairs, quad, (long long)smem});
   }
 };
+// The CTAs' shares.  The units of the product: a camera's rows in the pairs
+// (0,1) (2,3) (4,5) (6,7) and row 8, the first level of the camera's p.q sum.
+// A row costs the camera's blocks m (off-diagonal + diagonal), a pair 2 m; the
+// units are cut into P runs of about equal cost.  Units of a camera that start
+// before the cost bound t, the rows before the camera costing `before` in all.
+__host__ __device__ inline int units5_below(long long t, long long before, long long m) {
+  if (t <= before) return 0;
+  const long long r = (t - before + 2 * m - 1) / (2 * m);
+  return r > 5 ? 5 : (int)r;
+}
+// CTA w's cost bound, of `rows` = the problem's blocks (the diagonal ones
+// included): it owns the units that start in [bound(w), bound(w + 1)).
+__host__ __device__ inline long long grid_bound(int w, int P, long long rows) { return ((long long)w * 9 * rows + P - 1) / P; }
+// CTA w's run of `total` camera blocks or chunks of cameras: from here to w + 1's.
+__host__ __device__ inline int grid_run(int w, int P, int total) { return (int)((long long)w * total / P); }
+// Only a CTA that publishes something every iteration may read what the
+// others publish: nothing holds a slot for a reader that no one waits for.
+__host__ __device__ inline bool grid_takes_part(int units, int blocks, int chunks) { return units > 0 || blocks > 0 || chunks > 0; }
 // Sizes the launch from the problem's explicit-complement structure
 // (sblk_row, nc + 1, and sblk_col); false when the form does not apply (a
 // batch, the mixed form, the implicit complement), when the CTAs' rows of S
