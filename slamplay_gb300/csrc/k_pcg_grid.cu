@@ -33,12 +33,12 @@
 // 30-camera walk own no unit, block or chunk).  One exchange from every CTA
 // to every CTA would be 152 x 152 readers of the same lines (5 us, measured),
 // so the p.q goes in two hops, over the CTAs that sum a chunk of 32 cameras,
-// and what every CTA
-// reads is published in kGridCopies copies.  A hop costs 0.4-1.3 us, most of
-// it the lines' way between the SMs and the two dies' L2.  Measured per PCG
-// iteration, against two grid-wide counter barriers with the values read
-// after them (which the values' copies and one read more replace): 75 cameras
-// of a walk 8.1 -> 6.7 us, 120 8.5 -> 7.1, 170 8.9 -> 7.5, 250 9.9 -> 8.0.
+// and what every CTA reads is published in kGridCopies copies.  A hop costs
+// 0.4-1.3 us, most of it the lines' way between the SMs and the two dies' L2.
+// Measured per PCG iteration, against two grid-wide counter barriers with the
+// values read after them (which the values' copies and one read more replace):
+// 75 cameras of a walk 8.1 -> 6.7 us, 120 8.5 -> 7.1, 170 8.9 -> 7.5, 250
+// 9.9 -> 8.0.
 // Left out, measured no faster: the CTAs that update camera blocks summing all
 // chunks themselves (75 cameras 6.75 us as now, 250 8.4 against 8.2); slower:
 // two warps or one pipelined warp polling a slot in turns (250 cameras 8.9 and
@@ -131,8 +131,8 @@ __device__ void grid_abort(const DeviceBatch &B) {
 }
 
 // Waits until the N slots of every lane with `need` carry `tag` and returns
-// their values; on a wait that ran out or was aborted sets *fail (the CTA
-// looks at it after its next barrier).  Call from a whole warp: the lanes
+// their values; on a wait that ran out or was aborted sets the threads' *fail
+// (the CTA's next checking barrier collects it).  Call from a whole warp: the lanes
 // leave the loop together (lanes that left one by one would run on apart, an
 // FP64 instruction issued for each).
 template <int N>
@@ -207,7 +207,7 @@ __host__ __device__ __forceinline__ int step_entries(int m, int s) { return m > 
 template <bool QUAD>
 __global__ void __launch_bounds__(kGThreads, 1) k_pcg_grid(DeviceBatch B, int cap_cols, int cap_pairs) {
   extern __shared__ __align__(16) unsigned char g_smem[];
-  __shared__ int s_ticket, s_P, s_ua, s_ub, s_stop, s_pass_end, s_npairs, s_nstep, s_good, s_fail, s_ncol;
+  __shared__ int s_ticket, s_P, s_ua, s_ub, s_stop, s_pass_end, s_npairs, s_nstep, s_good, s_ncol;
   __shared__ unsigned cmask[kGMaxCams / 32], cpre[kGMaxCams / 32];
   __shared__ int lbeg[kGSteps + 1];
   __shared__ double sc[3], s_inv_rz;
@@ -252,7 +252,6 @@ __global__ void __launch_bounds__(kGThreads, 1) k_pcg_grid(DeviceBatch B, int ca
     s_P = P;
     s_ua = 0;
     s_ub = 0;
-    s_fail = 0;
     s_ncol = 0;
   }
   for (int i = t; i < kGMaxCams / 32; i += kGThreads) cmask[i] = 0u;
@@ -434,6 +433,11 @@ __global__ void __launch_bounds__(kGThreads, 1) k_pcg_grid(DeviceBatch B, int ca
   const double lim = o.pcg_tolerance * L->r0_norm;
   const long long lim2_bits = __double_as_longlong(lim * lim);
   int k = 0;
+  // a wait of the thread's that ran out or was aborted: the two barriers that
+  // check it carry it to every thread (a flag in shared memory could be set by
+  // a warp past the check before the others have read it, and they would leave
+  // that warp behind at its next barrier)
+  int fail = 0;
   bool linear_ok = true, aborted = false;
 
   // the update's coordinate of this thread (coordinate m of a camera block
@@ -498,7 +502,7 @@ __global__ void __launch_bounds__(kGThreads, 1) k_pcg_grid(DeviceBatch B, int ca
             const double *row = (v < m - 1 ? vals + 81 * (size_t)(rr0 + v) : Sii + 81 * (size_t)(c0 + cl)) + 9 * q;
             const GridSlot *ps = sl_p + so + 9 * (size_t)pcol[roff[j] + v];
             double d = 0.0;
-            for (int cc = 0; cc < 9; ++cc) d = fma(row[cc], slot_wait(B, ps + cc, wait_tag, true, &s_fail), d);
+            for (int cc = 0; cc < 9; ++cc) d = fma(row[cc], slot_wait(B, ps + cc, wait_tag, true, &fail), d);
             if (v0 + lane < m) pd[roff[j] + v] = d;
           }
         }
@@ -545,8 +549,8 @@ __global__ void __launch_bounds__(kGThreads, 1) k_pcg_grid(DeviceBatch B, int ca
         const double qv = pd[roff[tr]], qv1 = pair ? pd[roff[tr + 1]] : 0.0;
         if (in) slot_put(sl_q + so + rho, qv, tag);
         // p_k at the unit's own coordinates: the diagonal block's column
-        const double p0 = slot_wait(B, sl_p + so + rho, wait_tag, even, &s_fail);
-        const double p1 = slot_wait(B, sl_p + so + rho + (pair ? 1 : 0), wait_tag, pair, &s_fail);
+        const double p0 = slot_wait(B, sl_p + so + rho, wait_tag, even, &fail);
+        const double p1 = slot_wait(B, sl_p + so + rho + (pair ? 1 : 0), wait_tag, pair, &fail);
         const double y0 = __dmul_rn(p0, qv), y1 = __dadd_rn(y0, __dmul_rn(p1, qv1));
         if (even) slot_put(sl_pq + so + (size_t)(q >> 1) * n + cl, pair ? y1 : y0, tag);
       }
@@ -561,7 +565,7 @@ __global__ void __launch_bounds__(kGThreads, 1) k_pcg_grid(DeviceBatch B, int ca
       const GridSlot *const pq0 = sl_pq + so + min(c, n - 1);
       const GridSlot *const a[5] = {pq0, pq0 + n, pq0 + 2 * (size_t)n, pq0 + 3 * (size_t)n, pq0 + 4 * (size_t)n};
       double y[5];
-      slots_wait<5>(B, a, wait_tag, c < n, y, &s_fail);
+      slots_wait<5>(B, a, wait_tag, c < n, y, &fail);
       double x = ((y[0] + y[1]) + (y[2] + y[3])) + y[4];  // (0 beyond the problem's cameras)
       x = warp_sum(x);
       if (lane < kGridCopies) slot_put(sl_c + so + (size_t)lane * nch + j, x, tag);
@@ -570,11 +574,11 @@ __global__ void __launch_bounds__(kGThreads, 1) k_pcg_grid(DeviceBatch B, int ca
     // tree: cta_chunked_sum's order), alpha; the update
     double qv = 0.0;
     if (one_round && __any_sync(full, u_lead))
-      qv = slot_wait(B, sl_q + so + (u_lead ? kPcgBlockCams * 9 * (size_t)(kb0 + u_slot) + u_m : 0), wait_tag, u_lead, &s_fail);
+      qv = slot_wait(B, sl_q + so + (u_lead ? kPcgBlockCams * 9 * (size_t)(kb0 + u_slot) + u_m : 0), wait_tag, u_lead, &fail);
     if (nch > 32) {
       for (int j0 = 32 * warp; j0 < nch; j0 += kGThreads) {
         const int j = min(j0 + lane, nch - 1);
-        chs[j] = slot_wait(B, sl_c + so + (size_t)copy * nch + j, wait_tag, true, &s_fail);
+        chs[j] = slot_wait(B, sl_c + so + (size_t)copy * nch + j, wait_tag, true, &fail);
       }
       __syncthreads();
       cta_pairwise_tree(chs, nch);
@@ -582,7 +586,7 @@ __global__ void __launch_bounds__(kGThreads, 1) k_pcg_grid(DeviceBatch B, int ca
     if (warp == 0) {
       double s2;
       if (nch <= 32) {  // the tree by one warp's shuffles
-        s2 = slot_wait(B, sl_c + so + (size_t)copy * nch + min(lane, nch - 1), wait_tag, lane < nch, &s_fail);
+        s2 = slot_wait(B, sl_c + so + (size_t)copy * nch + min(lane, nch - 1), wait_tag, lane < nch, &fail);
         for (int s = 1; s < nch; s <<= 1) {
           const double y = __shfl_down_sync(full, s2, s);
           s2 += (lane & (2 * s - 1)) == 0 && lane + s < nch ? y : 0.0;
@@ -598,8 +602,7 @@ __global__ void __launch_bounds__(kGThreads, 1) k_pcg_grid(DeviceBatch B, int ca
     } else if (t == kGThreads - 32) {
       s_inv_rz = recip_nr(rz_k);  // for beta, off the deciding warp's chain
     }
-    __syncthreads();
-    if (s_fail) {
+    if (__syncthreads_or(fail)) {
       aborted = true;
       break;
     }
@@ -616,7 +619,7 @@ __global__ void __launch_bounds__(kGThreads, 1) k_pcg_grid(DeviceBatch B, int ca
       bool lead = u_lead;
       if (!one_round) {
         lead = load_coordinate(blk, false);
-        qv = slot_wait(B, sl_q + so + (lead ? i : 0), wait_tag, lead, &s_fail);
+        qv = slot_wait(B, sl_q + so + (lead ? i : 0), wait_tag, lead, &fail);
       }
       if (lead) {
         ur = fma(-alpha, qv, ur);
@@ -682,7 +685,7 @@ __global__ void __launch_bounds__(kGThreads, 1) k_pcg_grid(DeviceBatch B, int ca
         const GridSlot *s3[3] = {p3, p3 + nblk, p3 + 2 * (size_t)nblk};
         const GridSlot *const(&sN)[N] = *reinterpret_cast<const GridSlot *const(*)[N]>(&s3);
         double y[N];
-        slots_wait<N>(B, sN, wait_tag, bb < nblk, y, &s_fail);
+        slots_wait<N>(B, sN, wait_tag, bb < nblk, y, &fail);
         if (b0 == 0)
           a = y[0], b = y[1], x = QUAD ? y[N - 1] : 0.0;
         else if (bb < nblk)
@@ -721,11 +724,10 @@ __global__ void __launch_bounds__(kGThreads, 1) k_pcg_grid(DeviceBatch B, int ca
       if (staged)
         for (int e0 = 32 * (warp - 1); e0 < 9 * ncol; e0 += kGThreads - 32) {
           const int e = min(e0 + lane, 9 * ncol - 1), cl = e / 9;
-          zc[e] = slot_wait(B, sl_z + so + 9 * (size_t)clist[cl] + (e - 9 * cl), wait_tag, true, &s_fail);
+          zc[e] = slot_wait(B, sl_z + so + 9 * (size_t)clist[cl] + (e - 9 * cl), wait_tag, true, &fail);
         }
     }
-    __syncthreads();
-    if (s_fail) {
+    if (__syncthreads_or(fail)) {
       aborted = true;
       break;
     }
