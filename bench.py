@@ -438,6 +438,8 @@ def linear_solver_name(prof: list[dict]) -> dict:
     pcg = "two kernels per PCG iteration"
     if "pcg_cluster" in names:
         pcg = "cluster (one launch per LM iteration)"
+    elif "pcg_cluster64" in names:
+        pcg = "FP64 cluster (one launch per LM iteration)"
     elif "pcg_grid" in names:
         pcg = "grid (one launch per LM iteration)"
     return {"schur": "explicit" if "schur_form" in names else "implicit", "pcg": pcg}

@@ -466,7 +466,10 @@ gba_status gba_evaluate_noalloc(const gba_device_problem *p, int32_t loss, doubl
                                 double *residuals, double *cost, void *stream);
 
 /* Per-kernel device times of the last gba_solve / gba_batch_solve when
- * profiling is on: kernel names, launches and total milliseconds. */
+ * profiling is on: kernel names, launches and total milliseconds.
+ * "pcg_grid" is the FP64 form's PCG in one launch per LM iteration, as a
+ * cluster per problem or over the whole GPU; "pcg_cluster64" counts those of
+ * them that were clusters (their time and bytes are under "pcg_grid"). */
 gba_status gba_set_profiling(gba_handle *h, int32_t on);
 int32_t gba_profile_count(const gba_handle *h);
 gba_status gba_profile_entry(const gba_handle *h, int32_t i, const char **name,

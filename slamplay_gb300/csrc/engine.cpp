@@ -49,12 +49,13 @@ enum ProfSlot {
   PF_FORM,
   PF_CLUSTER,
   PF_GRID,
+  PF_CLUSTER64,  // a count only (its time is PF_GRID's)
   PF_COUNT
 };
 const char *kProfNames[PF_COUNT] = {"eval_jacobian",  "post_eval", "point_schur",  "camera_schur",
                                     "schur_matvec",   "pcg_camera", "back_substitute", "candidate_cost",
                                     "decide",         "camera_table", "setup_misc", "schur_form",
-                                    "pcg_cluster",    "pcg_grid"};
+                                    "pcg_cluster",    "pcg_grid",   "pcg_cluster64"};
 
 double now_s() {
   return std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count();
@@ -898,6 +899,7 @@ gba_status Engine::enqueue_pcg_one_launch(cudaStream_t s, std::string *err) {
     if (st == GBA_OK && c64_late_.cs > 0)
       st = check(launch_pcg_cluster64(db_, c64_late_, s), "PCG cluster kernel", err);
     prof_end(s, PF_GRID, bytes_pcg_grid(db_));  // (the FP64 form's one-launch PCG)
+    if (profiling_) profile_[PF_CLUSTER64].launches += 1;
     return st;
   }
   if (gr_plan_.grid > 0) {

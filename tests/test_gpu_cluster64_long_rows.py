@@ -75,7 +75,7 @@ def test_hub_camera_equals_two_kernel_bitwise(cams, points, batch, hub):
         probs.append(BALProblem.synthetic(3, index=1, seed=3, num_cameras=6, num_points=250))
     ga, sa, pa = _solve(probs, persistent_pcg=1)
     gb, sb, pb = _solve(probs, persistent_pcg=0)
-    assert pa.get("pcg_grid", 0) > 0 and pb.get("pcg_grid", 0) == 0
+    assert pa["pcg_cluster64"] > 0 and pb["pcg_grid"] == 0
     for a, b, x, y in zip(ga, gb, sa, sb):
         np.testing.assert_array_equal(x.trace_cost, y.trace_cost)
         np.testing.assert_array_equal(x.trace_linear_iterations, y.trace_linear_iterations)
