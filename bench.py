@@ -206,12 +206,12 @@ def launches_per_solve(s, prof_launches: dict) -> int:
     """Kernels of one solve: setup (parameter sync, LM state, camera table,
     two evaluations of two kernels each, Jacobi scale, post-evaluation) and
     the gather = 10; per LM iteration point/Schur chunk, camera Schur, back-
-    substitution, candidate cameras, candidate cost, decide, camera table,
-    evaluation (chunk + camera), post-evaluation = 10, + 1 for the formation
+    substitution, candidate cameras (with their tables), candidate cost, decide,
+    evaluation (chunk + camera), post-evaluation = 9, + 1 for the formation
     of the explicit Schur complement; the PCG either as one launch per LM
     iteration (cluster or grid form) or as two kernels per PCG iteration.  prof_launches:
     launches per profile entry of a host-driven pass of the same solve."""
-    per_lm = 10 + (1 if prof_launches.get("schur_form") else 0)
+    per_lm = 9 + (1 if prof_launches.get("schur_form") else 0)
     pcg = prof_launches.get("pcg_cluster") or prof_launches.get("pcg_grid") or 2 * s.num_linear_solver_iterations
     return 10 + per_lm * s.num_iterations + pcg
 
@@ -376,7 +376,7 @@ def run_gpu(args) -> None:
                 "frac": ach / peak, "traffic": ncu_traffic(top["name"], "fp64"), "bytes_per_launch": bytes_per,
                 "avg_launch_ms": avg_ms,
                 "binding_roof": ("FP64 latency chain: exchanges between SMs and problem-wide FP64 reductions between "
-                                 "the products (FP64 pipe 23% active, DRAM 0.06% of peak; "
+                                 "the products (FP64 pipe 18% active, DRAM 0.08% of peak; "
                                  "profiles/pcg_grid_config1_fp64.md)") if top["name"] == "pcg_grid" else None,
                 "timing": "CUDA events around each launch on the solver stream, host-driven pass of the same "
                           "solve (kernels inside the conditional graph cannot be bracketed one by one)",
