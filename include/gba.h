@@ -186,9 +186,11 @@ typedef struct gba_options {
                                          thread-block cluster per problem (mixed
                                          precision up to 1,024 cameras; FP64 up to
                                          128 cameras whose blocks of S fit the
-                                         cluster's shared memory), a larger single
-                                         FP64 problem over the whole GPU
-                                         (grid-wide barriers; it
+                                         cluster's shared memory), a single FP64
+                                         problem that is larger, or too dense for
+                                         16 SMs (some from 30 cameras on), over
+                                         the whole GPU (values exchanged through
+                                         the L2, every wait bounded; it
                                          expects the GPU to itself: beside other
                                          kernels it runs on the SMs it finds free,
                                          correct but slower; the server's slots

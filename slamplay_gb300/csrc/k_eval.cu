@@ -13,7 +13,8 @@
 //                       partials).
 //  K7  k_post_eval      per problem: cost, gradient max-norm, |x|, Ceres'
 //                       termination tests, LM-loop condition.
-//  K5b k_candidate      per camera: candidate camera + its table (R only).
+//  K5b k_candidate_cameras  per camera: candidate camera + its table (with the
+//                       derivatives: an accepted step evaluates from it).
 //  K2  k_cost_chunk     per chunk: candidate cost in FP64.
 #include <cuda_runtime.h>
 

@@ -7,8 +7,8 @@
 // sooner, whatever the active lanes; a predicated-off one holds the pipe as
 // long, hence the uniform loops below), so the iteration's ~45 dependent
 // FP64 operations take about 1.5 us, and every exchange between SMs comes on
-// top.  The grid form (k_pcg_grid.cu) pays two grid-wide barriers and two L2
-// read-backs per iteration; the two-kernel form of a batch pays two kernel
+// top.  The grid form (k_pcg_grid.cu) pays three exchanges through L2 per
+// iteration (0.4-1.3 us each); the two-kernel form of a batch pays two kernel
 // boundaries and iterates until its slowest problem ends.  Here a cluster of
 // cs <= 16 CTAs keeps its problem's rows of S in shared memory and exchanges
 // through distributed shared memory between hardware cluster barriers (about
@@ -23,11 +23,11 @@
 //   C. every CTA: the blocks' sums, the stopping test, beta (one warp), while
 //      the other warps fetch z of the columns the CTA's rows touch; then
 //      p = z + beta p.
-// Measured (us per PCG iteration, local windows and rings, grid form -> this
-// one): 8 cameras 5.1 -> 3.4, 16 cameras 5.6 -> 4.0, 23 cameras 5.6 -> 4.1,
-// 39 cameras 6.2 -> 5.5.  Batches (the PCG of one LM iteration, two-kernel
-// form -> this one): 16 windows of 5-40 cameras 8.3 -> 2.1 ms, 48 windows
-// 8.8 -> 2.6 ms, 200 windows 18.6 -> 8.5 ms.
+// Measured (us per PCG iteration, local windows and rings, the grid form with
+// counter barriers -> this one): 8 cameras 5.1 -> 3.4, 16 cameras 5.6 -> 4.0,
+// 23 cameras 5.6 -> 4.1, 39 cameras 6.2 -> 5.5.  Batches (the PCG of one LM
+// iteration, two-kernel form -> this one): 16 windows of 5-40 cameras 8.3 ->
+// 2.1 ms, 48 windows 8.8 -> 2.6 ms, 200 windows 18.6 -> 8.5 ms.
 // The sums are the two-kernel form's and the grid form's, addition for
 // addition (kernels.cuh's trees; a butterfly level whose upper half holds
 // only zeros is left out, which changes no nonzero sum), so a problem gets

@@ -3,8 +3,9 @@
 // The LM system (J^T J + D^2) y = J^T r is solved with the points eliminated
 // (Schur complement on the cameras), as Ceres' SPARSE_SCHUR does for the
 // reference (test_bundle_adjustment_ceres.cpp:97), but the reduced camera
-// matrix S = B + Dc^2 - W C^-1 W^T is never formed: it is applied implicitly
-// inside a block-Jacobi PCG.
+// matrix S = B + Dc^2 - W C^-1 W^T is solved by a block-Jacobi PCG: formed as
+// camera-camera blocks where the view graph is sparse (k_schur.cu), else
+// applied implicitly.
 //
 //  K3a k_point_schur     per chunk: C = J_p^T J_p + Dp^2, FP64 inverse, Cinv g_p,
 //                        and per (camera segment) the partial Schur diagonal
@@ -12,8 +13,9 @@
 //  K3b k_camera_schur    per camera (CTA): S_ii and the reduced rhs from the
 //                        partials, parallel FP64 9x9 inverse, PCG start
 //                        (x = 0, r = v, z = M r)
-//  K4  (k_pcg.cu)        implicit-Schur PCG: mat-vec over point-segment
-//                        chunks, camera reduce, vector update
+//  K4  (k_pcg.cu, k_pcg_cluster.cu, k_pcg_cluster64.cu, k_pcg_grid.cu)
+//                        the PCG: two kernels per iteration (implicit
+//                        mat-vec, or the product with S), or one launch
 //  K5  k_back_substitute per chunk: y_p = C^-1 (g_p - W^T y_c), model cost
 //                        change, candidate points
 //  K6  k_decide          per problem: Ceres' accept / reject / radius update

@@ -86,8 +86,8 @@ struct Cluster64Plan {
 bool pcg_cluster64_plan(const ProblemInfo *prob, int num_problems, const int32_t *sblk_row, bool quad, int running,
                         Cluster64Plan *plan);
 cudaError_t launch_pcg_cluster64(const DeviceBatch &b, const Cluster64Plan &plan, cudaStream_t s);
-// K4 grid form: the whole PCG of one problem in one launch, one CTA per SM
-// with grid-wide barriers (FP64 form, explicit Schur complement).
+// K4 grid form: the whole PCG of one problem in one launch, one CTA per SM,
+// values exchanged as tagged slots (FP64 form, explicit Schur complement).
 struct GridPlan {
   int grid = 0;        // CTAs launched (the ones that register share the work)
   int cap_cols = 0;    // touched columns a CTA's shared-memory layout holds
