@@ -1,6 +1,7 @@
 // The key a captured solve is replayed by: two batches of equal totals whose
 // cameras are split over their problems in another way differ in nothing the
 // device arrays are sized by, so every plan field a launch carries is in it.
+#include <algorithm>
 #include <cstdio>
 #include <cstring>
 

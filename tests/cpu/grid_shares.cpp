@@ -2,6 +2,7 @@
 // camera block and chunk of cameras has one owner, and the CTAs that stay are
 // those that own something (a CTA that publishes nothing must not read what
 // the others publish: nobody waits for it before the values change).
+#include <algorithm>
 #include <cstdio>
 
 #include "kernels.h"
